@@ -455,7 +455,7 @@ typedef struct {
                               same brick word share one load (__match_any_sync + __shfl_sync) */
     int32_t l2_persist;    /* 1 = render launches carry an L2 access-policy window over the world's brick
                               words (persisting, as much as the device's persisting L2 holds) */
-    int32_t bounce_refill; /* deferred bounce rays: idle lanes (1..32) that make a warp refill; 0 = 8 */
+    int32_t bounce_refill; /* deferred bounce rays: idle lanes (1..32) that make a warp refill; 0 = 12 */
     int32_t bounce_walk;   /* deferred bounce rays: 0 = brick-run walk (unit steps of an occupied brick
                               in an inner loop), 1 = one advance per turn for jumps and unit steps alike */
     int32_t bounce_sort;   /* deferred bounce rays: 1 = each 16x16-pixel block of the frame kernel appends

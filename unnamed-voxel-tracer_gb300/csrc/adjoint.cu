@@ -55,7 +55,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // One block of 16x16 pixels of the view (f, hits, target, rgb); the rest of
 // the arguments are shared by all views.
-template <bool BWD>
+template <bool BWD, bool LONG>
 __device__ __forceinline__ void shade_block(const AdjArgs& a, const FrameParams& f, const uint4* __restrict__ hits,
                                             const float* __restrict__ target, float* __restrict__ rgb) {
     extern __shared__ float s_mem[];
@@ -104,7 +104,7 @@ __device__ __forceinline__ void shade_block(const AdjArgs& a, const FrameParams&
                 PRay rs;
                 pray_init(rs, so, a.sun);
                 TraceHit hs;
-                lit = !trace_fast<false, true, true>(a.w, cd, rs, a.shadow_steps, hs) &&
+                lit = !trace_fast<false, true, true, false, LONG>(a.w, cd, rs, a.shadow_steps, hs) &&
                       !(a.w.n_entities > 0 && entity_occluded(a.w, so, a.sun));
             }
             ndl_raw = dot3(nrm, a.sun_n);
@@ -193,9 +193,9 @@ __device__ __forceinline__ void shade_block(const AdjArgs& a, const FrameParams&
     }
 }
 
-template <bool BWD>
+template <bool BWD, bool LONG>
 __global__ void __launch_bounds__(kAdjBlock) k_shade(AdjArgs a) {
-    shade_block<BWD>(a, a.f, a.hits, a.target, a.rgb);
+    shade_block<BWD, LONG>(a, a.f, a.hits, a.target, a.rgb);
 }
 
 // Several views of one world in one launch (blockIdx.z = view): one launch
@@ -219,7 +219,7 @@ static_assert(sizeof(ViewsArgs) <= 4096, "the views travel in the kernel paramet
 // Register caps: 40 for the backward kernel (6 blocks per SM; a 12-byte
 // spill) and 48 for the forward one (5 blocks), the fastest of 40/48/59
 // measured on 16 views of 512x512.
-template <bool BWD>
+template <bool BWD, bool LONG>
 __global__ void __launch_bounds__(kAdjBlock, BWD ? 6 : 5) k_shade_views(ViewsArgs va) {
     const ViewP& V = va.v[blockIdx.z];
     if ((int)blockIdx.x * 16 >= V.width || (int)blockIdx.y * 16 >= V.height) return;  // the view is smaller
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kAdjBlock, BWD ? 6 : 5) k_shade_views(ViewsArg
     f.tan_half_fov = V.tan_half_fov;
     f.width = V.width;
     f.height = V.height;
-    shade_block<BWD>(va.a, f, V.hits, V.target, V.rgb);
+    shade_block<BWD, LONG>(va.a, f, V.hits, V.target, V.rgb);
 }
 
 // Checks the arguments shared by all views, brings the distances up to date on
@@ -280,8 +280,8 @@ vt_status launch_shade(vt_ctx* ctx, const vt_world* world, const vt_camera* cam,
     if (s) return s;
     a.hits = reinterpret_cast<const uint4*>(d_hits);
     const dim3 grid((cam->width + 15) / 16, (cam->height + 15) / 16);
-    if (bwd) k_shade<true><<<grid, kAdjBlock, kShadeSmem, st>>>(a);
-    else k_shade<false><<<grid, kAdjBlock, kShadeSmem, st>>>(a);
+    if (bwd) k_shade<true, true><<<grid, kAdjBlock, kShadeSmem, st>>>(a);
+    else k_shade<false, true><<<grid, kAdjBlock, kShadeSmem, st>>>(a);
     VT_CUDA(ctx, cudaGetLastError());
     return VT_OK;
 }
@@ -318,8 +318,10 @@ vt_status launch_shade_views(vt_ctx* ctx, const vt_world* world, int32_t n, cons
             gh = c.height > gh ? c.height : gh;
         }
         const dim3 grid((gw + 15) / 16, (gh + 15) / 16, nv);
-        if (bwd) k_shade_views<true><<<grid, kAdjBlock, kShadeSmem, st>>>(va);
-        else k_shade_views<false><<<grid, kAdjBlock, kShadeSmem, st>>>(va);
+        const bool lng = a.shadow_steps > kChunkSteps;
+        auto k = bwd ? (lng ? k_shade_views<true, true> : k_shade_views<true, false>)
+                     : (lng ? k_shade_views<false, true> : k_shade_views<false, false>);
+        k<<<grid, kAdjBlock, kShadeSmem, st>>>(va);
         VT_CUDA(ctx, cudaGetLastError());
     }
     return VT_OK;

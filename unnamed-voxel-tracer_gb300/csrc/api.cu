@@ -225,8 +225,8 @@ vt_status vt_ctx_destroy(vt_ctx* ctx) {
     if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
     if (ctx->h_status) host_free(ctx->h_status);
     if (ctx->ev_status) cudaEventDestroy(ctx->ev_status);
-    dev_free(ctx->d_bounce_jobs);
-    dev_free(ctx->d_bounce_open);
+    dev_free(ctx->d_bounce_head);
+    dev_free(ctx->d_bounce_tail);
     dev_free(ctx->d_bounce_ctr);
     if (ctx->ev_bounce) cudaEventDestroy(ctx->ev_bounce);
     for (int i = 0; i < ctx->n_screen; ++i) dev_free(ctx->screen[i].d);

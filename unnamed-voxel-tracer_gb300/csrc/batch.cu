@@ -78,7 +78,7 @@ static_assert(sizeof(JobChunk) <= 32764, "a kernel's parameters are limited to 3
 // One thread per pixel; the 256-thread block covers a 16 x 16 tile as eight
 // 8 x 4 warp tiles (the single-frame kernel's default shape), with the same
 // register cap (4 blocks per SM).
-template <bool CHECKED>
+template <bool CHECKED, bool BOUNCE, bool LONG>
 __global__ void __launch_bounds__(kBatchBlock, 4) k_render_jobs(const __grid_constant__ JobChunk p, unsigned* status) {
     const unsigned b = blockIdx.x;
     int lo = 0, hi = p.njobs - 1;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kBatchBlock, 4) k_render_jobs(const __grid_con
         uv.gv = s_row[2][ly];
     }
     PixelCounters pc;
-    const uint4 rec = render_pixel<false, CHECKED>(p.w, CoarseGlobal{p.w.coarse}, p.w.cdist, f, px, py, uv, status, pc);
+    const uint4 rec = render_pixel<false, CHECKED, CoarseGlobal, false, false, BOUNCE, LONG>(p.w, CoarseGlobal{p.w.coarse}, p.w.cdist, f, px, py, uv, status, pc);
     p.cam[lo].out[(size_t)py * f.width + px] = rec;
 }
 
@@ -356,10 +356,11 @@ vt_status vt_batch_launch(vt_batch* b, vt_stream stream) {
                     for (const auto& pc : chain_plan(wt)) {
                         const JobChunk& ch = b->chunks[pc.first];
                         const unsigned blocks = ch.first_block[ch.njobs];
-                        if (checked)
-                            k_render_jobs<true><<<blocks, kBatchBlock, 0, chain[pc.second]>>>(ch, ctx->d_status);
-                        else
-                            k_render_jobs<false><<<blocks, kBatchBlock, 0, chain[pc.second]>>>(ch, nullptr);
+                        const bool bounce = (b->params.rays & VT_RAYS_BOUNCE) != 0, lng = long_steps(ch.f);
+                        auto k = checked ? k_render_jobs<true, true, true>
+                                 : bounce ? (lng ? k_render_jobs<false, true, true> : k_render_jobs<false, true, false>)
+                                          : (lng ? k_render_jobs<false, false, true> : k_render_jobs<false, false, false>);
+                        k<<<blocks, kBatchBlock, 0, chain[pc.second]>>>(ch, checked ? ctx->d_status : nullptr);
                     }
                 } else {
                     std::vector<double> wt(b->jobs.size());

@@ -1,6 +1,6 @@
 // bounce.cu -- the deferred bounce pass (see bounce.cuh): a persistent
-// kernel that traces the queued bounce rays with per-lane refill, and a kernel
-// that shades the pixels whose bounce ray was deferred.
+// kernel that traces the queued bounce rays with per-lane refill and recolours
+// the pixels whose ray leaves.
 #include "bounce.cuh"
 #include "launch.cuh"
 #include "trace_p.cuh"
@@ -11,27 +11,76 @@ namespace {
 
 constexpr int kBounceBlock = 256;
 // a warp takes new rays from the queue once this many of its lanes are idle
-// (tuning bounce_refill; 1, 4, 8, 16, 24 measured on a 4K cave-world frame
-// with the brick-run walk: 8 is fastest)
-constexpr int kRefill = 8;
-// walk iterations a busy lane makes between two refill checks (1, 2, 3, 4, 8
-// measured on the same frame: 2 and 3 are fastest, 4% less bounce time than 1)
-constexpr int kActions = 2;
+// (tuning bounce_refill), and a busy lane makes kActions iterations of the walk
+// between two refill checks: 12 and 3 are fastest of 4-16 and 1-4 with the
+// forward walk (4K cave frame 1145 us; 8 and 2: 1182, 16 and 4: 1146)
+constexpr int kRefill = 12;
+constexpr int kActions = 3;
+
+// The walk of one lane.  Both start a ray (kMore: under way; kHit or kMiss: it
+// is done already) and advance it by one step.
+template <bool FLAT, bool LONG>
+struct Walk;
+
+// Walker::step_flat (one code path for jumps and unit steps).
+template <bool LONG>
+struct Walk<true, LONG> {
+    Walker wk;
+    __device__ __forceinline__ int start(const WorldView& w, const float o[3], const float d[3], int steps) {
+        return wk.start(w, o, d, steps) ? Walker::kMore : Walker::kMiss;
+    }
+    __device__ __forceinline__ int step(const WorldView& w) {
+        TraceHit h;
+        return wk.step_flat<true>(w, w.cdist, h);
+    }
+};
+
+// The forward walk; a ray it does not take (a reciprocal out of its range) is
+// traced to its end by Walker at the start.
+template <bool LONG>
+struct Walk<false, LONG> {
+    FwdWalk fw;
+    __device__ __forceinline__ int start(const WorldView& w, const float o[3], const float d[3], int steps) {
+        PRay r;
+        pray_init(r, o, d);
+        if (ordinary_inv(r.inv)) return fw.start(w, r, steps) ? Walker::kMore : Walker::kMiss;
+        TraceHit h;
+        return trace_fast<false, true, true>(w, w.cdist, r, steps, h) ? Walker::kHit : Walker::kMiss;
+    }
+    __device__ __forceinline__ int step(const WorldView& w) {
+        unsigned wi, vb;
+        return fw.template step<LONG>(w, wi, vb);
+    }
+};
+
+// The record of a pixel whose bounce ray left without a hit: the open colour,
+// and the flags without VT_HIT_BOUNCE (the frame kernel wrote it as a hit).
+__device__ __forceinline__ void open_pixel(uint4* out, unsigned pixel, unsigned rgba) {
+    vt_hit* r = reinterpret_cast<vt_hit*>(out + (pixel & kJobPixel));
+    r->rgba = rgba;
+    r->flags = (uint8_t)(VT_HIT_PRIMARY | ((pixel & kJobShadowed) ? VT_HIT_SHADOWED : 0u) |
+                         ((pixel & kJobEntity) ? VT_HIT_ENTITY : 0u));
+}
 
 // Persistent: every warp loops until the queue is drained.  A lane walks one
-// ray at a time, kActions iterations of the walk per loop turn; open[j] receives 1
-// when ray j leaves without a hit (the sky lights its pixel), 0 otherwise.
-// FLAT: walk with Walker::step_flat (one code path for jumps and unit steps)
-// instead of Walker::step.
-template <bool FLAT>
-__global__ void __launch_bounds__(kBounceBlock) k_bounce_trace(WorldView w, const BounceJob* __restrict__ jobs,
+// ray at a time, kActions iterations of the walk per loop turn.
+// Bound: issue slots (76%) at 12 lanes an instruction, the lanes of a warp
+// being in different phases of unrelated walks; the register cap (4 blocks of
+// 64 registers; uncapped 96) hides the lookups' latency.  7 M rays of a 4K
+// cave frame: 614 us.  Measured slower: setting 32 rays up at a time in shared
+// memory for idle lanes to take (727 us: the copies cost more instructions
+// than the set-ups at few lanes), one code path for jumps and unit steps (568 us
+// here, but 11% slower on a 1021x577 frame whose queue is short).
+template <bool FLAT, bool LONG>
+__global__ void __launch_bounds__(kBounceBlock, 4) k_bounce_trace(WorldView w, const BounceHead* __restrict__ heads,
+                                                               const BounceTail* __restrict__ tails,
                                                                const unsigned* __restrict__ counters,
-                                                               unsigned* __restrict__ next, unsigned char* open,
+                                                               unsigned* __restrict__ next, uint4* __restrict__ out,
                                                                int max_steps, int refill) {
     const unsigned total = counters[0];
     const unsigned lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
-    Walker wk;
+    Walk<FLAT, LONG> wk;
     bool busy = false;
     unsigned job = 0;
     for (;;) {
@@ -44,50 +93,23 @@ __global__ void __launch_bounds__(kBounceBlock) k_bounce_trace(WorldView w, cons
             if (!busy) {
                 job = base + (unsigned)__popc(idle & below);
                 if (job < total) {
-                    const BounceJob J = jobs[job];
-                    busy = wk.start(w, J.o, J.d, max_steps);
-                    if (!busy) open[job] = 1;  // misses the grid or may take no step
+                    const BounceHead H = heads[job];
+                    const BounceTail T = tails[job];
+                    const float d[3] = {H.dx, T.dy, T.dz};
+                    const int s = wk.start(w, H.o, d, max_steps);
+                    busy = s == Walker::kMore;
+                    if (s == Walker::kMiss) open_pixel(out, T.pixel, T.open_rgba);
                 }
             }
         }
         if (busy) {
-            TraceHit h;
             int s = Walker::kMore;
-            for (int a = 0; a < kActions && s == Walker::kMore; ++a)
-                s = FLAT ? wk.step_flat<true>(w, w.cdist, h) : wk.step<false, true, true>(w, w.cdist, h);
+            for (int a = 0; a < kActions && s == Walker::kMore; ++a) s = wk.step(w);
             if (s != Walker::kMore) {
-                open[job] = s == Walker::kHit ? 0 : 1;
+                if (s == Walker::kMiss) open_pixel(out, tails[job].pixel, tails[job].open_rgba);
                 busy = false;
             }
         }
-    }
-}
-
-// One thread per deferred pixel: the shading render_pixel would have done with
-// this bounce result, and the record's rgba and VT_HIT_BOUNCE flag.
-__global__ void __launch_bounds__(kBounceBlock) k_bounce_finish(WorldView w, FrameParams f,
-                                                                const BounceJob* __restrict__ jobs,
-                                                                const unsigned* __restrict__ counters,
-                                                                const unsigned char* __restrict__ open,
-                                                                uint4* __restrict__ out) {
-    const unsigned total = counters[0];
-    for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < total; j += gridDim.x * blockDim.x) {
-        const BounceJob J = jobs[j];
-        const unsigned p = J.pixel;
-        const int px = (int)(p % (unsigned)f.width), py = (int)(p / (unsigned)f.width);
-        const PixelUV uv = f.screen ? table_uv(f, px, py) : pixel_uv(f, px, py);
-        uint4 r = out[p];
-        const unsigned face = r.w & 0xFFu, mat = (r.w >> 8) & 0xFFu;
-        unsigned flags = (r.w >> 16) & 0xFFu;
-        const bool shadowed = (flags & (VT_HIT_SHADOWED | VT_HIT_ENTITY)) != 0u;
-        const bool bounce_open = open[j] != 0;
-        if (!bounce_open) flags |= VT_HIT_BOUNCE;
-        const unsigned alb = __ldg(w.palette + mat);
-        float col[4];
-        shade_hit(f, alb, (int)(face >> 1), (face & 1u) == 0u, shadowed, bounce_open, J.d, col);
-        r.z = f.shade == VT_SHADE_NONE ? alb : composite_uv(f, uv, col);
-        r.w = face | (mat << 8) | (flags << 16);
-        out[p] = r;
     }
 }
 
@@ -96,13 +118,13 @@ __global__ void __launch_bounds__(kBounceBlock) k_bounce_finish(WorldView w, Fra
 vt_status bounce_buffers(vt_ctx* ctx, size_t pixels) {
     if (pixels <= ctx->bounce_capacity) return VT_OK;
     VT_CUDA(ctx, cudaDeviceSynchronize());
-    if (ctx->d_bounce_jobs) vt::dev_free(ctx->d_bounce_jobs);
-    if (ctx->d_bounce_open) vt::dev_free(ctx->d_bounce_open);
-    ctx->d_bounce_jobs = nullptr;
-    ctx->d_bounce_open = nullptr;
+    if (ctx->d_bounce_head) vt::dev_free(ctx->d_bounce_head);
+    if (ctx->d_bounce_tail) vt::dev_free(ctx->d_bounce_tail);
+    ctx->d_bounce_head = nullptr;
+    ctx->d_bounce_tail = nullptr;
     ctx->bounce_capacity = 0;
-    VT_CUDA(ctx, vt::dev_alloc(&ctx->d_bounce_jobs, pixels * sizeof(BounceJob)));
-    VT_CUDA(ctx, vt::dev_alloc(&ctx->d_bounce_open, pixels));
+    VT_CUDA(ctx, vt::dev_alloc(&ctx->d_bounce_head, pixels * sizeof(BounceHead)));
+    VT_CUDA(ctx, vt::dev_alloc(&ctx->d_bounce_tail, pixels * sizeof(BounceTail)));
     if (!ctx->d_bounce_ctr) VT_CUDA(ctx, vt::dev_alloc(&ctx->d_bounce_ctr, 2 * sizeof(unsigned)));
     if (!ctx->ev_bounce) VT_CUDA(ctx, cudaEventCreateWithFlags(&ctx->ev_bounce, cudaEventDisableTiming));
     ctx->bounce_capacity = pixels;
@@ -111,30 +133,24 @@ vt_status bounce_buffers(vt_ctx* ctx, size_t pixels) {
 
 vt_status launch_bounce(vt_ctx* ctx, const vt_world* world, const FrameParams& f, uint4* d_out, cudaStream_t st) {
     const WorldView w = world->view();
-    const int flat = ctx->tuning.bounce_walk == 1 ? 1 : 0;
+    const bool flat = ctx->tuning.bounce_walk == 1, lng = f.bounce_max_steps > kChunkSteps;
     const int refill = ctx->tuning.bounce_refill > 0 ? ctx->tuning.bounce_refill : kRefill;
-    if (ctx->bounce_blocks[flat] == 0) {
+    auto k = flat ? (lng ? k_bounce_trace<true, true> : k_bounce_trace<true, false>)
+                  : (lng ? k_bounce_trace<false, true> : k_bounce_trace<false, false>);
+    const int v = (flat ? 2 : 0) + (lng ? 1 : 0);
+    if (ctx->bounce_blocks[v] == 0) {
         int nb = 0;
-        if (flat) VT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_bounce_trace<true>, kBounceBlock, 0));
-        else VT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_bounce_trace<false>, kBounceBlock, 0));
-        ctx->bounce_blocks[flat] = ctx->sm_count * (nb > 0 ? nb : 1);
+        VT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kBounceBlock, 0));
+        ctx->bounce_blocks[v] = ctx->sm_count * (nb > 0 ? nb : 1);
     }
-    const BounceJob* jobs = reinterpret_cast<const BounceJob*>(ctx->d_bounce_jobs);
     cudaAccessPolicyWindow win_storage;
     const cudaAccessPolicyWindow* win = nullptr;  // L2 window over the brick words (tuning l2_persist)
     vt_status s = l2_policy(ctx, world, &win_storage, &win);
     if (s) return s;
-    if (flat)
-        VT_CUDA(ctx, launch_kernel(k_bounce_trace<true>, dim3(ctx->bounce_blocks[1]), dim3(kBounceBlock), 0, st, win, w,
-                                   jobs, (const unsigned*)ctx->d_bounce_ctr, ctx->d_bounce_ctr + 1, ctx->d_bounce_open,
-                                   f.bounce_max_steps, refill));
-    else
-        VT_CUDA(ctx, launch_kernel(k_bounce_trace<false>, dim3(ctx->bounce_blocks[0]), dim3(kBounceBlock), 0, st, win, w,
-                                   jobs, (const unsigned*)ctx->d_bounce_ctr, ctx->d_bounce_ctr + 1, ctx->d_bounce_open,
-                                   f.bounce_max_steps, refill));
-    k_bounce_finish<<<ctx->sm_count * 8, kBounceBlock, 0, st>>>(w, f, jobs, ctx->d_bounce_ctr, ctx->d_bounce_open,
-                                                                d_out);
-    VT_CUDA(ctx, cudaGetLastError());
+    VT_CUDA(ctx, launch_kernel(k, dim3(ctx->bounce_blocks[v]), dim3(kBounceBlock), 0, st, win, w,
+                               (const BounceHead*)ctx->d_bounce_head, (const BounceTail*)ctx->d_bounce_tail,
+                               (const unsigned*)ctx->d_bounce_ctr, ctx->d_bounce_ctr + 1, d_out, f.bounce_max_steps,
+                               refill));
     // the next deferred frame of this context reuses the queue after this one
     VT_CUDA(ctx, cudaEventRecord(ctx->ev_bounce, st));
     return VT_OK;

@@ -4,31 +4,61 @@
 // warp of neighbouring pixels their lengths differ by an order of magnitude,
 // so a warp tracing one per lane runs for its longest ray while most lanes
 // wait (a step-sequence simulation of a terrain frame puts the useful work at
-// a third of the issued work).  With deferral the frame kernel only appends
-// each hit's bounce ray (origin, direction, pixel) to a queue; a persistent
-// kernel traces the queue with per-lane refill (a lane whose ray ended takes
-// the next queued ray as soon as a quarter of the warp is idle), and a third
-// kernel shades the deferred pixels.  Every ray is walked by the same code as
-// before and the records are identical.  On a 4K frame of the 1 GiB cave
-// world the bounce rays' share of the frame fell from 1.49 to 1.08 ms.
+// a third of the issued work).  With deferral the frame kernel appends each
+// hit's bounce ray (origin, direction, pixel) to a queue, with the pixel's
+// colour if the ray leaves, and writes the record as if it hit (a coherent
+// warp shades both colours for a third of what a pass over the finished pixels
+// cost, 126 us of a 4K frame); a persistent kernel traces the queue with
+// per-lane refill and recolours the pixels whose ray left.  Every ray is
+// walked as in the inline path and the records are identical.
 #pragma once
 
 #include "shade.cuh"
 
 namespace vt {
 
-struct BounceJob {
+// A queued ray, kept as two arrays of 16 bytes so that a warp's appends and
+// reads are whole lines: its origin and the direction's x, then the rest.
+// pixel holds the pixel index (below 2^30) and, above it, whether its sun is
+// blocked by a voxel (kJobShadowed) or by an entity.
+struct __align__(16) BounceHead {
     float o[3];
-    float d[3];
-    unsigned pixel;
-    unsigned pad;
+    float dx;
 };
-static_assert(sizeof(BounceJob) == 32, "bounce job layout");
+struct __align__(16) BounceTail {
+    float dy, dz;
+    unsigned pixel;
+    unsigned open_rgba;   // the pixel's colour if the ray leaves without a hit
+};
+struct BounceJob {
+    BounceHead head;
+    BounceTail tail;
+};
+static_assert(sizeof(BounceHead) == 16 && sizeof(BounceTail) == 16, "bounce job layout");
+constexpr unsigned kJobPixel = (1u << 30) - 1u, kJobShadowed = 1u << 30, kJobEntity = 1u << 31;
+static_assert((unsigned long long)kMaxImageSide * kMaxImageSide <= kJobPixel + 1ull, "pixel index and flags share a word");
+
+__device__ __forceinline__ BounceJob bounce_job(const float o[3], const float d[3], unsigned pixel, unsigned flags,
+                                                unsigned open_rgba) {
+    BounceJob j;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) j.head.o[k] = o[k];
+    j.head.dx = d[0];
+    j.tail.dy = d[1];
+    j.tail.dz = d[2];
+    j.tail.pixel = pixel | ((flags & VT_HIT_SHADOWED) ? kJobShadowed : 0u) | ((flags & VT_HIT_ENTITY) ? kJobEntity : 0u);
+    j.tail.open_rgba = open_rgba;
+    return j;
+}
+
+__device__ __forceinline__ void store_bounce(const FrameParams& f, unsigned slot, const BounceJob& job) {
+    reinterpret_cast<BounceHead*>(f.bounce_head)[slot] = job.head;
+    reinterpret_cast<BounceTail*>(f.bounce_tail)[slot] = job.tail;
+}
 
 // Appends one bounce ray; called by the lanes of a warp that have one, with
 // the warp possibly diverged (one atomic per converged group).
-__device__ __forceinline__ void append_bounce(const FrameParams& f, const float o[3], const float d[3],
-                                              unsigned pixel) {
+__device__ __forceinline__ void append_bounce(const FrameParams& f, const BounceJob& job) {
     const unsigned act = __activemask();
     const unsigned lane = threadIdx.x & 31u;
     const int leader = __ffs(act) - 1;
@@ -36,14 +66,7 @@ __device__ __forceinline__ void append_bounce(const FrameParams& f, const float 
     if ((int)lane == leader) base = atomicAdd(f.bounce_count, (unsigned)__popc(act));
     base = __shfl_sync(act, base, leader);
     const unsigned slot = base + (unsigned)__popc(act & ((1u << lane) - 1u));
-    BounceJob* j = reinterpret_cast<BounceJob*>(f.bounce_jobs) + slot;
-    j->o[0] = o[0];
-    j->o[1] = o[1];
-    j->o[2] = o[2];
-    j->d[0] = d[0];
-    j->d[1] = d[1];
-    j->d[2] = d[2];
-    j->pixel = pixel;
+    store_bounce(f, slot, job);
 }
 
 // ---------------------------------------------------------------------------
@@ -89,16 +112,10 @@ __device__ __forceinline__ unsigned direction_bin(const float d[3]) {
 // Every thread of the block, before any stage_bounce.
 __device__ __forceinline__ void stage_begin() { bounce_stage().bin[threadIdx.x] = kNoBin; }
 
-__device__ __forceinline__ void stage_bounce(const float o[3], const float d[3], unsigned pixel) {
+__device__ __forceinline__ void stage_bounce(const BounceJob& job) {
     BounceStage& st = bounce_stage();
-    BounceJob& j = st.job[threadIdx.x];
-    j.o[0] = o[0];
-    j.o[1] = o[1];
-    j.o[2] = o[2];
-    j.d[0] = d[0];
-    j.d[1] = d[1];
-    j.d[2] = d[2];
-    j.pixel = pixel;
+    st.job[threadIdx.x] = job;
+    const float d[3] = {job.head.dx, job.tail.dy, job.tail.dz};
     st.bin[threadIdx.x] = (unsigned char)direction_bin(d);
 }
 
@@ -135,7 +152,7 @@ __device__ __forceinline__ void stage_flush(const FrameParams& f) {
         if (lane == 31) st.base = total ? atomicAdd(f.bounce_count, total) : 0u;
     }
     __syncthreads();
-    if (b != kNoBin) reinterpret_cast<BounceJob*>(f.bounce_jobs)[st.base + st.hist[b] + rank] = st.job[t];
+    if (b != kNoBin) store_bounce(f, st.base + st.hist[b] + rank, st.job[t]);
 }
 
 }  // namespace vt

@@ -47,7 +47,8 @@ struct BlockTile {
 // SHARE: the lanes of a warp that look up the same brick word share one load
 // (Walker::brick_word).  BIN: deferred bounce rays are appended per block,
 // sorted by direction (stage_flush).
-template <bool STATS, bool CHECKED, bool SMEM, int TW, bool OCC, bool SHARE = false, bool BIN = false>
+template <bool STATS, bool CHECKED, bool SMEM, int TW, bool OCC, bool SHARE = false, bool BIN = false, bool BOUNCE = true,
+          bool LONG = true>
 __global__ void __launch_bounds__(kBlock, OCC ? kOccBlocks : 1) k_render(WorldView w, FrameParams f, uint4* __restrict__ out,
                                                                unsigned* status, unsigned long long* counters) {
     // shared copy of the coarse bits for the model traversal (STATS or
@@ -94,7 +95,7 @@ __global__ void __launch_bounds__(kBlock, OCC ? kOccBlocks : 1) k_render(WorldVi
         }
         uint4 rec;
         if (SMEM) rec = render_pixel<STATS, CHECKED>(w, CoarseShared{s_coarse}, w.cdist, f, px, py, uv, status, pc);
-        else rec = render_pixel<STATS, CHECKED, CoarseGlobal, SHARE, BIN>(w, CoarseGlobal{w.coarse}, w.cdist, f, px,
+        else rec = render_pixel<STATS, CHECKED, CoarseGlobal, SHARE, BIN, BOUNCE, LONG>(w, CoarseGlobal{w.coarse}, w.cdist, f, px,
                                                                           py, uv, status, pc);
         out[(size_t)py * f.width + px] = rec;
     }
@@ -103,10 +104,10 @@ __global__ void __launch_bounds__(kBlock, OCC ? kOccBlocks : 1) k_render(WorldVi
 }
 
 // Explicit ray list (production traversal); record.rgba is 0.
-template <bool CHECKED>
+template <bool LONG>
 __global__ void __launch_bounds__(kBlock) k_trace_rays(WorldView w, const float* __restrict__ origins,
                                                        const float* __restrict__ dirs, int n, int max_steps,
-                                                       uint4* __restrict__ out, unsigned* status) {
+                                                       uint4* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float o[3], d[3];
@@ -118,8 +119,7 @@ __global__ void __launch_bounds__(kBlock) k_trace_rays(WorldView w, const float*
     PRay r;
     pray_init(r, o, d);
     TraceHit h;
-    TraceCounters cnt;
-    const bool hit = near_origin(r.o) ? trace_fast<true, true, true>(w, w.cdist, r, max_steps, h)
+    const bool hit = near_origin(r.o) ? trace_fast<true, true, true, false, LONG>(w, w.cdist, r, max_steps, h)
                                       : trace_fast<true, true, false>(w, w.cdist, r, max_steps, h);
     if (hit) {
         const int e = h.axis;
@@ -302,7 +302,8 @@ FrameParams make_frame(const vt_camera* cam, const vt_params* p) {
     f.height = cam->height;
     f.row0 = 0;
     f.row_end = cam->height;
-    f.bounce_jobs = nullptr;
+    f.bounce_head = nullptr;
+    f.bounce_tail = nullptr;
     f.bounce_count = nullptr;
     f.screen = nullptr;
     f.max_steps = p->max_steps;
@@ -460,7 +461,8 @@ vt_status launch_render(vt_ctx* ctx, const vt_world* world, const vt_camera* cam
         if (s) return s;
         VT_CUDA(ctx, cudaStreamWaitEvent(stream, ctx->ev_bounce, 0));
         VT_CUDA(ctx, cudaMemsetAsync(ctx->d_bounce_ctr, 0, 2 * sizeof(unsigned), stream));
-        f.bounce_jobs = ctx->d_bounce_jobs;
+        f.bounce_head = ctx->d_bounce_head;
+        f.bounce_tail = ctx->d_bounce_tail;
         f.bounce_count = ctx->d_bounce_ctr;
     }
     cudaError_t le = cudaSuccess;
@@ -492,7 +494,16 @@ vt_status launch_render(vt_ctx* ctx, const vt_world* world, const vt_camera* cam
                                               (rows + BlockTile<8>::kH - 1) / BlockTile<8>::kH),
                                          dim3(kBlock), sm, stream, win, w, f, d_out, ctx->d_status, ctx->d_counters); }
         else if (tu.occupancy && tu.share_bricks) { VT_LAUNCH_X(false, false, false, 8, true, true); }
-        else if (tu.occupancy) { VT_LAUNCH(false, false, false, 8, true); }
+        else if (tu.occupancy) {
+            const bool bounce = (p->rays & VT_RAYS_BOUNCE) != 0, lng = long_steps(f);
+            auto k = bounce ? (lng ? k_render<false, false, false, 8, true, false, false, true, true>
+                                   : k_render<false, false, false, 8, true, false, false, true, false>)
+                            : (lng ? k_render<false, false, false, 8, true, false, false, false, true>
+                                   : k_render<false, false, false, 8, true, false, false, false, false>);
+            le = launch_kernel(k, dim3((cam->width + BlockTile<8>::kW - 1) / BlockTile<8>::kW,
+                                       (rows + BlockTile<8>::kH - 1) / BlockTile<8>::kH),
+                               dim3(kBlock), sm, stream, win, w, f, d_out, ctx->d_status, ctx->d_counters);
+        }
         else { VT_LAUNCH(false, false, false, 8, false); }
     }
 #undef VT_LAUNCH_M
@@ -643,8 +654,9 @@ vt_status vt_trace_rays(vt_ctx* ctx, const vt_world* world, const float* d_origi
         if (s) return s;
     }
     const WorldView w = world->view();
-    k_trace_rays<true><<<(n + kBlock - 1) / kBlock, kBlock, 0, (cudaStream_t)stream>>>(
-        w, d_origins, d_dirs, n, max_steps, reinterpret_cast<uint4*>(d_out), ctx->d_status);
+    (max_steps > kChunkSteps ? k_trace_rays<true> : k_trace_rays<false>)<<<(n + kBlock - 1) / kBlock, kBlock, 0,
+                                                                            (cudaStream_t)stream>>>(
+        w, d_origins, d_dirs, n, max_steps, reinterpret_cast<uint4*>(d_out));
     VT_CUDA(ctx, cudaGetLastError());
     return note_status_writer(ctx, (cudaStream_t)stream);
 }

@@ -9,6 +9,12 @@
 
 namespace vt {
 
+// Whether some ray kind of the frame may walk far enough for chunk jumps to
+// pay.
+inline bool long_steps(const FrameParams& f) {
+    return f.max_steps > kChunkSteps || f.shadow_max_steps > kChunkSteps || f.bounce_max_steps > kChunkSteps;
+}
+
 struct PixelCounters {
     unsigned v[kNumCounters];
 };
@@ -19,20 +25,24 @@ struct PixelCounters {
 // NEAR: the caller knows the origin passes near_origin (secondary rays start
 // on a hit inside the grid); otherwise the primary ray checks it once.
 // SHARE: brick words shared between the lanes of a warp (Walker::brick_word).
-template <bool STATS, bool CHECKED, bool MAT, bool NEAR, bool SHARE, class Coarse>
+template <bool STATS, bool CHECKED, bool MAT, bool NEAR, bool SHARE, bool LONG, class Coarse>
 __device__ __forceinline__ bool trace_any(const WorldView& w, const Coarse& coarse, const unsigned char* cd,
                                           const PRay& r, int max_steps, TraceHit& h, TraceCounters& cnt,
                                           unsigned* status) {
     if (STATS || CHECKED) return trace_p<STATS, CHECKED, MAT>(w, coarse, r, max_steps, h, cnt, status);
-    if (NEAR || near_origin(r.o)) return trace_fast<MAT, true, true, SHARE>(w, cd, r, max_steps, h);
-    return trace_fast<MAT, true, false, SHARE>(w, cd, r, max_steps, h);
+    if (NEAR || near_origin(r.o)) return trace_fast<MAT, true, true, SHARE, LONG>(w, cd, r, max_steps, h);
+    return trace_fast<MAT, true, false, SHARE, LONG>(w, cd, r, max_steps, h);
 }
 
 // uv: the pixel's screen coordinates (pixel_uv(f, px, py); the frame kernel
 // reads them from the frame's screen table or its per-block tables).
 // BIN: a deferred bounce ray is staged in the block's shared memory for the
 // block's direction-sorted append (stage_flush) instead of appended at once.
-template <bool STATS, bool CHECKED, class Coarse, bool SHARE = false, bool BIN = false>
+// BOUNCE: false leaves the bounce rays' code out (frames without them: the
+// kernel's registers and code then serve the walk alone).  LONG: a ray kind's
+// step limit is above kChunkSteps (trace_fast).
+template <bool STATS, bool CHECKED, class Coarse, bool SHARE = false, bool BIN = false, bool BOUNCE = true,
+          bool LONG = true>
 __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& coarse, const unsigned char* cd,
                                               const FrameParams& f, int px, int py, const PixelUV& uv,
                                               unsigned* status, PixelCounters& pc) {
@@ -42,7 +52,7 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
     pray_init(r, o, d);
     TraceHit h;
     TraceCounters cnt;
-    const bool hit = trace_any<STATS, CHECKED, true, false, SHARE>(w, coarse, cd, r, f.max_steps, h, cnt, status);
+    const bool hit = trace_any<STATS, CHECKED, true, false, SHARE, LONG>(w, coarse, cd, r, f.max_steps, h, cnt, status);
     if (STATS) {
         pc.v[0] += 1;
         pc.v[9] += 16;
@@ -75,7 +85,7 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
             PRay rs;
             pray_init_dir(rs, so, f.sun_d, f.sun_inv);
             TraceHit hs;
-            shadowed = trace_any<STATS, CHECKED, false, true, SHARE>(w, coarse, cd, rs, f.shadow_max_steps, hs, cnt, status);
+            shadowed = trace_any<STATS, CHECKED, false, true, SHARE, LONG>(w, coarse, cd, rs, f.shadow_max_steps, hs, cnt, status);
             if (shadowed) flags |= VT_HIT_SHADOWED;
             if (STATS) {
                 pc.v[2] += 1;
@@ -89,20 +99,25 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
         bool bounce_open = false;
         bool deferred = false;
         float bdir[3] = {0.0f, 0.0f, 0.0f};
-        if (f.rays & VT_RAYS_BOUNCE) {
+        if (BOUNCE && (f.rays & VT_RAYS_BOUNCE)) {
             unsigned seed = ((unsigned)px * 1973u + (unsigned)py * 9277u) ^ f.seed;
             cosine_hemisphere(nrm, seed, bdir);
-            deferred = !STATS && !CHECKED && f.bounce_jobs != nullptr;
+            deferred = !STATS && !CHECKED && f.bounce_head != nullptr;
         }
         if (deferred) {
-            // traced and shaded by the bounce kernels (bounce.cu)
-            if (BIN) stage_bounce(so, bdir, (unsigned)py * (unsigned)f.width + (unsigned)px);
-            else append_bounce(f, so, bdir, (unsigned)py * (unsigned)f.width + (unsigned)px);
-        } else if (f.rays & VT_RAYS_BOUNCE) {
+            // traced by the bounce kernel (bounce.cu).  The record assumes a
+            // hit; a ray that leaves turns it into the open colour
+            shade_hit(f, alb, e, pe, shadowed, true, bdir, col);
+            const unsigned open = f.shade == VT_SHADE_NONE ? alb : composite_uv(f, uv, col);
+            const BounceJob job = bounce_job(so, bdir, (unsigned)py * (unsigned)f.width + (unsigned)px, flags, open);
+            if (BIN) stage_bounce(job);
+            else append_bounce(f, job);
+            flags |= VT_HIT_BOUNCE;
+        } else if (BOUNCE && (f.rays & VT_RAYS_BOUNCE)) {
             PRay rb;
             pray_init(rb, so, bdir);
             TraceHit hb;
-            const bool bh = trace_any<STATS, CHECKED, false, true, SHARE>(w, coarse, cd, rb, f.bounce_max_steps, hb, cnt, status);
+            const bool bh = trace_any<STATS, CHECKED, false, true, SHARE, LONG>(w, coarse, cd, rb, f.bounce_max_steps, hb, cnt, status);
             if (bh) flags |= VT_HIT_BOUNCE;
             bounce_open = !bh;
             if (STATS) {
@@ -110,12 +125,8 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
                 pc.v[5] += bh ? 1u : 0u;
             }
         }
-        if (deferred) {
-            rgba = 0u;
-        } else {
-            shade_hit(f, alb, e, pe, shadowed, bounce_open, bdir, col);
-            rgba = f.shade == VT_SHADE_NONE ? alb : composite_uv(f, uv, col);
-        }
+        shade_hit(f, alb, e, pe, shadowed, bounce_open, bdir, col);
+        rgba = f.shade == VT_SHADE_NONE ? alb : composite_uv(f, uv, col);
     } else {
         shade_miss(f, d, col);
         rgba = f.shade == VT_SHADE_NONE ? 0u : composite_uv(f, uv, col);

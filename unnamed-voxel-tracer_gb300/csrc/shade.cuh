@@ -35,7 +35,8 @@ struct FrameParams {
     float sun_inv[3];   // its correctly rounded reciprocal
     float cross_r2;     // the largest x with sqrt(x) <= 0.002 (crosshair radius test without a square root)
     int row0, row_end;  // rows [row0, row_end) of the image this launch renders
-    void* bounce_jobs;       // non-null: bounce rays are queued here (BounceJob), not traced inline
+    void* bounce_head;       // non-null: bounce rays are queued here (BounceHead), not traced inline
+    void* bounce_tail;       // and here (BounceTail)
     unsigned* bounce_count;  // the queue's length
     const float4* screen;    // the frame's screen table (ScreenTable), or null: computed per block
 };

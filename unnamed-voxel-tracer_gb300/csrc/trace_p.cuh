@@ -672,7 +672,7 @@ struct Walker {
 // Bound: compares, selects and integer logic share one half-rate pipe, which
 // bounds the frame kernel with the issue slots; adds and fused multiply-adds
 // do not use it, hence the arithmetic on magic floats.  1080p terrain frame,
-// primary + shadow: 166 -> 108 us, 3.04 G thread instructions at 30.3 lanes
+// primary + shadow: 168 -> 109 us, 3.05 G thread instructions at 30.3 lanes
 // (Walker: 27.4), 40 M of 100 M warp instructions on that pipe.
 constexpr float kMagic = 12582912.0f;    // 1.5 * 2^23: float spacing 1, and integers of either sign around it
 constexpr float kMagic4 = 50331648.0f;   // 1.5 * 2^25: the same with spacing 4
@@ -713,12 +713,12 @@ __device__ __forceinline__ float magic_brick(float n) {
 #endif
 }
 
-// Step limits above this walk with chunk jumps.  A brick jump already crosses
-// up to 66 cells, and a chunk jump has to cross more (distance 3 or above)
-// to pay for its lookup: with limits of 512 the walk without them is faster
-// (1080p frames equal, 16-scene batch 1361 against 1405 us, a million
-// unrelated rays 78 against 80 us); a walk of thousands of empty cells needs
-// up to 7 times fewer jumps with them.
+// Kernels whose rays have a step limit above this are compiled with chunk
+// jumps.  A brick jump already crosses up to 66 cells, and a chunk jump has to
+// cross more (distance 3 or above) to pay for its lookup: with limits of 512
+// the walk without them is faster (1080p frame 109 against 111 us, 16-scene
+// batch 1318 against 1343 us); a walk of thousands of empty cells needs up to
+// 7 times fewer jumps with them.
 constexpr int kChunkSteps = 1024;
 
 // A ray the forward walk takes: near origin, and reciprocals in
@@ -764,7 +764,7 @@ struct FwdWalk {
         // no walk makes 2^20 crossings, and sums stay exact below 2^24
         limit = ((nk[0] + nk[1]) + nk[2]) + __int2float_rn(min(steps, 1 << 20));
         flip = (unsigned)((m[0] & 3) | (m[1] & 12) | (m[2] & 48) | (box ? 64 : 0));
-        field = ((r.pos[0] ? 1u : 0u) | (r.pos[1] ? 2u : 0u) | (r.pos[2] ? 4u : 0u)) * w.nwords;
+        field = (unsigned)((~m[0] & 1) | (~m[1] & 2) | (~m[2] & 4)) * w.nwords;
         return true;
     }
 
@@ -898,8 +898,9 @@ struct FwdWalk {
 };
 
 // Traces one ray to its end.  NEAR: the origin passes near_origin; SHARE:
-// brick words shared between the lanes of a warp (Walker only).
-template <bool MAT, bool RUN = true, bool NEAR = false, bool SHARE = false>
+// brick words shared between the lanes of a warp (Walker only); LONG: step
+// limits above kChunkSteps (chunk jumps; without them only speed is lost).
+template <bool MAT, bool RUN = true, bool NEAR = false, bool SHARE = false, bool LONG = true>
 __device__ __forceinline__ bool trace_fast(const WorldView& w, const unsigned char* cdist, const PRay& r,
                                            int max_steps, TraceHit& h) {
     int s;
@@ -907,12 +908,7 @@ __device__ __forceinline__ bool trace_fast(const WorldView& w, const unsigned ch
         FwdWalk fw;
         if (!fw.start(w, r, max_steps)) return false;
         unsigned wi = 0, vb = 0;
-        if (max_steps > kChunkSteps) {
-            while ((s = fw.step<true>(w, wi, vb)) == FwdWalk::kMore) {
-            }
-        } else {
-            while ((s = fw.step<false>(w, wi, vb)) == FwdWalk::kMore) {
-            }
+        while ((s = fw.step<LONG>(w, wi, vb)) == FwdWalk::kMore) {
         }
         if (s != FwdWalk::kHit) return false;
         fw.hit<MAT>(w, r, wi, vb, h);

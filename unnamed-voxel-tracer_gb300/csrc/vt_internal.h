@@ -132,16 +132,16 @@ struct vt_ctx {
     // it dirty and record ev_status; while it is clean vt_sync need not read it
     bool status_dirty = false;
     cudaEvent_t ev_status = nullptr;
-    // the deferred bounce pass (bounce.cu): ray queue, results, counters
-    void* d_bounce_jobs = nullptr;
-    unsigned char* d_bounce_open = nullptr;
+    // the deferred bounce pass (bounce.cu): ray queue, counters
+    void* d_bounce_head = nullptr;
+    void* d_bounce_tail = nullptr;
     unsigned* d_bounce_ctr = nullptr;  // {queued, taken}
     size_t bounce_capacity = 0;
     cudaEvent_t ev_bounce = nullptr;   // the last deferred frame is done with the queue
     // screen tables of the frame sizes rendered so far (see screen_table)
     vt::ScreenTable screen[vt::kScreenTables];
     int n_screen = 0;
-    int bounce_blocks[2] = {0, 0};     // resident blocks of the bounce walk kernels (brick-run, one-path)
+    int bounce_blocks[4] = {0, 0, 0, 0};  // resident blocks of the bounce walk kernels (brick-run, one-path; short, long step limits)
 };
 
 namespace vt {
