@@ -39,7 +39,7 @@ __device__ __forceinline__ void center_ray(const PickRay& f, float o[3], float d
 // edit_mode < 0: pick only; 0: clear the hit voxel; 1..255: write material
 // edit_mode into the cell in front of the hit face (skipped outside the
 // world).  `out` (may be null) receives the pick as a vt_hit record; d_edit
-// receives {x, y, z, valid} of the voxel written.
+// receives {x, y, z, valid, whether a coarse bit changed} of the voxel written.
 __global__ void __launch_bounds__(512) k_pick_edit(WorldView w, unsigned long long* mask, unsigned char* mats,
                                                    unsigned long long* coarse, PickRay f, int max_steps, int edit_mode,
                                                    uint4* __restrict__ out, int* __restrict__ d_edit) {
@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(512) k_pick_edit(WorldView w, unsigned long lo
             d_edit[1] = target[1];
             d_edit[2] = target[2];
             d_edit[3] = target[3];
+            d_edit[4] = 0;
         }
     }
     __syncthreads();
@@ -93,8 +94,8 @@ __global__ void __launch_bounds__(512) k_pick_edit(WorldView w, unsigned long lo
     const int any = __syncthreads_or(mask[ci * 512u + threadIdx.x] != 0ull);
     if (threadIdx.x == 0) {
         const unsigned long long bit = 1ull << (ci & 63u);
-        if (any) atomicOr(coarse + (ci >> 6), bit);
-        else atomicAnd(coarse + (ci >> 6), ~bit);
+        const unsigned long long was = any ? atomicOr(coarse + (ci >> 6), bit) : atomicAnd(coarse + (ci >> 6), ~bit);
+        d_edit[4] = ((was & bit) != 0ull) != (any != 0) ? 1 : 0;   // the chunk distances are stale
     }
 }
 

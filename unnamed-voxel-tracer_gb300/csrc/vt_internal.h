@@ -164,7 +164,7 @@ struct vt_world {
     unsigned char* d_cdist = nullptr;
     unsigned char* d_dtmp = nullptr;   // x (2 fields, 16 B/brick) and y (10 fields, 4 B/brick) pass results of the brick distances (kept)
     unsigned char* d_ctmp = nullptr;   // the same 6 fields for the chunk distances
-    int* d_edit = nullptr;             // {x, y, z, valid} of the last device-side edit
+    int* d_edit = nullptr;             // {x, y, z, valid, coarse bit changed} of the last device-side edit
     float* d_entities = nullptr;       // kMaxEntities boxes of 6 floats
     int n_entities = 0;
     bool dist_dirty = true;            // distances rebuilt before the next render

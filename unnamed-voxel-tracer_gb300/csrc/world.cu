@@ -10,6 +10,8 @@
 //              b = bx + 8*(by + 8*bz), voxel v = x + 4*(y + 4*z) in the brick
 //   mask       one u64 per brick, bit v set iff material != 0
 //   coarse     one bit per chunk, set iff any brick word of the chunk is != 0
+#include <cuda_fp16.h>
+
 #include <algorithm>
 #include <cstring>
 
@@ -99,29 +101,36 @@ __global__ void __launch_bounds__(512) k_set_voxel(WorldView w, unsigned long lo
 // the direction of axis i (1: +) for axes 0..axis; the pass reads input field
 // v & ((1 << axis) - 1) (pass 0 reads the coarse bits instead).  Fields are
 // `stride` bytes apart.  The pass covers the whole chunk grid.
+// The window's reads are independent and all in flight at once.  d_changed
+// (null: always run): the pass is skipped when it points to 0, a device-side
+// edit that left every coarse bit as it was.
 __global__ void k_dist_pass(const unsigned long long* __restrict__ coarse, const unsigned char* __restrict__ in,
-                            unsigned char* __restrict__ out, int axis, int CX, int CY, int CZ, size_t stride) {
+                            unsigned char* __restrict__ out, int axis, int CX, int CY, int CZ, size_t stride,
+                            const int* __restrict__ d_changed) {
+    if (d_changed && !*d_changed) return;
     const unsigned v = blockIdx.y;
     const bool fwd = ((v >> axis) & 1u) != 0u;
     if (axis > 0) in += (size_t)(v & ((1u << axis) - 1u)) * stride;
     out += (size_t)v * stride;
-    const int dlo = fwd ? 0 : -kDistCap, dhi = fwd ? kDistCap : 0;
-    const int g[3] = {CX, CY, CZ};
-    const size_t total = (size_t)CX * CY * CZ;
-    for (size_t lin = blockIdx.x * (size_t)blockDim.x + threadIdx.x; lin < total; lin += (size_t)gridDim.x * blockDim.x) {
-        int p[3] = {(int)(lin % CX), (int)((lin / CX) % CY), (int)(lin / ((size_t)CX * CY))};
-        const int u = p[axis];
-        int best = kDistCap + 1;
-        for (int dd = dlo; dd <= dhi; ++dd) {
-            const int q = u + dd;
-            if (q < 0 || q >= g[axis]) continue;
-            p[axis] = q;
-            const unsigned idx = (unsigned)p[0] + (unsigned)CX * ((unsigned)p[1] + (unsigned)CY * (unsigned)p[2]);
-            const int val = axis == 0 ? (((coarse[idx >> 6] >> (idx & 63u)) & 1ull) ? 0 : kDistCap + 1) : (int)in[idx];
-            best = min(best, max(abs(dd), val));
+    const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
+    if (lin >= (unsigned)CX * (unsigned)CY * (unsigned)CZ) return;
+    const unsigned p[3] = {lin % (unsigned)CX, (lin / (unsigned)CX) % (unsigned)CY, lin / ((unsigned)CX * (unsigned)CY)};
+    const int u = (int)(axis == 0 ? p[0] : (axis == 1 ? p[1] : p[2])), g = axis == 0 ? CX : (axis == 1 ? CY : CZ);
+    const int step = (axis == 0 ? 1 : (axis == 1 ? CX : CX * CY)) * (fwd ? 1 : -1);
+    int val[kDistCap + 1];
+#pragma unroll
+    for (int d = 0; d <= kDistCap; ++d) {
+        const int q = fwd ? u + d : u - d;
+        val[d] = kDistCap + 1;
+        if (q >= 0 && q < g) {
+            const unsigned idx = (unsigned)((int)lin + d * step);
+            val[d] = axis == 0 ? (((__ldg(coarse + (idx >> 6)) >> (idx & 63u)) & 1ull) ? 0 : kDistCap + 1) : (int)__ldg(in + idx);
         }
-        out[lin] = (unsigned char)best;
     }
+    int best = kDistCap + 1;
+#pragma unroll
+    for (int d = 0; d <= kDistCap; ++d) best = min(best, max(d, val[d]));
+    out[lin] = (unsigned char)best;
 }
 
 // Brick level, in voxels.  With vertical weight w = 2^shape, brick b has
@@ -142,10 +151,19 @@ __global__ void k_dist_pass(const unsigned long long* __restrict__ coarse, const
 //      the shape choice.
 // The intermediates are x-fastest arrays: X over (GX bricks, GY*4, GZ*4
 // voxels), Y over (GX, GY bricks, GZ*4 voxels).  Each pass covers a box of
-// its own output grid, [lo, lo + ext) clipped to the grid; with `d_cell`
-// ({x, y, z, valid} of an edited voxel in device memory) the box is taken
-// relative to that voxel's brick (brick axes) or the brick's first voxel
-// (voxel axes), and skipped when !valid.
+// its own output grid, [lo, lo + ext) clipped to the grid (and widened in x to
+// whole chunks or groups of four bricks: recomputing a cell that cannot have
+// changed gives the value it has); with `d_cell` ({x, y, z, valid, coarse bit
+// changed} of an edited voxel in device memory) the box is taken relative to that voxel's brick
+// (brick axes) or the brick's first voxel (voxel axes), and skipped when
+// !valid.
+//
+// Bound: the passes are scans over L2-resident bytes.  One byte per thread and
+// step was bound by instruction issue (512x256x512 cave world: x 485, y 1111,
+// z 804 us).  The x pass now finds first voxels with bit scans of 32-voxel row
+// words, and the y and z passes scan four bricks at a time (one 32-bit load,
+// 16-bit pair minima and maxima), the four shapes of a downward field in one
+// scan: x 42, y 108, z 126 us.
 __device__ __forceinline__ unsigned brick_index(int bx, int by, int bz, int CX, int CY) {
     const unsigned ci = (unsigned)(bx >> 3) + (unsigned)CX * ((unsigned)(by >> 3) + (unsigned)CY * (unsigned)(bz >> 3));
     return ci * 512u + (unsigned)((bx & 7) | ((by & 7) << 3) | ((bz & 7) << 6));
@@ -161,13 +179,6 @@ struct BrickGrid {
 constexpr int kYFields = 2 + 2 * kBoxShapes;
 __host__ __device__ constexpr int y_field(int xs, int ys, int shape) { return ys ? xs : 2 + xs + 2 * shape; }
 
-__device__ __forceinline__ bool box_cell(size_t lin, int3 lo, int3 ext, int3 g, int& x, int& y, int& z) {
-    x = lo.x + (int)(lin % ext.x);
-    y = lo.y + (int)((lin / ext.x) % ext.y);
-    z = lo.z + (int)(lin / ((size_t)ext.x * ext.y));
-    return x >= 0 && y >= 0 && z >= 0 && x < g.x && y < g.y && z < g.z;
-}
-
 __device__ __forceinline__ int3 edit_origin(int3 lo, const int* d_cell, bool vx, bool vy, bool vz) {
     const int bx = d_cell[0] >> 2, by = d_cell[1] >> 2, bz = d_cell[2] >> 2;
     lo.x += vx ? 4 * bx : bx;
@@ -176,127 +187,272 @@ __device__ __forceinline__ int3 edit_origin(int3 lo, const int* d_cell, bool vx,
     return lo;
 }
 
+// Item `lin` of the box [lo, lo + ext) whose x axis counts groups of `group`
+// bricks (the ones that meet the box): its coordinates, x in groups.  False
+// past the box or the grid.
+__device__ __forceinline__ bool box_item(unsigned lin, int3 lo, int3 ext, int group, int3 g, int& x, int& y, int& z) {
+    const int x0 = max(lo.x, 0) / group, nx = (lo.x + ext.x - 1) / group - x0 + 1;
+    if (lo.x + ext.x <= 0 || nx <= 0) return false;
+    x = x0 + (int)(lin % (unsigned)nx);
+    const unsigned r = lin / (unsigned)nx;
+    y = lo.y + (int)(r % (unsigned)ext.y);
+    const unsigned rz = r / (unsigned)ext.y;
+    if (rz >= (unsigned)ext.z) return false;
+    z = lo.z + (int)rz;
+    return y >= 0 && z >= 0 && x * group < g.x && y < g.y && z < g.z;
+}
+
+// One thread: the 8 bricks of a chunk on the 4 voxel rows of brick row by in
+// layer qz, both directions.  A row of a chunk is one 32-bit word; the first
+// voxel ahead lies in it or in the next two (64 layers, the cap is 63).
 __global__ void k_bdist_x(const unsigned long long* __restrict__ mask, unsigned char* __restrict__ xf, BrickGrid b,
                           int3 lo, int3 ext, const int* __restrict__ d_cell) {
     if (d_cell) {
         if (!d_cell[3]) return;
-        lo = edit_origin(lo, d_cell, false, true, true);
+        lo = edit_origin(lo, d_cell, false, false, true);
     }
-    const bool fwd = blockIdx.y != 0;
-    const int3 g = make_int3(b.GX, b.GY * 4, b.GZ * 4);
-    const size_t fsize = (size_t)g.x * g.y * g.z;
-    xf += blockIdx.y * fsize;
-    const size_t total = (size_t)ext.x * ext.y * ext.z;
-    for (size_t lin = blockIdx.x * (size_t)blockDim.x + threadIdx.x; lin < total; lin += (size_t)gridDim.x * blockDim.x) {
-        int bx, qy, qz;
-        if (!box_cell(lin, lo, ext, g, bx, qy, qz)) continue;
-        const unsigned row = 4u * (unsigned)(qy & 3) + 16u * (unsigned)(qz & 3);
-        int best = kVoxCap + 1;
-        for (int j = 0;; ++j) {
-            const int nb = fwd ? bx + j : bx - j;
-            // a voxel of brick nb lies at least 4j - 3 layers beyond bx's far face
-            if (max(0, 4 * j - 3) >= best || nb < 0 || nb >= g.x) break;
-            const unsigned bits = (unsigned)(mask[brick_index(nb, qy >> 2, qz >> 2, b.CX, b.CY)] >> row) & 15u;
-            if (bits) {
-                best = fwd ? max(0, 4 * j + (__ffs(bits) - 1) - 3) : max(0, 4 * j - (31 - __clz(bits)));
-                break;
-            }
+    int cx, by, qz;
+    if (!box_item(blockIdx.x * blockDim.x + threadIdx.x, lo, ext, 8, make_int3(b.GX, b.GY, b.GZ * 4), cx, by, qz)) return;
+    // r[k][y]: row y of chunk cx - 2 + k
+    unsigned r[5][4];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+#pragma unroll
+        for (int y = 0; y < 4; ++y) r[k][y] = 0u;
+        const int c = cx - 2 + k;
+        if (c < 0 || c >= b.CX) continue;
+        const unsigned short* w = reinterpret_cast<const unsigned short*>(mask + brick_index(8 * c, by, qz >> 2, b.CX, b.CY)) + (qz & 3);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const unsigned v = __ldg(w + 4 * i);   // 16 voxels of brick i: 4 rows of 4
+#pragma unroll
+            for (int y = 0; y < 4; ++y) r[k][y] |= ((v >> (4 * y)) & 15u) << (4 * i);
         }
-        xf[(size_t)bx + (size_t)g.x * ((size_t)qy + (size_t)g.y * qz)] = (unsigned char)min(best, kVoxCap + 1);
+    }
+    const size_t fsize = (size_t)b.GX * (b.GY * 4) * (b.GZ * 4);
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+        unsigned char* row = xf + (size_t)(8 * cx) + (size_t)b.GX * ((size_t)(4 * by + y) + (size_t)(b.GY * 4) * qz);
+        unsigned out[2][2] = {{0u, 0u}, {0u, 0u}};
+        const unsigned own = r[2][y];
+        // layers from the chunk's far face to the first voxel of the next two
+        const unsigned ahead = r[3][y] ? (unsigned)__ffs(r[3][y]) : (r[4][y] ? 32u + (unsigned)__ffs(r[4][y]) : 64u);
+        const unsigned behind = r[1][y] ? 1u + (unsigned)__clz(r[1][y]) : (r[0][y] ? 33u + (unsigned)__clz(r[0][y]) : 64u);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const bool occ = ((own >> (4 * i)) & 15u) != 0u;
+            const unsigned up = i < 7 ? own >> (4 * i + 4) : 0u, down = own & ((1u << (4 * i)) - 1u);
+            unsigned f = up ? (unsigned)__ffs(up) : (unsigned)(28 - 4 * i) + ahead;
+            unsigned n = down ? (unsigned)(4 * i - 31) + (unsigned)__clz(down) : (unsigned)(4 * i) + behind;
+            f = occ ? 0u : min(f, (unsigned)(kVoxCap + 1));
+            n = occ ? 0u : min(n, (unsigned)(kVoxCap + 1));
+            out[0][i >> 2] |= n << (8 * (i & 3));
+            out[1][i >> 2] |= f << (8 * (i & 3));
+        }
+        *reinterpret_cast<uint2*>(row) = make_uint2(out[0][0], out[0][1]);
+        *reinterpret_cast<uint2*>(row + fsize) = make_uint2(out[1][0], out[1][1]);
     }
 }
 
+// Four bytes (at most 63) as two pairs of 16-bit values with the byte on top:
+// bytes 1 and 3 in place, bytes 0 and 2 shifted up.  What lies below the byte
+// only breaks ties.  Such values are positive finite halves, whose order is
+// that of their bits, so the half-precision pair minimum and maximum (one
+// instruction each) apply.
+struct Quad {
+    unsigned odd, even;
+};
+__device__ __forceinline__ unsigned pair_min(unsigned a, unsigned b) {
+    const __half2 r = __hmin2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
+    return *reinterpret_cast<const unsigned*>(&r);
+}
+__device__ __forceinline__ unsigned pair_max(unsigned a, unsigned b) {
+    const __half2 r = __hmax2(*reinterpret_cast<__half2*>(&a), *reinterpret_cast<__half2*>(&b));
+    return *reinterpret_cast<const unsigned*>(&r);
+}
+__device__ __forceinline__ unsigned quad_bytes(Quad q) { return (q.odd & 0xFF00FF00u) | ((q.even >> 8) & 0x00FF00FFu); }
+// best = min(best, max(dist, v)) in each byte; d2: dist in both pair bytes.
+__device__ __forceinline__ void quad_take(Quad& best, unsigned v, unsigned d2) {
+    best.odd = pair_min(best.odd, pair_max(v, d2));
+    best.even = pair_min(best.even, pair_max(v * 256u, d2));
+}
+// The largest of the four.
+__device__ __forceinline__ unsigned quad_max(Quad q) {
+    const unsigned m = pair_max(q.odd, q.even);
+    return max(m & 0xFFFFu, m >> 16) >> 8;
+}
+
+// Scans the layers ahead of a brick, four bricks at a time: NF input fields f,
+// `step` bytes from one layer to the next, layers 0..3 the brick's own, `count`
+// (a multiple of 4) in the grid.  Result k of a field: min over layers of
+// max(distance << k, byte), k < NW (NF or NW is 1).  Four layers are in
+// flight; a layer whose distance reaches every best cannot lower one, and with
+// weight 2^k the distances end at layer 3 + 62 / 2^k.  PREFETCH: the next four
+// are on their way before four are used (the z pass, whose loads go to L2: 126
+// against 153 us, 18 against 75 us after one edit; the y pass, whose loads hit
+// L1, is 8% faster without).
+template <int NF, int NW, bool PREFETCH>
+__device__ __forceinline__ void scan_layers(const unsigned char* const* f, ptrdiff_t step, int count, Quad* best) {
+    static_assert(NF == 1 || NW == 1, "several fields or several weights");
+#pragma unroll
+    for (int k = 0; k < NF * NW; ++k) best[k].odd = best[k].even = 0x3FFF3FFFu;   // kVoxCap + 1
+    static_assert(kVoxCap + 1 == 0x3F, "the cap's byte");
+    // the brick's own layers: distance 0, the same for every weight
+    unsigned v[NF][4], n[NF][4];
+    auto load = [&](unsigned (&to)[NF][4], int t) {
+#pragma unroll
+        for (int k = 0; k < NF; ++k)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                to[k][j] = __ldg(reinterpret_cast<const unsigned*>(f[k] + (ptrdiff_t)(t + j) * step));
+    };
+    load(v, 0);
+    if (PREFETCH && count > 4) load(n, 4);
+#pragma unroll
+    for (int k = 0; k < NF; ++k) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            best[k].odd = pair_min(best[k].odd, v[k][j]);
+            best[k].even = pair_min(best[k].even, v[k][j] * 256u);
+        }
+#pragma unroll
+        for (int s = 1; s < NW; ++s) best[s] = best[0];
+    }
+    unsigned most = quad_max(best[0]);
+#pragma unroll
+    for (int k = 1; k < NF; ++k) most = max(most, quad_max(best[k]));
+    int t = 4;
+    unsigned d2 = 0x01000100u;
+#pragma unroll
+    for (int weights = NW; weights >= 1; --weights) {   // results 0 .. weights - 1 are still open
+        const int end = weights == 1 ? count : min(count, (4 + (kVoxCap >> (weights - 1)) + 3) / 4 * 4);
+        // t - 3: the next layer's distance; the other weights end no later
+        for (; (unsigned)(t - 3) < most && t < end; t += 4) {
+            if (PREFETCH) {
+#pragma unroll
+                for (int k = 0; k < NF; ++k)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) v[k][j] = n[k][j];
+                if (t + 4 < count) load(n, t + 4);
+            } else {
+                load(v, t);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                // (distances past the cap, at most 62 + 28, change nothing)
+#pragma unroll
+                for (int k = 0; k < NF; ++k)
+#pragma unroll
+                    for (int s = 0; s < weights; ++s) quad_take(best[k + s], v[k][j], d2 << s);
+                d2 += 0x01000100u;
+            }
+            most = quad_max(best[0]);
+#pragma unroll
+            for (int k = 1; k < NF; ++k) most = max(most, quad_max(best[k]));
+        }
+    }
+}
+
+// One thread: four bricks in x, one field (up) or the four shapes (down).
+// blockIdx.y: x direction, y direction << 1.
 __global__ void k_bdist_y(const unsigned char* __restrict__ xf, unsigned char* __restrict__ yf, BrickGrid b, int3 lo,
                           int3 ext, const int* __restrict__ d_cell) {
     if (d_cell) {
         if (!d_cell[3]) return;
         lo = edit_origin(lo, d_cell, false, false, true);
     }
-    const int yi = (int)blockIdx.y;  // y_field(xs, ys, shape)
-    const bool fwd = yi < 2;
-    const int xs = fwd ? yi : (yi - 2) & 1, shape = fwd ? 0 : (yi - 2) >> 1;
-    const int wy = 1 << shape;
+    const int xs = (int)(blockIdx.y & 1u);
+    const bool fwd = (blockIdx.y & 2u) != 0u;
     const int Y = b.GY * 4;
     const int3 g = make_int3(b.GX, b.GY, b.GZ * 4);
-    xf += (size_t)xs * ((size_t)b.GX * Y * g.z);
-    yf += (size_t)yi * ((size_t)g.x * g.y * g.z);
-    const size_t total = (size_t)ext.x * ext.y * ext.z;
-    for (size_t lin = blockIdx.x * (size_t)blockDim.x + threadIdx.x; lin < total; lin += (size_t)gridDim.x * blockDim.x) {
-        int bx, by, qz;
-        if (!box_cell(lin, lo, ext, g, bx, by, qz)) continue;
-        int best = kVoxCap + 1;
-        for (int t = 0;; ++t) {
-            const int dy = max(0, t - 3);
-            const int qy = fwd ? 4 * by + t : 4 * by + 3 - t;
-            if (wy * dy >= best || qy < 0 || qy >= Y) break;
-            best = min(best, max(wy * dy, (int)xf[(size_t)bx + (size_t)g.x * ((size_t)qy + (size_t)Y * qz)]));
-        }
-        yf[(size_t)bx + (size_t)g.x * ((size_t)by + (size_t)g.y * qz)] = (unsigned char)best;
+    int x4, by, qz;
+    if (!box_item(blockIdx.x * blockDim.x + threadIdx.x, lo, ext, 4, g, x4, by, qz)) return;
+    const unsigned char* near = xf + (size_t)xs * ((size_t)b.GX * Y * g.z) + (size_t)(4 * x4) +
+                                (size_t)b.GX * ((size_t)(fwd ? 4 * by : 4 * by + 3) + (size_t)Y * qz);
+    const size_t field = (size_t)g.x * g.y * g.z, cell = (size_t)(4 * x4) + (size_t)g.x * ((size_t)by + (size_t)g.y * qz);
+    const unsigned char* const in[1] = {near};
+    if (fwd) {
+        Quad q[1];
+        scan_layers<1, 1, false>(in, b.GX, Y - 4 * by, q);
+        *reinterpret_cast<unsigned*>(yf + (size_t)y_field(xs, 1, 0) * field + cell) = quad_bytes(q[0]);
+    } else {
+        Quad q[kBoxShapes];
+        scan_layers<1, kBoxShapes, false>(in, -(ptrdiff_t)b.GX, 4 * by + 4, q);
+#pragma unroll
+        for (int shape = 0; shape < kBoxShapes; ++shape)
+            *reinterpret_cast<unsigned*>(yf + (size_t)y_field(xs, 0, shape) * field + cell) = quad_bytes(q[shape]);
     }
 }
 
+// One thread: four bricks in x, one octant (blockIdx.y).
 __global__ void k_bdist_z(const unsigned char* __restrict__ yf, unsigned char* __restrict__ out, BrickGrid b, int3 lo,
                           int3 ext, const int* __restrict__ d_cell, size_t stride) {
     if (d_cell) {
         if (!d_cell[3]) return;
         lo = edit_origin(lo, d_cell, false, false, false);
     }
-    const unsigned v = blockIdx.y;   // the octant
+    const unsigned v = blockIdx.y;
     const bool fwd = (v & 4u) != 0u, up = (v & 2u) != 0u;
     const int xs = (int)(v & 1u);
     const int Z = b.GZ * 4;
-    const int3 g = make_int3(b.GX, b.GY, b.GZ);
-    const size_t yfield = (size_t)b.GX * b.GY * Z;
-    out += (size_t)v * stride;
-    const size_t total = (size_t)ext.x * ext.y * ext.z;
-    for (size_t lin = blockIdx.x * (size_t)blockDim.x + threadIdx.x; lin < total; lin += (size_t)gridDim.x * blockDim.x) {
-        int bx, by, bz;
-        if (!box_cell(lin, lo, ext, g, bx, by, bz)) continue;
-        const size_t col = (size_t)bx + (size_t)g.x * (size_t)by;
-        unsigned char res = 0;
-        int best_score = -1;
-        for (int shape = 0; shape < (up ? 1 : kBoxShapes); ++shape) {
-            const unsigned char* f = yf + (size_t)y_field(xs, up ? 1 : 0, shape) * yfield;
-            int best = kVoxCap + 1;
-            for (int t = 0;; ++t) {
-                const int dz = max(0, t - 3);
-                const int qz = fwd ? 4 * bz + t : 4 * bz + 3 - t;
-                if (dz >= best || qz < 0 || qz >= Z) break;
-                best = min(best, max(dz, (int)f[col + (size_t)g.x * g.y * qz]));
+    int x4, by, bz;
+    if (!box_item(blockIdx.x * blockDim.x + threadIdx.x, lo, ext, 4, make_int3(b.GX, b.GY, b.GZ), x4, by, bz)) return;
+    const size_t layer = (size_t)b.GX * b.GY, yfield = layer * Z;
+    const unsigned char* near = yf + (size_t)(4 * x4) + (size_t)b.GX * by + layer * (size_t)(fwd ? 4 * bz : 4 * bz + 3);
+    const ptrdiff_t step = fwd ? (ptrdiff_t)layer : -(ptrdiff_t)layer;
+    const int count = fwd ? Z - 4 * bz : 4 * bz + 4;
+    unsigned res = 0u;
+    if (up) {
+        const unsigned char* const in[1] = {near + (size_t)y_field(xs, 1, 0) * yfield};
+        Quad q[1];
+        scan_layers<1, 1, true>(in, step, count, q);
+        res = quad_bytes(q[0]);
+    } else {
+        const unsigned char* in[kBoxShapes];
+#pragma unroll
+        for (int shape = 0; shape < kBoxShapes; ++shape) in[shape] = near + (size_t)y_field(xs, 0, shape) * yfield;
+        Quad q[kBoxShapes];
+        scan_layers<kBoxShapes, 1, true>(in, step, count, q);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            unsigned cell = 0u;
+            int best_score = -1;
+#pragma unroll
+            for (int shape = 0; shape < kBoxShapes; ++shape) {
+                const int s = (int)((((i & 1) ? q[shape].odd : q[shape].even) >> ((i >> 1) * 16 + 8)) & 0xFFu);
+                const int score = box_score(s, shape);
+                if (s != 0 && score > best_score) {   // s is 0 for every shape where the brick is occupied
+                    best_score = score;
+                    cell = (unsigned)(s | (shape << 6));
+                }
             }
-            if (best == 0) break;   // the brick is occupied
-            const int score = box_score(best, shape);
-            if (score > best_score) {
-                best_score = score;
-                res = (unsigned char)(best | (shape << 6));
-            }
+            res |= cell << (8 * i);
         }
-        out[brick_index(bx, by, bz, b.CX, b.CY)] = res;
     }
+    *reinterpret_cast<unsigned*>(out + (size_t)v * stride + brick_index(4 * x4, by, bz, b.CX, b.CY)) = res;
 }
 
 namespace {
 
 constexpr int kDistThreads = 256;
 
-unsigned dist_blocks(size_t n) {
-    return (unsigned)std::min<size_t>((n + kDistThreads - 1) / kDistThreads, 65535u * 4u);
-}
+unsigned dist_blocks(size_t n) { return (unsigned)((n + kDistThreads - 1) / kDistThreads); }
 
 size_t volume(int3 e) { return (size_t)e.x * e.y * e.z; }
 
 // The chunk level over the whole chunk grid (at most a few tens of thousands
-// of cells: cheap enough to redo after any edit): x into 2 fields of tmp, y
+// of cells: cheap enough to redo after any edit, and skipped on the device
+// after an edit that changed no coarse bit, the rule for single voxels): x into 2 fields of tmp, y
 // into the 4 fields after them, z into the 8 output fields.
-void chunk_passes(vt_world* w, cudaStream_t st) {
+void chunk_passes(vt_world* w, cudaStream_t st, const int* d_changed) {
     const int CX = w->cdim[0], CY = w->cdim[1], CZ = w->cdim[2];
     const size_t stride = cdist_stride((unsigned)w->nchunks);
     unsigned char* fx = w->d_ctmp;
     unsigned char* fy = w->d_ctmp + 2 * stride;
     const unsigned nb = dist_blocks(w->nchunks);
-    k_dist_pass<<<dim3(nb, 2), kDistThreads, 0, st>>>(w->d_coarse, nullptr, fx, 0, CX, CY, CZ, stride);
-    k_dist_pass<<<dim3(nb, 4), kDistThreads, 0, st>>>(w->d_coarse, fx, fy, 1, CX, CY, CZ, stride);
-    k_dist_pass<<<dim3(nb, 8), kDistThreads, 0, st>>>(w->d_coarse, fy, w->d_cdist, 2, CX, CY, CZ, stride);
+    k_dist_pass<<<dim3(nb, 2), kDistThreads, 0, st>>>(w->d_coarse, nullptr, fx, 0, CX, CY, CZ, stride, d_changed);
+    k_dist_pass<<<dim3(nb, 4), kDistThreads, 0, st>>>(w->d_coarse, fx, fy, 1, CX, CY, CZ, stride, d_changed);
+    k_dist_pass<<<dim3(nb, 8), kDistThreads, 0, st>>>(w->d_coarse, fy, w->d_cdist, 2, CX, CY, CZ, stride, d_changed);
 }
 
 // The brick level, each pass over its own box (x: bricks x voxels x voxels,
@@ -308,14 +464,13 @@ void brick_passes(vt_world* w, cudaStream_t st, const int3 lo[3], const int3 ext
     const size_t nb = w->nchunks * kBricksPerChunk;
     unsigned char* xf = w->d_dtmp;             // 2 fields of 16 bytes per brick
     unsigned char* yf = w->d_dtmp + 32 * nb;   // kYFields fields of 4 bytes per brick
-    if (volume(ext[0]))
-        k_bdist_x<<<dim3(dist_blocks(volume(ext[0])), 2), kDistThreads, 0, st>>>(w->d_mask, xf, b, lo[0], ext[0], d_cell);
-    if (volume(ext[1]))
-        k_bdist_y<<<dim3(dist_blocks(volume(ext[1])), kYFields), kDistThreads, 0, st>>>(xf, yf, b, lo[1], ext[1],
-                                                                                        d_cell);
-    if (volume(ext[2]))
-        k_bdist_z<<<dim3(dist_blocks(volume(ext[2])), 8), kDistThreads, 0, st>>>(yf, w->d_bdist, b, lo[2], ext[2],
-                                                                                 d_cell, nb);
+    // (an aligned group more than the box's bricks need, on either side)
+    const size_t nx = (size_t)((ext[0].x + 7) / 8 + 1) * ext[0].y * ext[0].z,
+                 ny = (size_t)((ext[1].x + 3) / 4 + 1) * ext[1].y * ext[1].z,
+                 nz = (size_t)((ext[2].x + 3) / 4 + 1) * ext[2].y * ext[2].z;
+    k_bdist_x<<<dist_blocks(nx), kDistThreads, 0, st>>>(w->d_mask, xf, b, lo[0], ext[0], d_cell);
+    k_bdist_y<<<dim3(dist_blocks(ny), 4), kDistThreads, 0, st>>>(xf, yf, b, lo[1], ext[1], d_cell);
+    k_bdist_z<<<dim3(dist_blocks(nz), 8), kDistThreads, 0, st>>>(yf, w->d_bdist, b, lo[2], ext[2], d_cell, nb);
 }
 
 // After the bricks of box [blo, blo + bext) changed occupancy only these
@@ -328,8 +483,8 @@ void brick_passes(vt_world* w, cudaStream_t st, const int3 lo[3], const int3 ext
 // leaves every buffer equal to a full rebuild.
 void edit_boxes(int3 blo, int3 bext, int3 lo[3], int3 ext[3]) {
     const int R = (kVoxCap + 3) / 4;
-    lo[0] = make_int3(blo.x - R, 4 * blo.y, 4 * blo.z);
-    ext[0] = make_int3(bext.x + 2 * R, 4 * bext.y, 4 * bext.z);
+    lo[0] = make_int3(blo.x - R, blo.y, 4 * blo.z);
+    ext[0] = make_int3(bext.x + 2 * R, bext.y, 4 * bext.z);
     lo[1] = make_int3(blo.x - R, blo.y - R, 4 * blo.z);
     ext[1] = make_int3(bext.x + 2 * R, bext.y + 2 * R, 4 * bext.z);
     lo[2] = make_int3(blo.x - R, blo.y - R, blo.z - R);
@@ -342,9 +497,9 @@ vt_status rebuild_distances(vt_world* w, cudaStream_t st) {
     const int GX = w->cdim[0] * 8, GY = w->cdim[1] * 8, GZ = w->cdim[2] * 8;
     const int3 o = make_int3(0, 0, 0);
     const int3 lo[3] = {o, o, o};
-    const int3 ext[3] = {make_int3(GX, 4 * GY, 4 * GZ), make_int3(GX, GY, 4 * GZ), make_int3(GX, GY, GZ)};
+    const int3 ext[3] = {make_int3(GX, GY, 4 * GZ), make_int3(GX, GY, 4 * GZ), make_int3(GX, GY, GZ)};
     brick_passes(w, st, lo, ext, nullptr);
-    chunk_passes(w, st);
+    chunk_passes(w, st, nullptr);
     VT_CUDA(w->ctx, cudaGetLastError());
     w->dist_dirty = false;
     w->dist_box = false;
@@ -361,7 +516,7 @@ vt_status update_distances(vt_world* w, cudaStream_t st) {
     edit_boxes(blo, bext, lo, ext);
     if (volume(ext[2]) >= w->nchunks * kBricksPerChunk / 2) return rebuild_distances(w, st);
     brick_passes(w, st, lo, ext, nullptr);
-    chunk_passes(w, st);
+    chunk_passes(w, st, nullptr);
     VT_CUDA(w->ctx, cudaGetLastError());
     w->dist_box = false;
     return VT_OK;
@@ -373,7 +528,7 @@ vt_status update_distances_at(vt_world* w, const int* d_cell, cudaStream_t st) {
     int3 lo[3], ext[3];
     edit_boxes(make_int3(0, 0, 0), make_int3(1, 1, 1), lo, ext);
     brick_passes(w, st, lo, ext, d_cell);
-    chunk_passes(w, st);
+    chunk_passes(w, st, d_cell + 4);
     VT_CUDA(w->ctx, cudaGetLastError());
     return VT_OK;
 }
@@ -456,9 +611,9 @@ vt_status vt_world_create(vt_ctx* ctx, const vt_world_desc* desc, vt_world** out
         (e = vt::dev_alloc(&w->d_cdist, kOctants * (size_t)cdist_stride((unsigned)w->nchunks))) != cudaSuccess ||
         (e = vt::dev_alloc(&w->d_dtmp, (32 + 4 * kYFields) * w->nchunks * kBricksPerChunk)) != cudaSuccess ||
         (e = vt::dev_alloc(&w->d_ctmp, 6 * (size_t)cdist_stride((unsigned)w->nchunks))) != cudaSuccess ||
-        (e = vt::dev_alloc(&w->d_edit, 4 * sizeof(int))) != cudaSuccess ||
+        (e = vt::dev_alloc(&w->d_edit, 5 * sizeof(int))) != cudaSuccess ||
         (e = vt::dev_alloc(&w->d_entities, kMaxEntities * 6 * sizeof(float))) != cudaSuccess ||
-        (e = cudaMemset(w->d_edit, 0, 4 * sizeof(int))) != cudaSuccess ||
+        (e = cudaMemset(w->d_edit, 0, 5 * sizeof(int))) != cudaSuccess ||
         (e = cudaMemset(w->d_mask, 0, w->nchunks * kBricksPerChunk * 8)) != cudaSuccess ||
         (e = cudaMemset(w->d_mats, 0, w->nchunks * (size_t)kChunkBytes)) != cudaSuccess ||
         (e = cudaMemset(w->d_coarse, 0, w->ncoarse * 8)) != cudaSuccess) {
