@@ -114,18 +114,21 @@ VT_HD inline uint8_t cell_material(const vt_gen_desc* d, int x, int y, int z, in
 }
 
 // Tree t of a scene: its column (x, z) from draws 2t and 2t+1 of the tree
-// stream (SplitMix64 is counter based: draw k is mix64(s0 + (k+1) * gamma)),
-// and its surface height h; false when the tree does not fit under the top.
-VT_HD inline bool tree_site(const vt_gen_desc* d, int t, int* x, int* z, int* h) {
-    const int X = d->dims[0], Y = d->dims[1], Z = d->dims[2];
+// stream (SplitMix64 is counter based: draw k is mix64(s0 + (k+1) * gamma)).
+VT_HD inline void tree_column(const vt_gen_desc* d, int t, int* x, int* z) {
     const uint64_t s0 = stream_seed(d->seed, kTrees);
     const uint64_t g = 0x9E3779B97F4A7C15ull;
     const double ux = (double)(mix64(s0 + (uint64_t)(2 * t + 1) * g) >> 11) * 0x1p-53;
     const double uz = (double)(mix64(s0 + (uint64_t)(2 * t + 2) * g) >> 11) * 0x1p-53;
-    *x = 2 + (int)(ux * (double)(X - 4));
-    *z = 2 + (int)(uz * (double)(Z - 4));
+    *x = 2 + (int)(ux * (double)(d->dims[0] - 4));
+    *z = 2 + (int)(uz * (double)(d->dims[2] - 4));
+}
+
+// Its column and surface height h; false when it does not fit under the top.
+VT_HD inline bool tree_site(const vt_gen_desc* d, int t, int* x, int* z, int* h) {
+    tree_column(d, t, x, z);
     *h = height_at(d, *x, *z);
-    return *h + 8 < Y;
+    return *h + 8 < d->dims[1];
 }
 
 // Whether leaf cell (dx, dy, dz) in [-2, 2]^3 of tree t is kept (p = 0.7).

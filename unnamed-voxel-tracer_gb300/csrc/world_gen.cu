@@ -8,12 +8,19 @@
 // chunk layout directly: no dense staging grid, no host traffic.  The bytes
 // equal vt_gen_world's for every descriptor.
 //
-//   k_gen_chunks   one block per chunk, one thread per brick: the chunk's
+//   k_gen_tiles    one block per chunk, one thread per brick: the chunk's
 //                  32x32 column heights in shared memory, then 64 cells per
-//                  thread (terrain, water, caves), brick word and coarse bit
+//                  thread (terrain, water, caves), brick word and coarse bit;
+//                  the noise in 32 bits from shared lattice tables, decided in
+//                  64 bits where 32 cannot
+//   k_gen_chunks   the same in 64 bits cell by cell, for noise so fine that a
+//                  chunk's lattice tables would not fit
 //   k_gen_leaves   one block per tree, one thread per leaf cell
 //   k_gen_trunks   one thread per tree, after all leaves (see plant_trees on
 //                  why the parallel order gives the sequential bytes)
+#include <cmath>
+#include <cstring>
+
 #include "gen_noise.cuh"
 #include "vt_internal.h"
 
@@ -33,7 +40,9 @@ __device__ __forceinline__ void cell_addr(const WorldView& w, int x, int y, int 
 __device__ __forceinline__ void mark_solid(unsigned long long* mask, unsigned long long* coarse, unsigned wi, unsigned vb) {
     atomicOr(mask + wi, 1ull << vb);
     const unsigned ci = wi >> 9;
-    atomicOr(coarse + (ci >> 6), 1ull << (ci & 63u));
+    // most trees stand in chunks the terrain marked already
+    const unsigned long long bit = 1ull << (ci & 63u);
+    if (!(__ldcg(coarse + (ci >> 6)) & bit)) atomicOr(coarse + (ci >> 6), bit);
 }
 
 __global__ void __launch_bounds__(512) k_gen_chunks(WorldView w, unsigned long long* mask, unsigned char* mats,
@@ -83,21 +92,292 @@ __global__ void __launch_bounds__(512) k_gen_chunks(WorldView w, unsigned long l
     }
 }
 
+// ---------------------------------------------------------------------------
+// The generator's noise in 32 bits.
+//
+// Every material is decided by comparing an fbm value with a number: a cave
+// cell by fbm3 > cave_threshold, a column by the floor of base + amplitude *
+// fbm2.  The device has two double-precision lanes per SM and cycle, and the
+// 64-bit noise of a cave cell costs 48 lattice hashes and about 84 double
+// operations, so that the kernel was bound by them (512x256x512 cave world:
+// 6.22 ms).  A 32-bit value decides the same comparison unless it lies within
+// its error bound of the number; only then is the 64-bit value computed.
+// The lattice values a chunk needs (a few hundred) are hashed once into shared
+// memory, and the cave noise is interpolated along x once per lattice row.
+// The same world now takes 145 us.
+//
+// Error of the 32-bit values against the real ones, u = 2^-24: a lattice value
+// is in [-1, 1) (rounding u / 2), a weight smooth(t) is off by at most 4 u, an
+// interpolation a + (b - a) t adds 2 * 4 u for the weight and at most 2 u for
+// its rounding.  Two levels and a weighted mean of at most 16 octaves stay
+// below 32 u = 1.9e-6, three levels below 31 u, times 1.5 for the two octaves'
+// sum.  (The 64-bit values' own error is below 1e-14.)
+constexpr float kFbmError = 2.5e-6f, kCaveError = 4e-6f;
+
+// gen::lattice rounded to 32 bits: the hash as a signed fraction.
+__device__ __forceinline__ float lattice32(uint64_t seed, int x, int y, int z) {
+    uint64_t h = gen::mix64(seed ^ ((uint64_t)(int64_t)x * 0x9E3779B97F4A7C15ull));
+    h = gen::mix64(h ^ ((uint64_t)(int64_t)y * 0xC2B2AE3D27D4EB4Full));
+    h = gen::mix64(h ^ ((uint64_t)(int64_t)z * 0x165667B19E3779F9ull));
+    return __int2float_rn((int)((unsigned)(h >> 32) ^ 0x80000000u)) * 0x1p-31f;
+}
+
+// Lattice cell and interpolation weight of coordinate g (below 2^13) at a
+// frequency (below 2^2) held as a multiple of 2^-40: the position is exact to
+// 2^-28, and the noise is continuous across the cells.
+__device__ __forceinline__ void lattice_coord(int g, long long f, int& cell, float& weight) {
+    const long long x = (long long)g * f;
+    const float t = __uint2float_rn((unsigned)((unsigned long long)x >> 8)) * 0x1p-32f;
+    cell = (int)(x >> 40);
+    weight = t * t * (3.0f - 2.0f * t);
+}
+
+__device__ __forceinline__ float lerp32(float a, float b, float t) { return __fmaf_rn(b - a, t, a); }
+
+struct GenArgs {
+    vt_gen_desc d;
+    double cave_freq;            // 1 / cave_period
+    long long freq40, cave40;    // the frequencies, multiples of 2^-40
+    uint64_t terrain_seed, cave_seed, leaf_seed;
+    float norm;                  // 1 / (sum of the octaves' amplitudes)
+    int water;
+    // shared-memory layout of k_gen_tiles, in floats
+    int height_side[16];         // most lattice points a chunk meets on an axis, per octave
+    int height_floats;
+    int cave_side[2];
+    int cave_floats, cave_rows;  // lattice values; rows interpolated along x (32 values each)
+};
+
+// The 64-bit decisions, out of line: inlined they cost the kernels registers
+// (k_gen_tiles 368 bytes of spills) for one column or cell in thousands.
+__device__ __noinline__ int height_exact(const vt_gen_desc* d, int x, int z) { return gen::height_at(d, x, z); }
+__device__ __noinline__ bool cave_exact(const GenArgs* a, int x, int y, int z) {
+    return gen::fbm3(a->cave_seed, (double)x, (double)y, (double)z, a->cave_freq) > (double)a->d.cave_threshold;
+}
+
+// The column height from the 32-bit fbm value (gen::height_at's rounding and
+// clamps), or in 64 bits where that does not decide the floor.
+__device__ __forceinline__ int height_of(const GenArgs& a, float fbm, int x, int z) {
+    const float v = __fmaf_rn(a.d.amplitude, fbm, a.d.base_height);
+    const float margin = fabsf(a.d.amplitude) * kFbmError + fabsf(v) * 0x1p-22f;
+    const float lo = floorf(v - margin);
+    if (!(lo == floorf(v + margin)) || !(fabsf(lo) < 1e6f)) return height_exact(&a.d, x, z);
+    int h = (int)lo;
+    h = h < a.d.dims[1] - 1 ? h : a.d.dims[1] - 1;
+    return h > 1 ? h : 1;
+}
+
+// gen::height_at of one column without tables.
+__device__ int height_at32(const GenArgs& a, int x, int z) {
+    if (!a.freq40) return height_exact(&a.d, x, z);
+    long long f = a.freq40;
+    float sum = 0.0f, amp = 1.0f;
+    for (int o = 0; o < a.d.octaves; ++o) {
+        int cx, cz;
+        float sx, sz;
+        lattice_coord(x, f, cx, sx);
+        lattice_coord(z, f, cz, sz);
+        const uint64_t seed = a.terrain_seed + (uint64_t)o * gen::kOctaveSalt;
+        const float p = lerp32(lattice32(seed, cx, 0, cz), lattice32(seed, cx + 1, 0, cz), sx);
+        const float q = lerp32(lattice32(seed, cx, 0, cz + 1), lattice32(seed, cx + 1, 0, cz + 1), sx);
+        sum += amp * lerp32(p, q, sz);
+        amp *= 0.5f;
+        f *= 2;
+    }
+    return height_of(a, sum * a.norm, x, z);
+}
+
+// gen::tree_site with the 32-bit height.
+__device__ bool tree_site32(const GenArgs& a, int t, int* x, int* z, int* h) {
+    gen::tree_column(&a.d, t, x, z);
+    *h = height_at32(a, *x, *z);
+    return *h + 8 < a.d.dims[1];
+}
+
+// (two blocks per SM: 145 us on the cave world, one 366, three 154)
+__global__ void __launch_bounds__(512, 2) k_gen_tiles(WorldView w, unsigned long long* mask, unsigned char* mats,
+                                                   unsigned long long* coarse, const __grid_constant__ GenArgs a) {
+    extern __shared__ float s_gen[];
+    __shared__ int heights[32 * 32];
+    __shared__ float weight[16][2][32];       // [octave][axis][coordinate]; caves: [octave * 3 + axis][0]
+    __shared__ unsigned char cell[16][2][32]; // lattice cell relative to the chunk's first
+    __shared__ int first[16][2];              // the chunk's first lattice point
+    const unsigned ci = blockIdx.x;
+    const int cx = (int)(ci % (unsigned)w.cdim[0]);
+    const int cy = (int)((ci / (unsigned)w.cdim[0]) % (unsigned)w.cdim[1]);
+    const int cz = (int)(ci / ((unsigned)w.cdim[0] * (unsigned)w.cdim[1]));
+    const int tid = threadIdx.x;
+
+    // ---- heights
+    for (int i = tid; i < a.d.octaves * 64; i += 512) {
+        const int o = i >> 6, axis = (i >> 5) & 1, k = i & 31, g0 = (axis ? cz : cx) * 32;
+        int c;
+        float s;
+        lattice_coord(g0 + k, a.freq40 << o, c, s);
+        const int c0 = __shfl_sync(0xFFFFFFFFu, c, 0);   // k is the lane
+        weight[o][axis][k] = s;
+        cell[o][axis][k] = (unsigned char)(c - c0);
+        if (k == 0) first[o][axis] = c0;
+    }
+    __syncthreads();
+    for (int o = 0, base = 0; o < a.d.octaves; ++o) {
+        const int n = a.height_side[o];
+        const uint64_t seed = a.terrain_seed + (uint64_t)o * gen::kOctaveSalt;
+        for (int i = tid; i < n * n; i += 512) s_gen[base + i] = lattice32(seed, first[o][0] + i % n, 0, first[o][1] + i / n);
+        base += n * n;
+    }
+    __syncthreads();
+    for (int c = tid; c < 32 * 32; c += 512) {
+        const int lx = c & 31, lz = c >> 5, gx = cx * 32 + lx, gz = cz * 32 + lz;
+        int h = 0;
+        if (gx < w.dims[0] && gz < w.dims[2]) {
+            float sum = 0.0f, amp = 1.0f;
+            for (int o = 0, base = 0; o < a.d.octaves; ++o) {
+                const int n = a.height_side[o];
+                const float* l = s_gen + base + cell[o][0][lx] + n * cell[o][1][lz];
+                const float sx = weight[o][0][lx];
+                sum += amp * lerp32(lerp32(l[0], l[1], sx), lerp32(l[n], l[n + 1], sx), weight[o][1][lz]);
+                amp *= 0.5f;
+                base += n * n;
+            }
+            h = height_of(a, sum * a.norm, gx, gz);
+        }
+        heights[c] = h;
+    }
+    __syncthreads();
+
+    // ---- cave tables: per octave the lattice, then its rows along x (fixed
+    // lattice y and z) interpolated at the chunk's 32 coordinates
+    float* rows = s_gen + a.cave_floats;
+    if (a.d.caves) {
+        for (int i = tid; i < 2 * 96; i += 512) {
+            const int o = i / 96, axis = (i % 96) >> 5, k = i & 31, g0 = (axis == 0 ? cx : (axis == 1 ? cy : cz)) * 32;
+            int c;
+            float s;
+            lattice_coord(g0 + k, a.cave40 << o, c, s);
+            const int c0 = __shfl_sync(0xFFFFFFFFu, c, 0);
+            weight[o * 3 + axis][0][k] = s;
+            cell[o * 3 + axis][0][k] = (unsigned char)(c - c0);
+            if (k == 0) first[o * 3 + axis][0] = c0;
+        }
+        __syncthreads();
+        for (int o = 0, base = 0; o < 2; ++o) {
+            const int n = a.cave_side[o];
+            const uint64_t seed = a.cave_seed + (uint64_t)o * gen::kOctaveSalt;
+            for (int i = tid; i < n * n * n; i += 512)
+                s_gen[base + i] = lattice32(seed, first[o * 3][0] + i % n, first[o * 3 + 1][0] + (i / n) % n, first[o * 3 + 2][0] + i / (n * n));
+            base += n * n * n;
+        }
+        __syncthreads();
+        for (int o = 0, base = 0, row0 = 0; o < 2; ++o) {
+            const int n = a.cave_side[o];
+            for (int i = tid; i < n * n * 32; i += 512) {
+                const int x = i & 31, r = i >> 5;
+                const float* l = s_gen + base + n * r + cell[o * 3][0][x];
+                rows[row0 * 32 + i] = lerp32(l[0], l[1], weight[o * 3][0][x]);
+            }
+            base += n * n * n;
+            row0 += n * n;
+        }
+        __syncthreads();
+    }
+
+    // ---- the thread's brick
+    const int bx = tid & 7, by = (tid >> 3) & 7, bz = tid >> 6;
+    const int gy0 = cy * 32 + by * 4;
+    unsigned packed[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) packed[q] = 0u;
+    int top = 0;   // cells at or above it are air or water
+#pragma unroll
+    for (int c = 0; c < 16; ++c) top = max(top, heights[bx * 4 + (c & 3) + 32 * (bz * 4 + (c >> 2))]);
+    const float bound = 1.5f * a.d.cave_threshold;   // of noise + noise / 2
+    const float margin = kCaveError + 1e-6f * fabsf(bound);
+    if (gy0 < top || gy0 < a.water) {
+        const int n0 = a.cave_side[0], n1 = a.cave_side[1];
+#pragma unroll 1
+        for (int x = 0; x < 4; ++x) {
+            const int lx = bx * 4 + x, gx = cx * 32 + lx;
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                const int ly = by * 4 + y, gy = gy0 + y;
+                // the two octaves interpolated along x and y on the lattice
+                // planes around the z cell, kept while it lasts
+                float p0 = 0.0f, q0 = 0.0f, p1 = 0.0f, q1 = 0.0f;
+                int z0 = -1, z1 = -1;
+#pragma unroll
+                for (int z = 0; z < 4; ++z) {
+                    const int lz = bz * 4 + z, gz = cz * 32 + lz;
+                    const int h = heights[lx + 32 * lz];
+                    unsigned v = 0u;
+                    if (gx < w.dims[0] && gy < w.dims[1] && gz < w.dims[2]) {
+                        if (gy < h) {
+                            v = gy == h - 1 ? 1u : (gy >= h - 4 ? 2u : 3u);
+                            if (a.d.caves && gy > 0) {
+                                if (cell[2][0][lz] != z0) {
+                                    z0 = cell[2][0][lz];
+                                    const float* r = rows + 32 * (cell[1][0][ly] + n0 * z0) + lx;
+                                    const float s = weight[1][0][ly];
+                                    p0 = lerp32(r[0], r[32], s);
+                                    q0 = lerp32(r[32 * n0], r[32 * n0 + 32], s);
+                                }
+                                if (cell[5][0][lz] != z1) {
+                                    z1 = cell[5][0][lz];
+                                    const float* r = rows + 32 * (n0 * n0 + cell[4][0][ly] + n1 * z1) + lx;
+                                    const float s = weight[4][0][ly];
+                                    p1 = lerp32(r[0], r[32], s);
+                                    q1 = lerp32(r[32 * n1], r[32 * n1 + 32], s);
+                                }
+                                const float f = __fmaf_rn(0.5f, lerp32(p1, q1, weight[5][0][lz]), lerp32(p0, q0, weight[2][0][lz])) - bound;
+                                bool cave = f > 0.0f;
+                                if (fabsf(f) <= margin)
+                                    cave = cave_exact(&a, gx, gy, gz);
+                                if (cave) v = 0u;
+                            }
+                        } else if (gy < a.water) {
+                            v = 4u;
+                        }
+                    }
+                    packed[y + 4 * z] |= v << (8 * x);
+                }
+            }
+        }
+    }
+    unsigned long long m = 0ull;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+        // bit per nonzero byte
+        const unsigned nz = ((packed[q] & 0x7F7F7F7Fu) + 0x7F7F7F7Fu | packed[q]) & 0x80808080u;
+        m |= (unsigned long long)((nz * 0x00204081u) >> 28) << (4 * q);
+    }
+    const unsigned wi = ci * 512u + (unsigned)tid;
+    uint4* dst = reinterpret_cast<uint4*>(mats + (size_t)wi * 64u);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) dst[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+    mask[wi] = m;
+    const int any = __syncthreads_or(m != 0ull);
+    if (tid == 0) {
+        const unsigned long long bit = 1ull << (ci & 63u);
+        if (any) atomicOr(coarse + (ci >> 6), bit);
+        else atomicAnd(coarse + (ci >> 6), ~bit);
+    }
+}
+
 // Leaf cells of tree blockIdx.x: each kept cell that holds air or water
 // becomes 6.  Concurrent trees only ever write 6 over 0 or 4, so a cell
 // covered by several trees ends the same whichever comes first.
 __global__ void __launch_bounds__(128) k_gen_leaves(WorldView w, unsigned long long* mask, unsigned char* mats,
-                                                    unsigned long long* coarse, vt_gen_desc d) {
+                                                    unsigned long long* coarse, const __grid_constant__ GenArgs a) {
     __shared__ int site[4];
     const int t = blockIdx.x;
-    if (threadIdx.x == 0) site[3] = gen::tree_site(&d, t, &site[0], &site[1], &site[2]) ? 1 : 0;
+    if (threadIdx.x == 0) site[3] = tree_site32(a, t, &site[0], &site[1], &site[2]) ? 1 : 0;
     __syncthreads();
     const int c = threadIdx.x;
     if (!site[3] || c >= 125) return;
     const int dx = c % 5 - 2, dy = (c / 5) % 5 - 2, dz = c / 25 - 2;
     const int lx = site[0] + dx, ly = site[2] + 5 + dy, lz = site[1] + dz;
     if (lx < 0 || lz < 0 || lx >= w.dims[0] || lz >= w.dims[2] || ly >= w.dims[1]) return;
-    if (!gen::leaf_kept(gen::stream_seed(d.seed, gen::kLeaves), t, dx, dy, dz)) return;
+    if (!gen::leaf_kept(a.leaf_seed, t, dx, dy, dz)) return;
     unsigned wi, vb;
     cell_addr(w, lx, ly, lz, &wi, &vb);
     volatile unsigned char* cell = mats + (size_t)wi * 64u + vb;
@@ -108,12 +388,12 @@ __global__ void __launch_bounds__(128) k_gen_leaves(WorldView w, unsigned long l
 }
 
 // Trunks (material 5 over anything), after every leaf has landed.
-__global__ void __launch_bounds__(256) k_gen_trunks(WorldView w, unsigned long long* mask, unsigned char* mats,
-                                                    unsigned long long* coarse, vt_gen_desc d) {
+__global__ void __launch_bounds__(64) k_gen_trunks(WorldView w, unsigned long long* mask, unsigned char* mats,
+                                                    unsigned long long* coarse, const __grid_constant__ GenArgs a) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= d.trees) return;
+    if (t >= a.d.trees) return;
     int x, z, h;
-    if (!gen::tree_site(&d, t, &x, &z, &h)) return;
+    if (!tree_site32(a, t, &x, &z, &h)) return;
     for (int y = h; y < h + 6; ++y) {
         unsigned wi, vb;
         cell_addr(w, x, y, z, &wi, &vb);
@@ -152,6 +432,52 @@ __global__ void __launch_bounds__(512) k_gather_dense(WorldView w, const unsigne
             }
 }
 
+// Most dynamic shared memory k_gen_tiles is given (two blocks per SM).
+constexpr int kGenSmem = 96 * 1024;
+
+// The kernels' arguments, and the dynamic shared memory of k_gen_tiles; 0
+// where its tables would not fit (noise finer than about three voxels) and
+// k_gen_chunks generates the cells.
+int gen_args(const vt_gen_desc& d, GenArgs& a) {
+    std::memset(&a, 0, sizeof(a));
+    a.d = d;
+    const double freq = 1.0 / (double)d.period;
+    a.cave_freq = 1.0 / (double)d.cave_period;
+    a.terrain_seed = gen::stream_seed(d.seed, gen::kTerrain);
+    a.cave_seed = gen::stream_seed(d.seed, gen::kCaves);
+    a.leaf_seed = gen::stream_seed(d.seed, gen::kLeaves);
+    a.water = (int)ceil((double)d.water_level);
+    double norm = 0.0, amp = 1.0;
+    for (int o = 0; o < d.octaves; ++o, amp *= 0.5) norm += amp;
+    a.norm = (float)(1.0 / norm);
+    // 32 coordinates at frequency f meet at most floor(31 f) + 2 cells, one
+    // more lattice points
+    auto side = [](long long f40) { return (double)((31 * f40) >> 40) + 3.0; };
+    const double finest = freq * (double)(1 << (d.octaves - 1));
+    if (!(finest < 2.0)) return 0;
+    a.freq40 = (long long)(freq * 0x1p40);
+    if (d.caves && !(a.cave_freq < 1.0)) return 0;
+    a.cave40 = d.caves ? (long long)(a.cave_freq * 0x1p40) : 0;
+    double heights = 0.0, caves = 0.0, rows = 0.0;
+    for (int o = 0; o < d.octaves; ++o) {
+        const double n = side(a.freq40 << o);
+        a.height_side[o] = (int)n;
+        heights += n * n;
+    }
+    for (int o = 0; o < 2 && d.caves; ++o) {
+        const double n = side(a.cave40 << o);
+        a.cave_side[o] = (int)n;
+        caves += n * n * n;
+        rows += n * n;
+    }
+    const double floats = heights > caves + 32.0 * rows ? heights : caves + 32.0 * rows;
+    if (4.0 * floats > (double)kGenSmem) return 0;
+    a.height_floats = (int)heights;
+    a.cave_floats = (int)caves;
+    a.cave_rows = (int)rows;
+    return (int)floats * 4;
+}
+
 }  // namespace
 
 }  // namespace vt
@@ -170,12 +496,20 @@ vt_status vt_world_generate(vt_world* w, const vt_gen_desc* desc, vt_stream stre
         return fail(w->ctx, VT_ERR_ARG, "generator descriptor out of range");
     cudaStream_t st = (cudaStream_t)stream;
     const WorldView v = w->view();
-    k_gen_chunks<<<(unsigned)w->nchunks, 512, 0, st>>>(v, w->d_mask, w->d_mats, w->d_coarse, *desc);
+    GenArgs a;
+    const int smem = gen_args(*desc, a);
+    if (smem > 0) {
+        if (smem > 32 * 1024)
+            VT_CUDA(w->ctx, cudaFuncSetAttribute(k_gen_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, kGenSmem));
+        k_gen_tiles<<<(unsigned)w->nchunks, 512, smem, st>>>(v, w->d_mask, w->d_mats, w->d_coarse, a);
+    } else {
+        k_gen_chunks<<<(unsigned)w->nchunks, 512, 0, st>>>(v, w->d_mask, w->d_mats, w->d_coarse, *desc);
+    }
     VT_CUDA(w->ctx, cudaGetLastError());
     if (desc->trees > 0 && w->dims[0] >= 6 && w->dims[2] >= 6) {
-        k_gen_leaves<<<(unsigned)desc->trees, 128, 0, st>>>(v, w->d_mask, w->d_mats, w->d_coarse, *desc);
+        k_gen_leaves<<<(unsigned)desc->trees, 128, 0, st>>>(v, w->d_mask, w->d_mats, w->d_coarse, a);
         VT_CUDA(w->ctx, cudaGetLastError());
-        k_gen_trunks<<<(unsigned)((desc->trees + 255) / 256), 256, 0, st>>>(v, w->d_mask, w->d_mats, w->d_coarse, *desc);
+        k_gen_trunks<<<(unsigned)((desc->trees + 63) / 64), 64, 0, st>>>(v, w->d_mask, w->d_mats, w->d_coarse, a);
         VT_CUDA(w->ctx, cudaGetLastError());
     }
     w->dist_dirty = true;
