@@ -12,10 +12,10 @@
 // the hit exactly as the render kernel does (same origin arithmetic, same
 // traversal), instead of being stored between passes.  The backward kernel is
 // the forward kernel plus the loss and gradient epilogue, one thread per
-// pixel.  Palette gradients are summed per warp over the lanes that share a
-// material (the warp walks its distinct materials), per block in shared
-// memory, then once per block with global atomics; albedo gradients go to
-// global memory with one atomic per pixel.
+// pixel of up to four tiles.  Palette gradients are summed per warp over the
+// lanes that share a material (the warp walks its distinct materials), per
+// block in shared memory, then once per block with global atomics; albedo
+// gradients go to global memory with one atomic per pixel.
 #include <cstring>
 
 #include "shade.cuh"
@@ -29,178 +29,37 @@ constexpr int kAdjBlock = 256;
 
 struct AdjArgs {
     WorldView w;
-    FrameParams f;
-    const uint4* hits;
     const float* pal;
     const float* alb;
-    float sun[3], sun_n[3], inv_len;
+    float sun_d[3], sun_inv[3];   // the shadow rays' direction as traced, and its reciprocal (FrameParams)
+    float sun_raw[3];             // as given (entity boxes)
+    float sun_n[3], inv_len;
     float ka, kd;
     int shadow_steps;
+    int tiles;                    // 16x16-pixel tiles a block shades, side by side
     const unsigned char* vis_in;
     unsigned char* vis_out;
-    float* rgb;
-    const float* target;
     float* loss;
     float* gpal;
     float* galb;
     float* gsun;
+    double* sums;                 // 64-bit accumulators of the call, or null
 };
 
-
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    return v;
-}
-
-// One block of 16x16 pixels of the view (f, hits, target, rgb); the rest of
-// the arguments are shared by all views.
-template <bool BWD, bool LONG>
-__device__ __forceinline__ void shade_block(const AdjArgs& a, const FrameParams& f, const uint4* __restrict__ hits,
-                                            const float* __restrict__ target, float* __restrict__ rgb) {
-    extern __shared__ float s_mem[];
-    float* s_gpal = s_mem;            // 768
-    float* s_acc = s_mem + 768;       // loss, sun x3
-    const unsigned char* cd = a.w.cdist;
-    if (BWD) {
-        for (int i = threadIdx.x; i < 772; i += blockDim.x) s_mem[i] = 0.0f;
-    }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int px = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
-    const int py = blockIdx.y * 16 + (warp >> 1) * 4 + (lane >> 3);
-    const bool inside = px < f.width && py < f.height;
-    const size_t p = inside ? (size_t)py * f.width + px : 0;
-
-    bool hit = false;
-    int m = 0;
-    unsigned v = 0;
-    float c[3] = {0.0f, 0.0f, 0.0f}, shade = 0.0f, albv = 1.0f, ndl_raw = 0.0f, nrm[3] = {0.0f, 0.0f, 0.0f};
-    bool lit = false;
-    if (inside) {
-        const uint4 rec = hits[p];
-        hit = ((rec.w >> 16) & VT_HIT_PRIMARY) != 0;
-        if (hit) {
-            v = rec.x;
-            const float t = __uint_as_float(rec.y);
-            const unsigned face = rec.w & 0xFFu;
-            m = (int)((rec.w >> 8) & 0xFFu);
-            const int axis = (int)(face >> 1);
-            const bool pos = (face & 1u) == 0u;
-            float o[3], d[3];
-            primary_ray(f, px, py, o, d);
-            PRay r;
-            pray_init(r, o, d);
-            float so[3];
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                nrm[j] = (j == axis) ? (pos ? -1.0f : 1.0f) : 0.0f;
-                so[j] = __fmaf_rn(r.d[j], t, o[j]);
-                if (j == axis) so[j] = so[j] + nrm[j] * 0.001f;
-            }
-            if (a.vis_in) {
-                lit = a.vis_in[p] != 0;
-            } else {
-                PRay rs;
-                pray_init(rs, so, a.sun);
-                TraceHit hs;
-                lit = !trace_fast<false, true, true, false, LONG>(a.w, cd, rs, a.shadow_steps, hs) &&
-                      !(a.w.n_entities > 0 && entity_occluded(a.w, so, a.sun));
-            }
-            ndl_raw = dot3(nrm, a.sun_n);
-            const float ndl = ndl_raw > 0.0f ? ndl_raw : 0.0f;
-            shade = a.ka + a.kd * ndl * (lit ? 1.0f : 0.0f);
-            albv = a.alb ? __ldg(a.alb + v) : 1.0f;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) c[k] = (__ldg(a.pal + 3 * m + k) * albv) * shade;
-        }
-    }
-    if (!BWD) {
-        if (inside) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) rgb[3 * p + k] = c[k];
-            if (a.vis_out) a.vis_out[p] = (unsigned char)(hit && lit ? 1 : 0);
-        }
-        return;
-    }
-
-    // ---- loss and gradients
-    float g[3] = {0.0f, 0.0f, 0.0f}, lossv = 0.0f;
-    if (inside) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float diff = c[k] - __ldg(target + 3 * p + k);
-            g[k] = 2.0f * diff;
-            lossv += diff * diff;
-        }
-    }
-    float gp[3] = {0.0f, 0.0f, 0.0f}, ga = 0.0f, gs[3] = {0.0f, 0.0f, 0.0f};
-    if (hit) {
-        float gb = 0.0f;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float pk = __ldg(a.pal + 3 * m + k);
-            gp[k] = g[k] * albv * shade;
-            ga += g[k] * pk * shade;
-            gb += g[k] * pk * albv;
-        }
-        if (lit && ndl_raw > 0.0f) {
-            const float coef = gb * a.kd * a.inv_len;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) gs[k] = coef * (nrm[k] - ndl_raw * a.sun_n[k]);
-        }
-    }
-    // palette: one shared-memory atomic per (warp, material).  The warp walks
-    // its distinct materials (few per warp) with butterfly sums, no
-    // divergence.
-    {
-        unsigned todo = __ballot_sync(0xFFFFFFFFu, hit);
-        while (todo) {
-            const int leader = __ffs(todo) - 1;
-            const int key = __shfl_sync(0xFFFFFFFFu, m, leader);
-            const bool mine = hit && m == key;
-            todo &= ~__ballot_sync(0xFFFFFFFFu, mine);
-            const float s0 = warp_sum(mine ? gp[0] : 0.0f), s1 = warp_sum(mine ? gp[1] : 0.0f),
-                        s2 = warp_sum(mine ? gp[2] : 0.0f);
-            if (lane == leader) {
-                atomicAdd(s_gpal + 3 * key + 0, s0);
-                atomicAdd(s_gpal + 3 * key + 1, s1);
-                atomicAdd(s_gpal + 3 * key + 2, s2);
-            }
-        }
-    }
-    // albedo: one global atomic per hit pixel (voxels differ across most of
-    // a warp; the L2 absorbs the few repeats)
-    if (a.galb && hit) atomicAdd(a.galb + v, ga);
-    // loss and sun: warp sums, then shared memory
-    {
-        const float l = warp_sum(lossv), x = warp_sum(gs[0]), y = warp_sum(gs[1]), z = warp_sum(gs[2]);
-        if (lane == 0) {
-            atomicAdd(s_acc + 0, l);
-            atomicAdd(s_acc + 1, x);
-            atomicAdd(s_acc + 2, y);
-            atomicAdd(s_acc + 3, z);
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 768; i += blockDim.x)
-        if (s_gpal[i] != 0.0f) atomicAdd(a.gpal + i, s_gpal[i]);
-    if (threadIdx.x == 0) {
-        atomicAdd(a.loss, s_acc[0]);
-        atomicAdd(a.gsun + 0, s_acc[1]);
-        atomicAdd(a.gsun + 1, s_acc[2]);
-        atomicAdd(a.gsun + 2, s_acc[3]);
-    }
-}
-
-template <bool BWD, bool LONG>
-__global__ void __launch_bounds__(kAdjBlock) k_shade(AdjArgs a) {
-    shade_block<BWD, LONG>(a, a.f, a.hits, a.target, a.rgb);
+// A call's accumulators: 768 palette gradients, the loss and the sun's
+// gradient.  Zero between calls: k_shade_sums adds them to the caller's and
+// clears them.  (Thousands of blocks adding to one float leave it off by up to
+// 1e-5, in one direction where many blocks add the same value.)
+constexpr int kGradSums = 772;
+static_assert(kGradSums * sizeof(double) <= kShadeSumBytes, "accumulator region");
+__device__ __forceinline__ float* grad_sum(const AdjArgs& a, int i) {
+    return i < 768 ? a.gpal + i : (i == 768 ? a.loss : a.gsun + (i - 769));
 }
 
 // Several views of one world in one launch (blockIdx.z = view): one launch
 // instead of one per view, whose tails would leave the GPU partly idle.
 constexpr int kMaxViews = 16;
+constexpr int kMaxTiles = 4;
 struct ViewP {
     float pos[3];
     float view[16];
@@ -216,30 +75,188 @@ struct ViewsArgs {
 };
 static_assert(sizeof(ViewsArgs) <= 4096, "the views travel in the kernel parameters");
 
-// Register caps: 40 for the backward kernel (6 blocks per SM; a 12-byte
-// spill) and 48 for the forward one (5 blocks), the fastest of 40/48/59
-// measured on 16 views of 512x512.
-template <bool BWD, bool LONG>
-__global__ void __launch_bounds__(kAdjBlock, BWD ? 6 : 5) k_shade_views(ViewsArgs va) {
+// Sums of four values over the warp, halving the values with the lanes: the
+// sums of a, b, c and d end in lanes 0, 8, 16 and 24 (6 shuffles instead of 20).
+__device__ __forceinline__ float warp_sum4(unsigned lane, float a, float b, float c, float d) {
+    const bool h16 = (lane & 16u) != 0u, h8 = (lane & 8u) != 0u;
+    const float x = (h16 ? c : a) + __shfl_xor_sync(0xFFFFFFFFu, h16 ? a : c, 16);
+    const float y = (h16 ? d : b) + __shfl_xor_sync(0xFFFFFFFFu, h16 ? b : d, 16);
+    float r = (h8 ? y : x) + __shfl_xor_sync(0xFFFFFFFFu, h8 ? x : y, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xFFFFFFFFu, r, o);
+    return r;
+}
+
+// One block: a.tiles tiles of 16x16 pixels in a row.  The forward kernel is
+// the shadow walks; the backward one adds the loss and gradients, per thread
+// over the block's tiles for the loss and the sun, in shared memory for the
+// palette, so that a block clears, sums and flushes them once.
+// Bound: issue slots (77-80%).  16 views of 512x512: forward 101 us, backward
+// 166 -> 130 us against one tile per block, a sum over the warp per value and
+// tile, and the general walk inlined beside the forward one.  GENERAL: long
+// step limits, or a sun direction the forward walk does not take (trace_fast).
+// Register caps: 7 and 6 blocks per SM, the fastest of 4-8 (36 and 40
+// registers, a few bytes spilled).
+template <bool BWD, bool GENERAL>
+__global__ void __launch_bounds__(kAdjBlock, BWD ? 6 : 7) k_shade_views(const __grid_constant__ ViewsArgs va) {
+    const AdjArgs& a = va.a;
     const ViewP& V = va.v[blockIdx.z];
-    if ((int)blockIdx.x * 16 >= V.width || (int)blockIdx.y * 16 >= V.height) return;  // the view is smaller
-    FrameParams f = va.a.f;
+    __shared__ float s_gpal[BWD ? 768 : 1], s_acc[4];   // palette gradient; loss and sun
+    __shared__ float s_col[16 * kMaxTiles], s_row[16];  // ray UVs (shade.cuh, ray_u and ray_v)
+    const int x0 = (int)blockIdx.x * 16 * a.tiles, y0 = (int)blockIdx.y * 16;
+    if (x0 >= V.width || y0 >= V.height) return;  // the view is smaller
+    if (BWD) {
+        for (int i = threadIdx.x; i < 768; i += kAdjBlock) s_gpal[i] = 0.0f;
+        if (threadIdx.x < 4) s_acc[threadIdx.x] = 0.0f;
+    }
+    if (threadIdx.x < 16 * a.tiles) {
+        const float u = (((float)(x0 + (int)threadIdx.x) / (float)V.width) * 2.0f) - 1.0f;
+        s_col[threadIdx.x] = u * V.tan_half_fov;
+    } else if (threadIdx.x >= 128 && threadIdx.x < 144) {
+        const float W = (float)V.width, H = (float)V.height;
+        float v = (((float)(y0 + (int)threadIdx.x - 128) / H) * 2.0f) - 1.0f;
+        v = v * (H / W);
+        s_row[threadIdx.x - 128] = v * V.tan_half_fov;
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5;
+    const unsigned lane = threadIdx.x & 31u;
+    const int lx = (warp & 1) * 8 + (int)(lane & 7u), ly = (warp >> 1) * 4 + (int)(lane >> 3);
+    float lossv = 0.0f, gsun[3] = {0.0f, 0.0f, 0.0f};
+    for (int tile = 0; tile < a.tiles; ++tile) {
+        const int px = x0 + 16 * tile + lx, py = y0 + ly;
+        if (x0 + 16 * tile >= V.width) break;
+        const bool inside = px < V.width && py < V.height;
+        const size_t p = inside ? (size_t)py * V.width + px : 0;
+        bool hit = false;
+        int m = 0;
+        unsigned v = 0;
+        float c[3] = {0.0f, 0.0f, 0.0f}, shade = 0.0f, albv = 1.0f, ndl_raw = 0.0f, nrm[3] = {0.0f, 0.0f, 0.0f};
+        bool lit = false;
+        if (inside) {
+            const uint4 rec = V.hits[p];
+            hit = ((rec.w >> 16) & VT_HIT_PRIMARY) != 0;
+            if (hit) {
+                v = rec.x;
+                const float t = __uint_as_float(rec.y);
+                const unsigned face = rec.w & 0xFFu;
+                m = (int)((rec.w >> 8) & 0xFFu);
+                const int axis = (int)(face >> 1);
+                const bool pos = (face & 1u) == 0u;
+                // the primary ray (primary_ray_uv) and the shadow origin
+                const float u = s_col[16 * tile + lx], w = s_row[ly];
+                float q[3], so[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) f.pos[j] = V.pos[j];
+                for (int j = 0; j < 3; ++j) q[j] = ((u * V.view[j] + w * V.view[4 + j]) + V.view[8 + j]) + V.view[12 + j];
+                const float len = __fsqrt_rn((q[0] * q[0] + q[1] * q[1]) + q[2] * q[2]);
 #pragma unroll
-    for (int j = 0; j < 16; ++j) f.view[j] = V.view[j];
-    f.tan_half_fov = V.tan_half_fov;
-    f.width = V.width;
-    f.height = V.height;
-    shade_block<BWD, LONG>(va.a, f, V.hits, V.target, V.rgb);
+                for (int j = 0; j < 3; ++j) {
+                    float d = __fdiv_rn(q[j], len);
+                    if (d == 0.0f) d = 0.001f;   // map.glsl:85-90
+                    nrm[j] = (j == axis) ? (pos ? -1.0f : 1.0f) : 0.0f;
+                    so[j] = __fmaf_rn(d, t, V.pos[j]);
+                    if (j == axis) so[j] = so[j] + nrm[j] * 0.001f;
+                }
+                if (a.vis_in) {
+                    lit = a.vis_in[p] != 0;
+                } else {
+                    PRay rs;
+                    pray_init_dir(rs, so, a.sun_d, a.sun_inv);
+                    TraceHit hs;
+                    lit = !(GENERAL ? trace_fast<false, true, true>(a.w, a.w.cdist, rs, a.shadow_steps, hs)
+                                    : trace_ordinary<false, false>(a.w, rs, a.shadow_steps, hs)) &&
+                          !(a.w.n_entities > 0 && entity_occluded(a.w, so, a.sun_raw));
+                }
+                ndl_raw = dot3(nrm, a.sun_n);
+                const float ndl = ndl_raw > 0.0f ? ndl_raw : 0.0f;
+                shade = a.ka + a.kd * ndl * (lit ? 1.0f : 0.0f);
+                albv = a.alb ? __ldg(a.alb + v) : 1.0f;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) c[k] = (__ldg(a.pal + 3 * m + k) * albv) * shade;
+            }
+        }
+        if (!BWD) {
+            if (inside) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) V.rgb[3 * p + k] = c[k];
+                if (a.vis_out) a.vis_out[p] = (unsigned char)(hit && lit ? 1 : 0);
+            }
+            continue;
+        }
+
+        // ---- loss and gradients
+        float g[3] = {0.0f, 0.0f, 0.0f};
+        if (inside) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float diff = c[k] - __ldg(V.target + 3 * p + k);
+                g[k] = 2.0f * diff;
+                lossv += diff * diff;
+            }
+        }
+        float gp[3] = {0.0f, 0.0f, 0.0f};
+        if (hit) {
+            float ga = 0.0f, gb = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float pk = __ldg(a.pal + 3 * m + k);
+                gp[k] = g[k] * albv * shade;
+                ga += g[k] * pk * shade;
+                gb += g[k] * pk * albv;
+            }
+            if (lit && ndl_raw > 0.0f) {
+                const float coef = gb * a.kd * a.inv_len;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) gsun[k] += coef * (nrm[k] - ndl_raw * a.sun_n[k]);
+            }
+            // albedo: one global atomic per hit pixel (voxels differ across
+            // most of a warp; the L2 absorbs the few repeats)
+            if (a.galb) atomicAdd(a.galb + v, ga);
+        }
+        // palette: one shared-memory atomic per (warp, material, channel).
+        // The warp walks its distinct materials (few per warp), no divergence.
+        unsigned todo = __ballot_sync(0xFFFFFFFFu, hit);
+        while (todo) {
+            const int key = __shfl_sync(0xFFFFFFFFu, m, __ffs(todo) - 1);
+            const bool mine = hit && m == key;
+            todo &= ~__ballot_sync(0xFFFFFFFFu, mine);
+            const float s = warp_sum4(lane, mine ? gp[0] : 0.0f, mine ? gp[1] : 0.0f, mine ? gp[2] : 0.0f, 0.0f);
+            if ((lane & 7u) == 0u && lane < 24u) atomicAdd(s_gpal + 3 * key + (lane >> 3), s);
+        }
+    }
+    if (!BWD) return;
+    {
+        const float s = warp_sum4(lane, lossv, gsun[0], gsun[1], gsun[2]);
+        if ((lane & 7u) == 0u) atomicAdd(s_acc + (lane >> 3), s);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kGradSums; i += kAdjBlock) {
+        const float g = i < 768 ? s_gpal[i] : s_acc[i - 768];
+        if (g == 0.0f) continue;
+        if (a.sums) atomicAdd(a.sums + i, (double)g);
+        else atomicAdd(grad_sum(a, i), g);   // (a captured launch may be replayed beside others)
+    }
+}
+
+// Adds the launches' accumulators to the caller's and clears them.  A launch
+// of its own: the last block of the launch before would have to know itself
+// the last, and a fence in every block waits for its albedo atomics (139
+// against 130 us).
+__global__ void __launch_bounds__(kAdjBlock) k_shade_sums(AdjArgs a) {
+    for (int i = threadIdx.x; i < kGradSums; i += kAdjBlock) {
+        const double g = a.sums[i];
+        if (g != 0.0) {
+            atomicAdd(grad_sum(a, i), (float)g);
+            a.sums[i] = 0.0;
+        }
+    }
 }
 
 // Checks the arguments shared by all views, brings the distances up to date on
 // st and fills the shared part of `a` (its frame from `cam`).
-vt_status prepare_shade(vt_ctx* ctx, const vt_world* world, const vt_camera* cam, const vt_shade_inputs* in, AdjArgs& a,
-                        cudaStream_t st) {
+vt_status prepare_shade(vt_ctx* ctx, const vt_world* world, const vt_shade_inputs* in, AdjArgs& a, cudaStream_t st) {
     if (!ctx) return VT_ERR_ARG;
-    if (!world || !cam || !in || !in->d_palette) return fail(ctx, VT_ERR_ARG, "null shading argument");
+    if (!world || !in || !in->d_palette) return fail(ctx, VT_ERR_ARG, "null shading argument");
     if (world->ctx != ctx) return fail(ctx, VT_ERR_ARG, "world belongs to another context");
     const float len2 = (in->sun[0] * in->sun[0] + in->sun[1] * in->sun[1]) + in->sun[2] * in->sun[2];
     if (!(len2 > 0.0f)) return fail(ctx, VT_ERR_ARG, "sun direction must be nonzero");
@@ -247,16 +264,18 @@ vt_status prepare_shade(vt_ctx* ctx, const vt_world* world, const vt_camera* cam
         vt_status s = update_distances(const_cast<vt_world*>(world), st);
         if (s) return s;
     }
-    vt_params p;
-    vt_params_default(&p);
-    for (int j = 0; j < 3; ++j) p.sun_dir[j] = in->sun[j];
+    FrameParams f;
+    std::memset(&f, 0, sizeof(f));
+    for (int j = 0; j < 3; ++j) f.sun[j] = in->sun[j];
+    frame_constants(f);
     a.w = world->view();
-    a.f = make_frame(cam, &p);
     a.pal = in->d_palette;
     a.alb = in->d_albedo;
     for (int j = 0; j < 3; ++j) {
-        a.sun[j] = in->sun[j];
-        a.sun_n[j] = a.f.sun_n[j];
+        a.sun_raw[j] = in->sun[j];
+        a.sun_d[j] = f.sun_d[j];
+        a.sun_inv[j] = f.sun_inv[j];
+        a.sun_n[j] = f.sun_n[j];
     }
     a.inv_len = 1.0f / sqrtf(len2);
     a.ka = in->ambient;
@@ -269,20 +288,18 @@ bool camera_size_ok(const vt_camera* cam) {
     return cam->width > 0 && cam->height > 0 && cam->width <= kMaxImageSide && cam->height <= kMaxImageSide;
 }
 
-constexpr size_t kShadeSmem = 776 * sizeof(float);
-
-vt_status launch_shade(vt_ctx* ctx, const vt_world* world, const vt_camera* cam, const vt_hit* d_hits,
-                       const vt_shade_inputs* in, AdjArgs a, bool bwd, cudaStream_t st) {
-    if (!ctx) return VT_ERR_ARG;
-    if (!cam || !d_hits) return fail(ctx, VT_ERR_ARG, "null shading argument");
-    if (!camera_size_ok(cam)) return fail(ctx, VT_ERR_ARG, "camera size out of range (1..32768)");
-    vt_status s = prepare_shade(ctx, world, cam, in, a, st);
-    if (s) return s;
-    a.hits = reinterpret_cast<const uint4*>(d_hits);
-    const dim3 grid((cam->width + 15) / 16, (cam->height + 15) / 16);
-    if (bwd) k_shade<true, true><<<grid, kAdjBlock, kShadeSmem, st>>>(a);
-    else k_shade<false, true><<<grid, kAdjBlock, kShadeSmem, st>>>(a);
-    VT_CUDA(ctx, cudaGetLastError());
+// One of the context's accumulator regions for a call on st, which first waits
+// for the call that used the region last (on any stream); the caller records
+// *used after its launches.  None while st is being captured: the
+// graph's replays could overlap other launches.
+vt_status shade_sums(vt_ctx* ctx, cudaStream_t st, double** sums, cudaEvent_t* used) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    VT_CUDA(ctx, cudaStreamIsCapturing(st, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return VT_OK;
+    const unsigned r = ctx->shade_region++ % kShadeRegions;
+    VT_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_shade[r], 0));
+    *sums = reinterpret_cast<double*>(static_cast<char*>(ctx->d_shade_sums) + (size_t)r * kShadeSumBytes);
+    *used = ctx->ev_shade[r];
     return VT_OK;
 }
 
@@ -295,14 +312,22 @@ vt_status launch_shade_views(vt_ctx* ctx, const vt_world* world, int32_t n, cons
         if (!d_hits[v] || (bwd ? !d_targets[v] : !d_rgb[v])) return fail(ctx, VT_ERR_ARG, "null view buffer");
         if (!camera_size_ok(&cams[v])) return fail(ctx, VT_ERR_ARG, "camera size out of range (1..32768)");
     }
-    vt_status s = prepare_shade(ctx, world, &cams[0], in, a, st);
+    vt_status s = prepare_shade(ctx, world, in, a, st);
     if (s) return s;
+    cudaEvent_t used = nullptr;
+    if (bwd) {
+        s = shade_sums(ctx, st, &a.sums, &used);
+        if (s) return s;
+    }
+    const bool general = a.shadow_steps > kChunkSteps || !ordinary_inv(a.sun_inv);
+    auto k = bwd ? (general ? k_shade_views<true, true> : k_shade_views<true, false>)
+                 : (general ? k_shade_views<false, true> : k_shade_views<false, false>);
     ViewsArgs va;
     std::memset(&va, 0, sizeof(va));
-    va.a = a;
     for (int v0 = 0; v0 < n; v0 += kMaxViews) {
         const int nv = n - v0 < kMaxViews ? n - v0 : kMaxViews;
         int gw = 0, gh = 0;
+        size_t tiles = 0;
         for (int i = 0; i < nv; ++i) {
             const vt_camera& c = cams[v0 + i];
             ViewP& V = va.v[i];
@@ -316,13 +341,23 @@ vt_status launch_shade_views(vt_ctx* ctx, const vt_world* world, int32_t n, cons
             V.rgb = bwd ? nullptr : d_rgb[v0 + i];
             gw = c.width > gw ? c.width : gw;
             gh = c.height > gh ? c.height : gh;
+            tiles += (size_t)((c.width + 15) / 16) * (size_t)((c.height + 15) / 16);
         }
-        const dim3 grid((gw + 15) / 16, (gh + 15) / 16, nv);
-        const bool lng = a.shadow_steps > kChunkSteps;
-        auto k = bwd ? (lng ? k_shade_views<true, true> : k_shade_views<true, false>)
-                     : (lng ? k_shade_views<false, true> : k_shade_views<false, false>);
-        k<<<grid, kAdjBlock, kShadeSmem, st>>>(va);
+        // A backward block's clearing and flushing is shared by up to four
+        // tiles (16 views of 512x512: 1 tile 280 us an iteration, 2 and 4 256
+        // us; the forward kernel has nothing to share and is slower), as long
+        // as the launch keeps 24 blocks per SM, four waves.
+        a.tiles = 1;
+        while (bwd && a.tiles < kMaxTiles && tiles / (size_t)(2 * a.tiles) >= (size_t)(24 * ctx->sm_count)) a.tiles *= 2;
+        va.a = a;
+        const dim3 grid((gw + 16 * a.tiles - 1) / (16 * a.tiles), (gh + 15) / 16, nv);
+        k<<<grid, kAdjBlock, 0, st>>>(va);
         VT_CUDA(ctx, cudaGetLastError());
+    }
+    if (a.sums) {
+        k_shade_sums<<<1, kAdjBlock, 0, st>>>(a);
+        VT_CUDA(ctx, cudaGetLastError());
+        VT_CUDA(ctx, cudaEventRecord(used, st));
     }
     return VT_OK;
 }
@@ -344,8 +379,8 @@ vt_status vt_shade_forward(vt_ctx* ctx, const vt_world* world, const vt_camera* 
     std::memset(&a, 0, sizeof(a));
     a.vis_in = d_vis_in;
     a.vis_out = d_vis_out;
-    a.rgb = d_rgb;
-    return launch_shade(ctx, world, cam, d_hits, in, a, false, (cudaStream_t)stream);
+    if (!cam || !d_hits) return fail(ctx, VT_ERR_ARG, "null shading argument");
+    return launch_shade_views(ctx, world, 1, cam, &d_hits, in, nullptr, &d_rgb, a, false, (cudaStream_t)stream);
 }
 
 vt_status vt_shade_backward(vt_ctx* ctx, const vt_world* world, const vt_camera* cam, const vt_hit* d_hits,
@@ -356,12 +391,12 @@ vt_status vt_shade_backward(vt_ctx* ctx, const vt_world* world, const vt_camera*
         return fail(ctx, VT_ERR_ARG, "null target, loss or gradient buffer");
     AdjArgs a;
     std::memset(&a, 0, sizeof(a));
-    a.target = d_target;
     a.loss = d_loss;
     a.gpal = d_grad_palette;
     a.galb = d_grad_albedo;
     a.gsun = d_grad_sun;
-    return launch_shade(ctx, world, cam, d_hits, in, a, true, (cudaStream_t)stream);
+    if (!cam || !d_hits) return fail(ctx, VT_ERR_ARG, "null shading argument");
+    return launch_shade_views(ctx, world, 1, cam, &d_hits, in, &d_target, nullptr, a, true, (cudaStream_t)stream);
 }
 
 vt_status vt_shade_forward_views(vt_ctx* ctx, const vt_world* world, int32_t n, const vt_camera* cams,

@@ -723,7 +723,7 @@ constexpr int kChunkSteps = 1024;
 
 // A ray the forward walk takes: near origin, and reciprocals in
 // [2^-100, 2^100] in magnitude (so no plane time overflows or is NaN).
-__device__ __forceinline__ bool ordinary_inv(const float inv[3]) {
+__host__ __device__ __forceinline__ bool ordinary_inv(const float inv[3]) {
     const float a = fabsf(inv[0]), b = fabsf(inv[1]), c = fabsf(inv[2]);
     return a <= 0x1p100f && b <= 0x1p100f && c <= 0x1p100f && a >= 0x1p-100f && b >= 0x1p-100f && c >= 0x1p-100f;
 }
@@ -897,23 +897,28 @@ struct FwdWalk {
     }
 };
 
+// Traces a ray that passes near_origin and ordinary_inv to its end.
+template <bool MAT, bool LONG>
+__device__ __forceinline__ bool trace_ordinary(const WorldView& w, const PRay& r, int max_steps, TraceHit& h) {
+    FwdWalk fw;
+    if (!fw.start(w, r, max_steps)) return false;
+    unsigned wi = 0, vb = 0;
+    int s;
+    while ((s = fw.step<LONG>(w, wi, vb)) == FwdWalk::kMore) {
+    }
+    if (s != FwdWalk::kHit) return false;
+    fw.hit<MAT>(w, r, wi, vb, h);
+    return true;
+}
+
 // Traces one ray to its end.  NEAR: the origin passes near_origin; SHARE:
 // brick words shared between the lanes of a warp (Walker only); LONG: step
 // limits above kChunkSteps (chunk jumps; without them only speed is lost).
 template <bool MAT, bool RUN = true, bool NEAR = false, bool SHARE = false, bool LONG = true>
 __device__ __forceinline__ bool trace_fast(const WorldView& w, const unsigned char* cdist, const PRay& r,
                                            int max_steps, TraceHit& h) {
+    if (NEAR && RUN && !SHARE && ordinary_inv(r.inv)) return trace_ordinary<MAT, LONG>(w, r, max_steps, h);
     int s;
-    if (NEAR && RUN && !SHARE && ordinary_inv(r.inv)) {
-        FwdWalk fw;
-        if (!fw.start(w, r, max_steps)) return false;
-        unsigned wi = 0, vb = 0;
-        while ((s = fw.step<LONG>(w, wi, vb)) == FwdWalk::kMore) {
-        }
-        if (s != FwdWalk::kHit) return false;
-        fw.hit<MAT>(w, r, wi, vb, h);
-        return true;
-    }
     Walker wk;
     if (!wk.start_ray(w, r, max_steps)) return false;
     while ((s = wk.step<MAT, RUN, NEAR, SHARE>(w, cdist, h)) == Walker::kMore) {

@@ -100,6 +100,10 @@ struct ScreenTable {
     float4* d = nullptr;
 };
 constexpr int kScreenTables = 8;
+// Accumulator regions of the shading gradients (adjoint.cu): calls of a
+// context that may be in flight at once (more wait), and bytes each.
+constexpr unsigned kShadeRegions = 8;
+constexpr size_t kShadeSumBytes = 6400;
 }  // namespace vt
 
 struct vt_ctx {
@@ -138,6 +142,9 @@ struct vt_ctx {
     unsigned* d_bounce_ctr = nullptr;  // {queued, taken}
     size_t bounce_capacity = 0;
     cudaEvent_t ev_bounce = nullptr;   // the last deferred frame is done with the queue
+    void* d_shade_sums = nullptr;      // kShadeRegions accumulator regions, zero between calls
+    unsigned shade_region = 0;
+    cudaEvent_t ev_shade[vt::kShadeRegions] = {};
     // screen tables of the frame sizes rendered so far (see screen_table)
     vt::ScreenTable screen[vt::kScreenTables];
     int n_screen = 0;
