@@ -53,7 +53,9 @@ constexpr unsigned kLaunchBlocks = 16384;
 // Per-job camera fields of a tile-shape launch.
 struct JobCam {
     float pos[3];
-    float view[16];
+    float cam_c[3];   // FrameParams
+    int cam_inside;
+    float view[12];   // the four rows' x, y, z
     float tan_half_fov;
     int width, height;
     const float4* screen;
@@ -92,7 +94,10 @@ __global__ void __launch_bounds__(kBatchBlock, 4) k_render_jobs(const __grid_con
 #pragma unroll
     for (int k = 0; k < 3; ++k) f.pos[k] = jc.pos[k];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) f.view[k] = jc.view[k];
+    for (int k = 0; k < 3; ++k) f.cam_c[k] = jc.cam_c[k];
+    f.cam_inside = jc.cam_inside;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) f.view[4 * (k / 3) + k % 3] = jc.view[k];
     f.tan_half_fov = jc.tan_half_fov;
     f.width = jc.width;
     f.height = jc.height;
@@ -204,6 +209,7 @@ vt_status build_chunks(vt_batch* b) {
     for (size_t i = 0; i < b->jobs.size(); ++i) {
         const vt_job& j = b->jobs[i];
         FrameParams f = make_frame(&j.camera, &b->params);
+        walk_constants(f, j.world->view());
         vt_status s = screen_table(ctx, f, ctx->stream, true, &f.screen);
         if (s) return s;
         const unsigned long long job_blocks = (unsigned long long)((j.camera.width + kUnit - 1) / kUnit) *
@@ -219,7 +225,9 @@ vt_status build_chunks(vt_batch* b) {
         const int n = c->njobs++;
         JobCam& jc = c->cam[n];
         for (int k = 0; k < 3; ++k) jc.pos[k] = f.pos[k];
-        for (int k = 0; k < 16; ++k) jc.view[k] = f.view[k];
+        for (int k = 0; k < 3; ++k) jc.cam_c[k] = f.cam_c[k];
+        jc.cam_inside = f.cam_inside;
+        for (int k = 0; k < 12; ++k) jc.view[k] = f.view[4 * (k / 3) + k % 3];
         jc.tan_half_fov = f.tan_half_fov;
         jc.width = f.width;
         jc.height = f.height;
@@ -279,6 +287,7 @@ vt_status vt_batch_create(vt_ctx* ctx, const vt_job* jobs, int32_t n, const vt_p
         JobDesc& d = host[(size_t)i];
         d.w = j.world->view();
         d.f = make_frame(&j.camera, params);
+        walk_constants(d.f, d.w);
         d.out = reinterpret_cast<uint4*>(j.d_out);
         d.first_unit = (unsigned)units;
         d.units_x = (unsigned)((j.camera.width + kUnit - 1) / kUnit);

@@ -49,7 +49,7 @@ struct BlockTile {
 // sorted by direction (stage_flush).
 template <bool STATS, bool CHECKED, bool SMEM, int TW, bool OCC, bool SHARE = false, bool BIN = false, bool BOUNCE = true,
           bool LONG = true>
-__global__ void __launch_bounds__(kBlock, OCC ? kOccBlocks : 1) k_render(WorldView w, FrameParams f, uint4* __restrict__ out,
+__global__ void __launch_bounds__(kBlock, OCC ? kOccBlocks : 1) k_render(const __grid_constant__ WorldView w, const __grid_constant__ FrameParams f, uint4* __restrict__ out,
                                                                unsigned* status, unsigned long long* counters) {
     // shared copy of the coarse bits for the model traversal (STATS or
     // CHECKED); the production walk reads the chunk distances through L1,
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kBlock, OCC ? kOccBlocks : 1) k_render(WorldVi
 
 // Explicit ray list (production traversal); record.rgba is 0.
 template <bool LONG>
-__global__ void __launch_bounds__(kBlock) k_trace_rays(WorldView w, const float* __restrict__ origins,
+__global__ void __launch_bounds__(kBlock) k_trace_rays(const __grid_constant__ WorldView w, const float* __restrict__ origins,
                                                        const float* __restrict__ dirs, int n, int max_steps,
                                                        uint4* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -243,11 +243,10 @@ __global__ void __launch_bounds__(kPersistBlock) k_render_persist(WorldView w, F
                 finish = true;
             }
             if (finish) {
-                const unsigned alb = __ldg(w.palette + mat);
                 float col[4];
-                shade_hit(f, alb, e_hit, pe_hit, (flags & VT_HIT_SHADOWED) != 0,
+                shade_hit(f, albedo_of(w, mat), e_hit, pe_hit, (flags & VT_HIT_SHADOWED) != 0,
                           (f.rays & VT_RAYS_BOUNCE) && !(flags & VT_HIT_BOUNCE), bdir, col);
-                const unsigned rgba = f.shade == VT_SHADE_NONE ? alb : composite(f, px, py, col);
+                const unsigned rgba = f.shade == VT_SHADE_NONE ? __ldg(w.palette + mat) : composite(f, px, py, col);
                 out[(size_t)py * f.width + px] =
                     make_uint4(voxel, __float_as_uint(thit), rgba, face | (mat << 8) | (flags << 16));
                 need_pixel = true;
@@ -318,6 +317,29 @@ FrameParams make_frame(const vt_camera* cam, const vt_params* p) {
     f.bounce_weight = p->bounce_weight;
     frame_constants(f);
     return f;
+}
+
+void walk_constants(FrameParams& f, const WorldView& w) {
+    f.cam_inside = near_origin(f.pos) ? 1 : 0;
+    for (int j = 0; j < 3; ++j) {
+        f.in_hi[j] = (float)(w.dims[j] - 1);
+        if (!(f.pos[j] >= 1.0f && f.pos[j] <= f.in_hi[j])) f.cam_inside = 0;
+    }
+    for (int j = 0; j < 3; ++j) f.cam_c[j] = f.cam_inside ? floorf(f.pos[j]) : 0.0f;
+    unsigned oct = 0;
+    f.sun_flip = 0;
+    for (int j = 0; j < 3; ++j) {
+        const bool up = f.sun_d[j] > 0.0f;
+        f.sun_m[j] = up ? 0 : -1;
+        f.sun_side[j] = up ? 1.0f : -1.0f;
+        f.sun_off[j] = up ? 1.0f : 0.0f;
+        f.sun_ad[j] = fabsf(f.sun_d[j]);
+        f.sun_ai[j] = fabsf(f.sun_inv[j]);
+        f.sun_exit[j] = up ? (float)w.dims[j] : 0.0f;
+        if (up) oct |= 1u << j;
+        else f.sun_flip |= 3u << (2 * j);
+    }
+    f.sun_field = oct * w.nwords;
 }
 
 vt_status check_frame_args(vt_ctx* ctx, const vt_world* world, const vt_camera* cam, const vt_params* p) {
@@ -412,6 +434,7 @@ vt_status launch_render(vt_ctx* ctx, const vt_world* world, const vt_camera* cam
     f.row_end = row1;
     const int rows = row1 - row0;
     const WorldView w = world->view();
+    walk_constants(f, w);
     const bool checked = (p->flags & VT_FLAG_CHECKED) != 0;
     const size_t smem = (size_t)w.ncoarse * sizeof(unsigned long long);
     const bool use_smem = (stats || checked) && smem <= kMaxSharedCoarse;

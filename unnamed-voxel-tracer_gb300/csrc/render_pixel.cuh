@@ -10,9 +10,9 @@
 namespace vt {
 
 // Whether some ray kind of the frame may walk far enough for chunk jumps to
-// pay.
+// pay, or the sun's direction is not one the forward walk takes.
 inline bool long_steps(const FrameParams& f) {
-    return f.max_steps > kChunkSteps || f.shadow_max_steps > kChunkSteps || f.bounce_max_steps > kChunkSteps;
+    return f.max_steps > kChunkSteps || f.shadow_max_steps > kChunkSteps || f.bounce_max_steps > kChunkSteps || !ordinary_inv(f.sun_inv);
 }
 
 struct PixelCounters {
@@ -34,6 +34,58 @@ __device__ __forceinline__ bool trace_any(const WorldView& w, const Coarse& coar
     return trace_fast<MAT, true, false, SHARE, LONG>(w, cd, r, max_steps, h);
 }
 
+// The primary ray of a frame whose camera is inside the grid: its cell is the
+// frame's (walk_constants).
+template <bool LONG>
+__device__ __forceinline__ bool trace_primary(const WorldView& w, const FrameParams& f, const PRay& r, TraceHit& h) {
+    FwdWalk fw;
+    bool go;
+    if (f.cam_inside) {   // uniform
+        fw.t = 0.0f;
+        go = fw.start_cell(w, r, f.cam_c, f.max_steps);
+    } else {
+        go = fw.start(w, r, f.max_steps);
+    }
+    return go && fw.finish<true, LONG>(w, r, h);
+}
+
+// The shadow ray from so: the fields of its walk that depend on the sun alone
+// are the frame's (walk_constants), and an origin at least one cell inside
+// the grid starts in its own cell (pray_start).
+template <bool LONG>
+__device__ __forceinline__ bool trace_sun(const WorldView& w, const FrameParams& f, const float so[3]) {
+    PRay r;
+    pray_init_dir(r, so, f.sun_d, f.sun_inv);
+    TraceHit h;
+    FwdWalk fw;
+    const bool inside = so[0] >= 1.0f && so[1] >= 1.0f && so[2] >= 1.0f && so[0] <= f.in_hi[0] && so[1] <= f.in_hi[1] &&
+                        so[2] <= f.in_hi[2];
+    bool go = true;
+    if (inside) {
+        if (f.shadow_max_steps <= 0) return false;
+        fw.t = 0.0f;
+        float x[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            fw.m[i] = f.sun_m[i];
+            fw.d[i] = f.sun_ad[i];
+            fw.a[i] = f.sun_ai[i];
+            fw.b[i] = r.oinv[i];
+            fw.o[i] = __fmaf_rn(so[i], f.sun_side[i], -0.25f);
+            fw.nk[i] = __fmaf_rn(magic_floor(so[i]) - kMagic, f.sun_side[i], f.sun_off[i]);
+            fw.tm[i] = __fmaf_rn(fw.nk[i], fw.a[i], fw.b[i]);
+            x[i] = __fmaf_rn(f.sun_exit[i], fw.a[i], fw.b[i]);
+        }
+        fw.texit = fminf(fminf(x[0], x[1]), x[2]);
+        fw.limit = ((fw.nk[0] + fw.nk[1]) + fw.nk[2]) + __int2float_rn(min(f.shadow_max_steps, 1 << 20));
+        fw.flip = f.sun_flip;
+        fw.field = f.sun_field;
+    } else {
+        go = fw.start(w, r, f.shadow_max_steps);
+    }
+    return go && fw.finish<false, LONG>(w, r, h);
+}
+
 // uv: the pixel's screen coordinates (pixel_uv(f, px, py); the frame kernel
 // reads them from the frame's screen table or its per-block tables).
 // BIN: a deferred bounce ray is staged in the block's shared memory for the
@@ -52,7 +104,10 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
     pray_init(r, o, d);
     TraceHit h;
     TraceCounters cnt;
-    const bool hit = trace_any<STATS, CHECKED, true, false, SHARE, LONG>(w, coarse, cd, r, f.max_steps, h, cnt, status);
+    constexpr bool kForward = !STATS && !CHECKED && !SHARE;
+    const bool hit = kForward && (f.cam_inside || near_origin(r.o)) && ordinary_inv(r.inv)
+                         ? trace_primary<LONG>(w, f, r, h)
+                         : trace_any<STATS, CHECKED, true, false, SHARE, LONG>(w, coarse, cd, r, f.max_steps, h, cnt, status);
     if (STATS) {
         pc.v[0] += 1;
         pc.v[9] += 16;
@@ -68,7 +123,7 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
         const bool pe = e == 0 ? r.pos[0] : (e == 1 ? r.pos[1] : r.pos[2]);
         face = 2u * (unsigned)e + (pe ? 0u : 1u);
         mat = h.mat;
-        const unsigned alb = __ldg(w.palette + mat);
+        const float4 alb = albedo_of(w, mat);
         if (STATS) {
             pc.v[1] += 1;
             pc.v[8] += 1;
@@ -82,10 +137,14 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
         }
         bool shadowed = false;
         if (f.rays & VT_RAYS_SHADOW) {
-            PRay rs;
-            pray_init_dir(rs, so, f.sun_d, f.sun_inv);
-            TraceHit hs;
-            shadowed = trace_any<STATS, CHECKED, false, true, SHARE, LONG>(w, coarse, cd, rs, f.shadow_max_steps, hs, cnt, status);
+            if (kForward && (!LONG || ordinary_inv(f.sun_inv))) {
+                shadowed = trace_sun<LONG>(w, f, so);
+            } else {
+                PRay rs;
+                pray_init_dir(rs, so, f.sun_d, f.sun_inv);
+                TraceHit hs;
+                shadowed = trace_any<STATS, CHECKED, false, true, SHARE, LONG>(w, coarse, cd, rs, f.shadow_max_steps, hs, cnt, status);
+            }
             if (shadowed) flags |= VT_HIT_SHADOWED;
             if (STATS) {
                 pc.v[2] += 1;
@@ -108,7 +167,7 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
             // traced by the bounce kernel (bounce.cu).  The record assumes a
             // hit; a ray that leaves turns it into the open colour
             shade_hit(f, alb, e, pe, shadowed, true, bdir, col);
-            const unsigned open = f.shade == VT_SHADE_NONE ? alb : composite_uv(f, uv, col);
+            const unsigned open = f.shade == VT_SHADE_NONE ? __ldg(w.palette + mat) : composite_uv(f, uv, col);
             const BounceJob job = bounce_job(so, bdir, (unsigned)py * (unsigned)f.width + (unsigned)px, flags, open);
             if (BIN) stage_bounce(job);
             else append_bounce(f, job);
@@ -126,7 +185,7 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
             }
         }
         shade_hit(f, alb, e, pe, shadowed, bounce_open, bdir, col);
-        rgba = f.shade == VT_SHADE_NONE ? alb : composite_uv(f, uv, col);
+        rgba = f.shade == VT_SHADE_NONE ? __ldg(w.palette + mat) : composite_uv(f, uv, col);
     } else {
         shade_miss(f, d, col);
         rgba = f.shade == VT_SHADE_NONE ? 0u : composite_uv(f, uv, col);

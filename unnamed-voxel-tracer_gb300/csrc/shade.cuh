@@ -33,6 +33,17 @@ struct FrameParams {
     float lit_a;        // illumination alpha 0.3 stored in RGBA8
     float sun_d[3];     // the shadow rays' direction as traced (a zero component made 0.001, map.glsl:85-90)
     float sun_inv[3];   // its correctly rounded reciprocal
+    // of the frame's world (walk_constants): where the camera's rays start,
+    // and the shadow rays' fields of FwdWalk, the same for all of them
+    int cam_inside;     // the camera is near and at least one cell inside the grid:
+    float cam_c[3];     // its cell
+    float in_hi[3];     // the grid's sides less one
+    int sun_m[3];       // 0, or -1 where it moves down the axis
+    float sun_side[3];  // 1, or -1 where the shadow ray moves down the axis
+    float sun_off[3];   // 1 or 0: the plane after cell c is sun_side * c + sun_off
+    float sun_ad[3], sun_ai[3];  // |sun_d|, |sun_inv|
+    float sun_exit[3];  // the grid's last plane, mirrored
+    unsigned sun_flip, sun_field;
     float cross_r2;     // the largest x with sqrt(x) <= 0.002 (crosshair radius test without a square root)
     int row0, row_end;  // rows [row0, row_end) of the image this launch renders
     void* bounce_head;       // non-null: bounce rays are queued here (BounceHead), not traced inline
@@ -142,7 +153,24 @@ __device__ __forceinline__ bool entity_occluded(const WorldView& w, const float 
 // and square root on both sides, no contraction).
 __host__ __device__ __forceinline__ float clampf(float x, float a, float b) { return x < a ? a : (x > b ? b : x); }
 
-__host__ __device__ __forceinline__ unsigned unorm8(float x) { return (unsigned)(int)rintf(clampf(x, 0.0f, 1.0f) * 255.0f); }
+// round(clamp(x, 0, 1) * 255), ties to even; 0 for NaN.  The device's saturate
+// is the clamp (NaN to 0), and adding 1.5 * 2^23 rounds as rintf does and
+// leaves the integer in the low bits.
+__host__ __device__ __forceinline__ unsigned unorm8(float x) {
+#ifdef __CUDA_ARCH__
+    return __float_as_uint(__saturatef(x) * 255.0f + 12582912.0f) & 255u;
+#else
+    return (unsigned)(int)rintf(clampf(x, 0.0f, 1.0f) * 255.0f);
+#endif
+}
+
+// Four of them, the first in the low byte.
+__device__ __forceinline__ unsigned pack_unorm8(const float c[4]) {
+    unsigned b[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = __float_as_uint(__saturatef(c[j]) * 255.0f + 12582912.0f);
+    return __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+}
 
 __host__ __device__ __forceinline__ float dot3(const float a[3], const float b[3]) { return (a[0] * b[0] + a[1] * b[1]) + a[2] * b[2]; }
 
@@ -246,12 +274,15 @@ __device__ __forceinline__ void cosine_hemisphere(const float n[3], unsigned& se
     normalize3(v, out);
 }
 
+// A material's albedo, channels / 255.
+__device__ __forceinline__ float4 albedo_of(const WorldView& w, unsigned mat) {
+    return __ldg(reinterpret_cast<const float4*>(w.palette + 256) + mat);
+}
+
 // Colour of a primary hit in REFERENCE / LAMBERT / NONE shading.
-__device__ __forceinline__ void shade_hit(const FrameParams& f, unsigned alb, int axis, bool pos_axis, bool shadowed,
+__device__ __forceinline__ void shade_hit(const FrameParams& f, const float4 alb, int axis, bool pos_axis, bool shadowed,
                                           bool bounce_open, const float bdir[3], float col[4]) {
-    float albf[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) albf[j] = unorm8_to_float((alb >> (8 * j)) & 255u);
+    const float albf[4] = {alb.x, alb.y, alb.z, alb.w};
     if (f.shade == VT_SHADE_REFERENCE) {
         const float a = shadowed ? 0.0f : f.lit_a;
 #pragma unroll
@@ -306,7 +337,7 @@ __device__ __forceinline__ unsigned composite_uv(const FrameParams& f, const Pix
             for (int j = 0; j < 4; ++j) col[j] = g * col[j];
         }
     }
-    return unorm8(col[0]) | (unorm8(col[1]) << 8) | (unorm8(col[2]) << 16) | (unorm8(col[3]) << 24);
+    return pack_unorm8(col);
 }
 
 __device__ __forceinline__ unsigned composite(const FrameParams& f, int px, int py, float col[4]) {
@@ -315,6 +346,10 @@ __device__ __forceinline__ unsigned composite(const FrameParams& f, int px, int 
 
 // FrameParams of a camera and parameter set (render.cu).
 FrameParams make_frame(const vt_camera* cam, const vt_params* p);
+
+// The constants that depend on the frame's world too (host side; after the
+// camera's and frame_constants).
+void walk_constants(FrameParams& f, const WorldView& w);
 
 // The per-frame constants of FrameParams (host side).
 inline void frame_constants(FrameParams& f) {

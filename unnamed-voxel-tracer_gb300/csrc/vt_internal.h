@@ -26,7 +26,7 @@ struct WorldView {
     const unsigned long long* mask;     // brick occupancy words, chunk-major
     const unsigned char* mats;          // 64 material bytes per brick, same order
     const unsigned long long* coarse;   // one bit per chunk
-    const unsigned* palette;            // 256 RGBA8
+    const unsigned* palette;            // 256 RGBA8, then the same as 256 float4 of channel / 255
     const unsigned char* bdist;         // kOctants fields of nwords bytes (octant-major), per brick:
                                         // 0 if occupied, else (E + 1) | shape << 6: the brick plus E
                                         // voxel layers ahead in that octant (E >> shape vertically)
@@ -84,6 +84,8 @@ __host__ __device__ constexpr int box_score(int s, int shape) {
 }
 // Capacity of a world's entity box list.
 constexpr int kMaxEntities = 1024;
+// Bytes of a world's device palette: 256 RGBA8 words, then 256 float4.
+constexpr size_t kPaletteBytes = 256 * (sizeof(unsigned) + 4 * sizeof(float));
 // Largest image width and height a frame may have.
 constexpr int kMaxImageSide = 32768;
 

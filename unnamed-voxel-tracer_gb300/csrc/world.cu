@@ -562,6 +562,18 @@ vt_status world_stage(vt_world* w, size_t bytes, unsigned char** out) {
     return VT_OK;
 }
 
+// The palette as given, and its channels / 255 (correctly rounded, as the
+// shading's table): a hit's albedo is then one 16-byte load.
+static cudaError_t upload_palette(vt_world* w, const uint32_t* rgba) {
+    unsigned char bytes[kPaletteBytes];
+    std::memcpy(bytes, rgba, 256 * sizeof(uint32_t));
+    for (int i = 0; i < 1024; ++i) {
+        const float v = (float)((rgba[i >> 2] >> (8 * (i & 3))) & 255u) / 255.0f;
+        std::memcpy(bytes + 256 * sizeof(uint32_t) + i * sizeof(float), &v, sizeof(float));
+    }
+    return cudaMemcpy(w->d_palette, bytes, sizeof(bytes), cudaMemcpyHostToDevice);
+}
+
 static void free_world(vt_world* w) {
     if (w->d_mask) vt::dev_free(w->d_mask);
     if (w->d_mats) vt::dev_free(w->d_mats);
@@ -606,7 +618,7 @@ vt_status vt_world_create(vt_ctx* ctx, const vt_world_desc* desc, vt_world** out
     if ((e = vt::dev_alloc(&w->d_mask, w->nchunks * kBricksPerChunk * 8)) != cudaSuccess ||
         (e = vt::dev_alloc(&w->d_mats, w->nchunks * (size_t)kChunkBytes)) != cudaSuccess ||
         (e = vt::dev_alloc(&w->d_coarse, w->ncoarse * 8)) != cudaSuccess ||
-        (e = vt::dev_alloc(&w->d_palette, 256 * sizeof(unsigned))) != cudaSuccess ||
+        (e = vt::dev_alloc(&w->d_palette, kPaletteBytes)) != cudaSuccess ||
         (e = vt::dev_alloc(&w->d_bdist, kOctants * w->nchunks * kBricksPerChunk)) != cudaSuccess ||
         (e = vt::dev_alloc(&w->d_cdist, kOctants * (size_t)cdist_stride((unsigned)w->nchunks))) != cudaSuccess ||
         (e = vt::dev_alloc(&w->d_dtmp, (32 + 4 * kYFields) * w->nchunks * kBricksPerChunk)) != cudaSuccess ||
@@ -622,7 +634,7 @@ vt_status vt_world_create(vt_ctx* ctx, const vt_world_desc* desc, vt_world** out
     }
     uint32_t pal[256];
     vt_default_palette(pal);
-    if ((e = cudaMemcpy(w->d_palette, pal, sizeof(pal), cudaMemcpyHostToDevice)) != cudaSuccess) {
+    if ((e = upload_palette(w, pal)) != cudaSuccess) {
         free_world(w);
         return check_cuda(ctx, e, "palette upload");
     }
@@ -713,7 +725,7 @@ vt_status vt_world_get_voxel(vt_world* w, int32_t x, int32_t y, int32_t z, uint8
 vt_status vt_world_set_palette(vt_world* w, const uint32_t* h_rgba256) {
     if (!w) return VT_ERR_ARG;
     if (!h_rgba256) return fail(w->ctx, VT_ERR_ARG, "null palette");
-    VT_CUDA(w->ctx, cudaMemcpy(w->d_palette, h_rgba256, 256 * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    VT_CUDA(w->ctx, upload_palette(w, h_rgba256));
     return VT_OK;
 }
 
