@@ -9,6 +9,7 @@
 // the edited voxel in device memory, from where the distance passes that
 // follow on the stream update the empty-space distances around it.  Nothing
 // goes back to the host between the pick and the edit.
+#include "dist.cuh"
 #include "render_pixel.cuh"
 #include "vt_internal.h"
 
@@ -42,7 +43,8 @@ __device__ __forceinline__ void center_ray(const PickRay& f, float o[3], float d
 // receives {x, y, z, valid, whether a coarse bit changed} of the voxel written.
 __global__ void __launch_bounds__(512) k_pick_edit(WorldView w, unsigned long long* mask, unsigned char* mats,
                                                    unsigned long long* coarse, PickRay f, int max_steps, int edit_mode,
-                                                   uint4* __restrict__ out, int* __restrict__ d_edit) {
+                                                   uint4* __restrict__ out, int* __restrict__ d_edit, BrickGrid grid,
+                                                   unsigned char* __restrict__ xf) {
     __shared__ int target[4];
     if (threadIdx.x == 0) {
         float o[3], d[3];
@@ -50,7 +52,8 @@ __global__ void __launch_bounds__(512) k_pick_edit(WorldView w, unsigned long lo
         PRay r;
         pray_init(r, o, d);
         TraceHit h;
-        const bool hit = trace_fast<true>(w, w.cdist, r, max_steps, h);
+        const bool hit = near_origin(o) ? trace_fast<true, true, true>(w, w.cdist, r, max_steps, h)
+                                        : trace_fast<true, true, false>(w, w.cdist, r, max_steps, h);
         target[3] = 0;
         if (hit) {
             const int e = h.axis;
@@ -75,9 +78,11 @@ __global__ void __launch_bounds__(512) k_pick_edit(WorldView w, unsigned long lo
             d_edit[1] = target[1];
             d_edit[2] = target[2];
             d_edit[3] = target[3];
-            d_edit[4] = 0;
+            d_edit[kEditCoarse] = 0;
         }
     }
+    if (d_edit)
+        for (int i = threadIdx.x; i < kEditGroups * kEditRows; i += 512) d_edit[kEditColumns + i] = 0;
     __syncthreads();
     if (!target[3]) return;
     const int x = target[0], y = target[1], z = target[2];
@@ -95,8 +100,15 @@ __global__ void __launch_bounds__(512) k_pick_edit(WorldView w, unsigned long lo
     if (threadIdx.x == 0) {
         const unsigned long long bit = 1ull << (ci & 63u);
         const unsigned long long was = any ? atomicOr(coarse + (ci >> 6), bit) : atomicAnd(coarse + (ci >> 6), ~bit);
-        d_edit[4] = ((was & bit) != 0ull) != (any != 0) ? 1 : 0;   // the chunk distances are stale
+        d_edit[kEditCoarse] = ((was & bit) != 0ull) != (any != 0) ? 1 : 0;   // the chunk distances are stale
     }
+    // the x pass of the brick distances on the edited brick's rows (a launch
+    // of its own for 24 threads' work otherwise)
+    const int bx = (x >> 2) - kEditReach, n = 2 * kEditReach + 1;
+    int cx, by, qz;
+    if (box_item(threadIdx.x, make_int3(bx, y >> 2, z & ~3), make_int3(n, 1, 4), 8, make_int3(grid.GX, grid.GY, 4 * grid.GZ),
+                 cx, by, qz))
+        bdist_x_item<true>(mask, xf, grid, cx, by, qz);
 }
 
 PickRay pick_ray(const vt_camera* cam) {
@@ -116,7 +128,10 @@ vt_status launch_pick(vt_ctx* ctx, vt_world* world, const vt_camera* cam, int32_
     vt_status s = update_distances(world, st);  // the pick walks the current distances
     if (s) return s;
     k_pick_edit<<<1, 512, 0, st>>>(world->view(), world->d_mask, world->d_mats, world->d_coarse, pick_ray(cam), max_steps,
-                                   edit_mode, reinterpret_cast<uint4*>(d_out), edit_mode >= 0 ? world->d_edit : nullptr);
+                                   edit_mode, reinterpret_cast<uint4*>(d_out), edit_mode >= 0 ? world->d_edit : nullptr,
+                                   BrickGrid{world->cdim[0], world->cdim[1], world->cdim[2], world->cdim[0] * 8,
+                                             world->cdim[1] * 8, world->cdim[2] * 8},
+                                   world->d_dtmp);
     VT_CUDA(ctx, cudaGetLastError());
     if (edit_mode >= 0) return update_distances_at(world, world->d_edit, st);
     return VT_OK;

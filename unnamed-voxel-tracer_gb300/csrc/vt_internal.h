@@ -82,6 +82,15 @@ constexpr int kBoxShapes = 4;
 __host__ __device__ constexpr int box_score(int s, int shape) {
     return (s + 3) * (s + 3) * (((s - 1) >> shape) + 4);
 }
+// An edit changes brick distances at most this many bricks away (a pass reads
+// at most kVoxCap + 3 layers past a brick's near face).
+constexpr int kEditReach = (kVoxCap + 3) / 4;
+// vt_world::d_edit: {x, y, z, valid} of the last device-side edit, whether it
+// changed a coarse bit, and per group of four bricks in x and brick in y of
+// its box whether the y pass changed its distances.
+constexpr int kEditCoarse = 4, kEditColumns = 8;
+constexpr int kEditGroups = (2 * kEditReach + 1 + 3) / 4 + 1, kEditRows = 2 * kEditReach + 1;
+constexpr int kEditInts = kEditColumns + kEditGroups * kEditRows;
 // Capacity of a world's entity box list.
 constexpr int kMaxEntities = 1024;
 // Bytes of a world's device palette: 256 RGBA8 words, then 256 float4.
@@ -173,7 +182,7 @@ struct vt_world {
     unsigned char* d_cdist = nullptr;
     unsigned char* d_dtmp = nullptr;   // x (2 fields, 16 B/brick) and y (10 fields, 4 B/brick) pass results of the brick distances (kept)
     unsigned char* d_ctmp = nullptr;   // the same 6 fields for the chunk distances
-    int* d_edit = nullptr;             // {x, y, z, valid, coarse bit changed} of the last device-side edit
+    int* d_edit = nullptr;             // the last device-side edit (kEditInts)
     float* d_entities = nullptr;       // kMaxEntities boxes of 6 floats
     int n_entities = 0;
     bool dist_dirty = true;            // distances rebuilt before the next render
@@ -237,8 +246,9 @@ vt_status rebuild_distances(vt_world* w, cudaStream_t st);
 // neighbourhood of the bricks edited since the last update.
 vt_status update_distances(vt_world* w, cudaStream_t st);
 // update_distances, then the neighbourhood of the voxel {x, y, z, valid}
-// that a kernel earlier on `st` wrote to d_cell (nothing when !valid).
-vt_status update_distances_at(vt_world* w, const int* d_cell, cudaStream_t st);
+// that a kernel earlier on `st` wrote to d_cell (nothing when !valid), having
+// run the x pass on its brick's rows and cleared the column marks.
+vt_status update_distances_at(vt_world* w, int* d_cell, cudaStream_t st);
 // The world's staging buffer, grown to at least `bytes` (synchronises the
 // device when it has to grow).
 vt_status world_stage(vt_world* w, size_t bytes, unsigned char** out);

@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "dist.cuh"
 #include "vt_internal.h"
 
 namespace vt {
@@ -101,19 +102,12 @@ __global__ void __launch_bounds__(512) k_set_voxel(WorldView w, unsigned long lo
 // the direction of axis i (1: +) for axes 0..axis; the pass reads input field
 // v & ((1 << axis) - 1) (pass 0 reads the coarse bits instead).  Fields are
 // `stride` bytes apart.  The pass covers the whole chunk grid.
-// The window's reads are independent and all in flight at once.  d_changed
-// (null: always run): the pass is skipped when it points to 0, a device-side
-// edit that left every coarse bit as it was.
-__global__ void k_dist_pass(const unsigned long long* __restrict__ coarse, const unsigned char* __restrict__ in,
-                            unsigned char* __restrict__ out, int axis, int CX, int CY, int CZ, size_t stride,
-                            const int* __restrict__ d_changed) {
-    if (d_changed && !*d_changed) return;
-    const unsigned v = blockIdx.y;
+// The window's reads are independent and all in flight at once.
+__device__ __forceinline__ void dist_cell(const unsigned long long* coarse, const unsigned char* in, unsigned char* out,
+                                          int axis, int CX, int CY, int CZ, size_t stride, unsigned v, unsigned lin) {
     const bool fwd = ((v >> axis) & 1u) != 0u;
     if (axis > 0) in += (size_t)(v & ((1u << axis) - 1u)) * stride;
     out += (size_t)v * stride;
-    const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lin >= (unsigned)CX * (unsigned)CY * (unsigned)CZ) return;
     const unsigned p[3] = {lin % (unsigned)CX, (lin / (unsigned)CX) % (unsigned)CY, lin / ((unsigned)CX * (unsigned)CY)};
     const int u = (int)(axis == 0 ? p[0] : (axis == 1 ? p[1] : p[2])), g = axis == 0 ? CX : (axis == 1 ? CY : CZ);
     const int step = (axis == 0 ? 1 : (axis == 1 ? CX : CX * CY)) * (fwd ? 1 : -1);
@@ -124,13 +118,37 @@ __global__ void k_dist_pass(const unsigned long long* __restrict__ coarse, const
         val[d] = kDistCap + 1;
         if (q >= 0 && q < g) {
             const unsigned idx = (unsigned)((int)lin + d * step);
-            val[d] = axis == 0 ? (((__ldg(coarse + (idx >> 6)) >> (idx & 63u)) & 1ull) ? 0 : kDistCap + 1) : (int)__ldg(in + idx);
+            val[d] = axis == 0 ? (((coarse[idx >> 6] >> (idx & 63u)) & 1ull) ? 0 : kDistCap + 1) : (int)in[idx];
         }
     }
     int best = kDistCap + 1;
 #pragma unroll
     for (int d = 0; d <= kDistCap; ++d) best = min(best, max(d, val[d]));
     out[lin] = (unsigned char)best;
+}
+
+// d_changed (null: always run): the pass is skipped when it points to 0, a
+// device-side edit that left every coarse bit as it was.
+__global__ void k_dist_pass(const unsigned long long* coarse, const unsigned char* in, unsigned char* out, int axis,
+                            int CX, int CY, int CZ, size_t stride, const int* d_changed) {
+    if (d_changed && !*d_changed) return;
+    const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
+    if (lin < (unsigned)CX * (unsigned)CY * (unsigned)CZ) dist_cell(coarse, in, out, axis, CX, CY, CZ, stride, blockIdx.y, lin);
+}
+
+// The three passes after a device-side edit of a small grid as one block, one
+// launch instead of three that mostly find nothing to do.
+__global__ void __launch_bounds__(1024) k_dist_edit(const unsigned long long* coarse, unsigned char* fx, unsigned char* fy,
+                                                    unsigned char* out, int CX, int CY, int CZ, size_t stride,
+                                                    const int* d_changed) {
+    if (!*d_changed) return;
+    const unsigned n = (unsigned)CX * (unsigned)CY * (unsigned)CZ;
+    for (int axis = 0; axis < 3; ++axis) {
+        const unsigned char* in = axis == 1 ? fx : fy;
+        unsigned char* to = axis == 0 ? fx : (axis == 1 ? fy : out);
+        for (unsigned i = threadIdx.x; i < (n << (axis + 1)); i += 1024u) dist_cell(coarse, in, to, axis, CX, CY, CZ, stride, i / n, i % n);
+        __syncthreads();
+    }
 }
 
 // Brick level, in voxels.  With vertical weight w = 2^shape, brick b has
@@ -164,94 +182,23 @@ __global__ void k_dist_pass(const unsigned long long* __restrict__ coarse, const
 // words, and the y and z passes scan four bricks at a time (one 32-bit load,
 // 16-bit pair minima and maxima), the four shapes of a downward field in one
 // scan: x 42, y 108, z 126 us.
-__device__ __forceinline__ unsigned brick_index(int bx, int by, int bz, int CX, int CY) {
-    const unsigned ci = (unsigned)(bx >> 3) + (unsigned)CX * ((unsigned)(by >> 3) + (unsigned)CY * (unsigned)(bz >> 3));
-    return ci * 512u + (unsigned)((bx & 7) | ((by & 7) << 3) | ((bz & 7) << 6));
-}
-
-struct BrickGrid {
-    int CX, CY, CZ;   // chunks
-    int GX, GY, GZ;   // bricks
-};
-
 // The y pass's fields: x direction xs, y direction ys (1: +y) and, for -y,
 // the box shape.
 constexpr int kYFields = 2 + 2 * kBoxShapes;
 __host__ __device__ constexpr int y_field(int xs, int ys, int shape) { return ys ? xs : 2 + xs + 2 * shape; }
 
-__device__ __forceinline__ int3 edit_origin(int3 lo, const int* d_cell, bool vx, bool vy, bool vz) {
-    const int bx = d_cell[0] >> 2, by = d_cell[1] >> 2, bz = d_cell[2] >> 2;
-    lo.x += vx ? 4 * bx : bx;
-    lo.y += vy ? 4 * by : by;
-    lo.z += vz ? 4 * bz : bz;
-    return lo;
+// lo relative to the brick of the edited voxel, or in z (voxel layers) to its
+// first voxel.
+__device__ __forceinline__ int3 edit_origin(int3 lo, const int* d_cell, bool z_voxels) {
+    const int bz = d_cell[2] >> 2;
+    return make_int3(lo.x + (d_cell[0] >> 2), lo.y + (d_cell[1] >> 2), lo.z + (z_voxels ? 4 * bz : bz));
 }
 
-// Item `lin` of the box [lo, lo + ext) whose x axis counts groups of `group`
-// bricks (the ones that meet the box): its coordinates, x in groups.  False
-// past the box or the grid.
-__device__ __forceinline__ bool box_item(unsigned lin, int3 lo, int3 ext, int group, int3 g, int& x, int& y, int& z) {
-    const int x0 = max(lo.x, 0) / group, nx = (lo.x + ext.x - 1) / group - x0 + 1;
-    if (lo.x + ext.x <= 0 || nx <= 0) return false;
-    x = x0 + (int)(lin % (unsigned)nx);
-    const unsigned r = lin / (unsigned)nx;
-    y = lo.y + (int)(r % (unsigned)ext.y);
-    const unsigned rz = r / (unsigned)ext.y;
-    if (rz >= (unsigned)ext.z) return false;
-    z = lo.z + (int)rz;
-    return y >= 0 && z >= 0 && x * group < g.x && y < g.y && z < g.z;
-}
-
-// One thread: the 8 bricks of a chunk on the 4 voxel rows of brick row by in
-// layer qz, both directions.  A row of a chunk is one 32-bit word; the first
-// voxel ahead lies in it or in the next two (64 layers, the cap is 63).
 __global__ void k_bdist_x(const unsigned long long* __restrict__ mask, unsigned char* __restrict__ xf, BrickGrid b,
-                          int3 lo, int3 ext, const int* __restrict__ d_cell) {
-    if (d_cell) {
-        if (!d_cell[3]) return;
-        lo = edit_origin(lo, d_cell, false, false, true);
-    }
+                          int3 lo, int3 ext) {
     int cx, by, qz;
-    if (!box_item(blockIdx.x * blockDim.x + threadIdx.x, lo, ext, 8, make_int3(b.GX, b.GY, b.GZ * 4), cx, by, qz)) return;
-    // r[k][y]: row y of chunk cx - 2 + k
-    unsigned r[5][4];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-#pragma unroll
-        for (int y = 0; y < 4; ++y) r[k][y] = 0u;
-        const int c = cx - 2 + k;
-        if (c < 0 || c >= b.CX) continue;
-        const unsigned short* w = reinterpret_cast<const unsigned short*>(mask + brick_index(8 * c, by, qz >> 2, b.CX, b.CY)) + (qz & 3);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const unsigned v = __ldg(w + 4 * i);   // 16 voxels of brick i: 4 rows of 4
-#pragma unroll
-            for (int y = 0; y < 4; ++y) r[k][y] |= ((v >> (4 * y)) & 15u) << (4 * i);
-        }
-    }
-    const size_t fsize = (size_t)b.GX * (b.GY * 4) * (b.GZ * 4);
-#pragma unroll
-    for (int y = 0; y < 4; ++y) {
-        unsigned char* row = xf + (size_t)(8 * cx) + (size_t)b.GX * ((size_t)(4 * by + y) + (size_t)(b.GY * 4) * qz);
-        unsigned out[2][2] = {{0u, 0u}, {0u, 0u}};
-        const unsigned own = r[2][y];
-        // layers from the chunk's far face to the first voxel of the next two
-        const unsigned ahead = r[3][y] ? (unsigned)__ffs(r[3][y]) : (r[4][y] ? 32u + (unsigned)__ffs(r[4][y]) : 64u);
-        const unsigned behind = r[1][y] ? 1u + (unsigned)__clz(r[1][y]) : (r[0][y] ? 33u + (unsigned)__clz(r[0][y]) : 64u);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const bool occ = ((own >> (4 * i)) & 15u) != 0u;
-            const unsigned up = i < 7 ? own >> (4 * i + 4) : 0u, down = own & ((1u << (4 * i)) - 1u);
-            unsigned f = up ? (unsigned)__ffs(up) : (unsigned)(28 - 4 * i) + ahead;
-            unsigned n = down ? (unsigned)(4 * i - 31) + (unsigned)__clz(down) : (unsigned)(4 * i) + behind;
-            f = occ ? 0u : min(f, (unsigned)(kVoxCap + 1));
-            n = occ ? 0u : min(n, (unsigned)(kVoxCap + 1));
-            out[0][i >> 2] |= n << (8 * (i & 3));
-            out[1][i >> 2] |= f << (8 * (i & 3));
-        }
-        *reinterpret_cast<uint2*>(row) = make_uint2(out[0][0], out[0][1]);
-        *reinterpret_cast<uint2*>(row + fsize) = make_uint2(out[1][0], out[1][1]);
-    }
+    if (box_item(blockIdx.x * blockDim.x + threadIdx.x, lo, ext, 8, make_int3(b.GX, b.GY, b.GZ * 4), cx, by, qz))
+        bdist_x_item<false>(mask, xf, b, cx, by, qz);
 }
 
 // Four bytes (at most 63) as two pairs of 16-bit values with the byte on top:
@@ -354,12 +301,14 @@ __device__ __forceinline__ void scan_layers(const unsigned char* const* f, ptrdi
 }
 
 // One thread: four bricks in x, one field (up) or the four shapes (down).
-// blockIdx.y: x direction, y direction << 1.
+// blockIdx.y: x direction, y direction << 1.  EDIT: a column group whose values
+// change is noted for the z pass.
+template <bool EDIT>
 __global__ void k_bdist_y(const unsigned char* __restrict__ xf, unsigned char* __restrict__ yf, BrickGrid b, int3 lo,
-                          int3 ext, const int* __restrict__ d_cell) {
-    if (d_cell) {
+                          int3 ext, int* __restrict__ d_cell) {
+    if (EDIT) {
         if (!d_cell[3]) return;
-        lo = edit_origin(lo, d_cell, false, false, true);
+        lo = edit_origin(lo, d_cell, true);
     }
     const int xs = (int)(blockIdx.y & 1u);
     const bool fwd = (blockIdx.y & 2u) != 0u;
@@ -371,25 +320,34 @@ __global__ void k_bdist_y(const unsigned char* __restrict__ xf, unsigned char* _
                                 (size_t)b.GX * ((size_t)(fwd ? 4 * by : 4 * by + 3) + (size_t)Y * qz);
     const size_t field = (size_t)g.x * g.y * g.z, cell = (size_t)(4 * x4) + (size_t)g.x * ((size_t)by + (size_t)g.y * qz);
     const unsigned char* const in[1] = {near};
+    bool changed = false;
+    auto store = [&](int f, Quad q) {
+        unsigned* at = reinterpret_cast<unsigned*>(yf + (size_t)f * field + cell);
+        const unsigned v = quad_bytes(q);
+        if (EDIT) changed = changed || *at != v;
+        *at = v;
+    };
     if (fwd) {
         Quad q[1];
-        scan_layers<1, 1, false>(in, b.GX, Y - 4 * by, q);
-        *reinterpret_cast<unsigned*>(yf + (size_t)y_field(xs, 1, 0) * field + cell) = quad_bytes(q[0]);
+        scan_layers<1, 1, EDIT>(in, b.GX, Y - 4 * by, q);
+        store(y_field(xs, 1, 0), q[0]);
     } else {
         Quad q[kBoxShapes];
-        scan_layers<1, kBoxShapes, false>(in, -(ptrdiff_t)b.GX, 4 * by + 4, q);
+        scan_layers<1, kBoxShapes, EDIT>(in, -(ptrdiff_t)b.GX, 4 * by + 4, q);
 #pragma unroll
-        for (int shape = 0; shape < kBoxShapes; ++shape)
-            *reinterpret_cast<unsigned*>(yf + (size_t)y_field(xs, 0, shape) * field + cell) = quad_bytes(q[shape]);
+        for (int shape = 0; shape < kBoxShapes; ++shape) store(y_field(xs, 0, shape), q[shape]);
     }
+    if (EDIT && changed) d_cell[kEditColumns + (x4 - max(lo.x, 0) / 4) + kEditGroups * (by - lo.y)] = 1;
 }
 
 // One thread: four bricks in x, one octant (blockIdx.y).
+// EDIT: only the column groups the y pass changed.
+template <bool EDIT>
 __global__ void k_bdist_z(const unsigned char* __restrict__ yf, unsigned char* __restrict__ out, BrickGrid b, int3 lo,
                           int3 ext, const int* __restrict__ d_cell, size_t stride) {
-    if (d_cell) {
+    if (EDIT) {
         if (!d_cell[3]) return;
-        lo = edit_origin(lo, d_cell, false, false, false);
+        lo = edit_origin(lo, d_cell, false);
     }
     const unsigned v = blockIdx.y;
     const bool fwd = (v & 4u) != 0u, up = (v & 2u) != 0u;
@@ -397,6 +355,7 @@ __global__ void k_bdist_z(const unsigned char* __restrict__ yf, unsigned char* _
     const int Z = b.GZ * 4;
     int x4, by, bz;
     if (!box_item(blockIdx.x * blockDim.x + threadIdx.x, lo, ext, 4, make_int3(b.GX, b.GY, b.GZ), x4, by, bz)) return;
+    if (EDIT && !d_cell[kEditColumns + (x4 - max(lo.x, 0) / 4) + kEditGroups * (by - lo.y)]) return;
     const size_t layer = (size_t)b.GX * b.GY, yfield = layer * Z;
     const unsigned char* near = yf + (size_t)(4 * x4) + (size_t)b.GX * by + layer * (size_t)(fwd ? 4 * bz : 4 * bz + 3);
     const ptrdiff_t step = fwd ? (ptrdiff_t)layer : -(ptrdiff_t)layer;
@@ -449,28 +408,51 @@ void chunk_passes(vt_world* w, cudaStream_t st, const int* d_changed) {
     const size_t stride = cdist_stride((unsigned)w->nchunks);
     unsigned char* fx = w->d_ctmp;
     unsigned char* fy = w->d_ctmp + 2 * stride;
+    // (2048 chunks in one block: 15 us when a coarse bit changed against 9, 2.7
+    // against 8 when none did)
+    if (d_changed && w->nchunks <= 4096) {
+        k_dist_edit<<<1, 1024, 0, st>>>(w->d_coarse, fx, fy, w->d_cdist, CX, CY, CZ, stride, d_changed);
+        return;
+    }
     const unsigned nb = dist_blocks(w->nchunks);
     k_dist_pass<<<dim3(nb, 2), kDistThreads, 0, st>>>(w->d_coarse, nullptr, fx, 0, CX, CY, CZ, stride, d_changed);
     k_dist_pass<<<dim3(nb, 4), kDistThreads, 0, st>>>(w->d_coarse, fx, fy, 1, CX, CY, CZ, stride, d_changed);
     k_dist_pass<<<dim3(nb, 8), kDistThreads, 0, st>>>(w->d_coarse, fy, w->d_cdist, 2, CX, CY, CZ, stride, d_changed);
 }
 
-// The brick level, each pass over its own box (x: bricks x voxels x voxels,
-// y: bricks x bricks x voxels, z: bricks).  The intermediates stay valid
-// between calls, which is what lets an edit recompute only the boxes it can
-// change.
-void brick_passes(vt_world* w, cudaStream_t st, const int3 lo[3], const int3 ext[3], const int* d_cell) {
-    const BrickGrid b = {w->cdim[0], w->cdim[1], w->cdim[2], w->cdim[0] * 8, w->cdim[1] * 8, w->cdim[2] * 8};
+BrickGrid brick_grid(const vt_world* w) {
+    return {w->cdim[0], w->cdim[1], w->cdim[2], w->cdim[0] * 8, w->cdim[1] * 8, w->cdim[2] * 8};
+}
+
+// Items of a pass over ext in groups of bricks in x (an aligned group more than
+// the box's bricks need).
+size_t box_items(int3 ext, int group) { return (size_t)((ext.x + group - 1) / group + 1) * ext.y * ext.z; }
+
+// The brick level, each pass over its own box (x: bricks x brick rows x voxel
+// layers, y: bricks x bricks x voxel layers, z: bricks).  The intermediates
+// stay valid between calls, which is what lets an edit recompute only the
+// boxes it can change.
+void brick_passes(vt_world* w, cudaStream_t st, const int3 lo[3], const int3 ext[3]) {
+    const BrickGrid b = brick_grid(w);
     const size_t nb = w->nchunks * kBricksPerChunk;
     unsigned char* xf = w->d_dtmp;             // 2 fields of 16 bytes per brick
     unsigned char* yf = w->d_dtmp + 32 * nb;   // kYFields fields of 4 bytes per brick
-    // (an aligned group more than the box's bricks need, on either side)
-    const size_t nx = (size_t)((ext[0].x + 7) / 8 + 1) * ext[0].y * ext[0].z,
-                 ny = (size_t)((ext[1].x + 3) / 4 + 1) * ext[1].y * ext[1].z,
-                 nz = (size_t)((ext[2].x + 3) / 4 + 1) * ext[2].y * ext[2].z;
-    k_bdist_x<<<dist_blocks(nx), kDistThreads, 0, st>>>(w->d_mask, xf, b, lo[0], ext[0], d_cell);
-    k_bdist_y<<<dim3(dist_blocks(ny), 4), kDistThreads, 0, st>>>(xf, yf, b, lo[1], ext[1], d_cell);
-    k_bdist_z<<<dim3(dist_blocks(nz), 8), kDistThreads, 0, st>>>(yf, w->d_bdist, b, lo[2], ext[2], d_cell, nb);
+    k_bdist_x<<<dist_blocks(box_items(ext[0], 8)), kDistThreads, 0, st>>>(w->d_mask, xf, b, lo[0], ext[0]);
+    k_bdist_y<false><<<dim3(dist_blocks(box_items(ext[1], 4)), 4), kDistThreads, 0, st>>>(xf, yf, b, lo[1], ext[1], nullptr);
+    k_bdist_z<false><<<dim3(dist_blocks(box_items(ext[2], 4)), 8), kDistThreads, 0, st>>>(yf, w->d_bdist, b, lo[2], ext[2],
+                                                                                          nullptr, nb);
+}
+
+// The y and z passes around the voxel of a device-side edit (whose kernel ran
+// the x pass): the z pass over the column groups the y pass changed.
+void edit_passes(vt_world* w, cudaStream_t st, const int3 lo[3], const int3 ext[3], int* d_cell) {
+    const BrickGrid b = brick_grid(w);
+    const size_t nb = w->nchunks * kBricksPerChunk;
+    unsigned char* xf = w->d_dtmp;
+    unsigned char* yf = w->d_dtmp + 32 * nb;
+    k_bdist_y<true><<<dim3((unsigned)((box_items(ext[1], 4) + 63) / 64), 4), 64, 0, st>>>(xf, yf, b, lo[1], ext[1], d_cell);
+    k_bdist_z<true><<<dim3((unsigned)((box_items(ext[2], 4) + 63) / 64), 8), 64, 0, st>>>(yf, w->d_bdist, b, lo[2], ext[2],
+                                                                                        d_cell, nb);
 }
 
 // After the bricks of box [blo, blo + bext) changed occupancy only these
@@ -482,7 +464,7 @@ void brick_passes(vt_world* w, cudaStream_t st, const int3 lo[3], const int3 ext
 // axis.  Recomputing those boxes, in pass order, from the current masks
 // leaves every buffer equal to a full rebuild.
 void edit_boxes(int3 blo, int3 bext, int3 lo[3], int3 ext[3]) {
-    const int R = (kVoxCap + 3) / 4;
+    const int R = kEditReach;
     lo[0] = make_int3(blo.x - R, blo.y, 4 * blo.z);
     ext[0] = make_int3(bext.x + 2 * R, bext.y, 4 * bext.z);
     lo[1] = make_int3(blo.x - R, blo.y - R, 4 * blo.z);
@@ -498,7 +480,7 @@ vt_status rebuild_distances(vt_world* w, cudaStream_t st) {
     const int3 o = make_int3(0, 0, 0);
     const int3 lo[3] = {o, o, o};
     const int3 ext[3] = {make_int3(GX, GY, 4 * GZ), make_int3(GX, GY, 4 * GZ), make_int3(GX, GY, GZ)};
-    brick_passes(w, st, lo, ext, nullptr);
+    brick_passes(w, st, lo, ext);
     chunk_passes(w, st, nullptr);
     VT_CUDA(w->ctx, cudaGetLastError());
     w->dist_dirty = false;
@@ -515,20 +497,20 @@ vt_status update_distances(vt_world* w, cudaStream_t st) {
     int3 lo[3], ext[3];
     edit_boxes(blo, bext, lo, ext);
     if (volume(ext[2]) >= w->nchunks * kBricksPerChunk / 2) return rebuild_distances(w, st);
-    brick_passes(w, st, lo, ext, nullptr);
+    brick_passes(w, st, lo, ext);
     chunk_passes(w, st, nullptr);
     VT_CUDA(w->ctx, cudaGetLastError());
     w->dist_box = false;
     return VT_OK;
 }
 
-vt_status update_distances_at(vt_world* w, const int* d_cell, cudaStream_t st) {
+vt_status update_distances_at(vt_world* w, int* d_cell, cudaStream_t st) {
     vt_status s = update_distances(w, st);
     if (s || w->dist_dirty) return s;
     int3 lo[3], ext[3];
     edit_boxes(make_int3(0, 0, 0), make_int3(1, 1, 1), lo, ext);
-    brick_passes(w, st, lo, ext, d_cell);
-    chunk_passes(w, st, d_cell + 4);
+    edit_passes(w, st, lo, ext, d_cell);
+    chunk_passes(w, st, d_cell + kEditCoarse);
     VT_CUDA(w->ctx, cudaGetLastError());
     return VT_OK;
 }
@@ -623,9 +605,9 @@ vt_status vt_world_create(vt_ctx* ctx, const vt_world_desc* desc, vt_world** out
         (e = vt::dev_alloc(&w->d_cdist, kOctants * (size_t)cdist_stride((unsigned)w->nchunks))) != cudaSuccess ||
         (e = vt::dev_alloc(&w->d_dtmp, (32 + 4 * kYFields) * w->nchunks * kBricksPerChunk)) != cudaSuccess ||
         (e = vt::dev_alloc(&w->d_ctmp, 6 * (size_t)cdist_stride((unsigned)w->nchunks))) != cudaSuccess ||
-        (e = vt::dev_alloc(&w->d_edit, 5 * sizeof(int))) != cudaSuccess ||
+        (e = vt::dev_alloc(&w->d_edit, kEditInts * sizeof(int))) != cudaSuccess ||
         (e = vt::dev_alloc(&w->d_entities, kMaxEntities * 6 * sizeof(float))) != cudaSuccess ||
-        (e = cudaMemset(w->d_edit, 0, 5 * sizeof(int))) != cudaSuccess ||
+        (e = cudaMemset(w->d_edit, 0, kEditInts * sizeof(int))) != cudaSuccess ||
         (e = cudaMemset(w->d_mask, 0, w->nchunks * kBricksPerChunk * 8)) != cudaSuccess ||
         (e = cudaMemset(w->d_mats, 0, w->nchunks * (size_t)kChunkBytes)) != cudaSuccess ||
         (e = cudaMemset(w->d_coarse, 0, w->ncoarse * 8)) != cudaSuccess) {
