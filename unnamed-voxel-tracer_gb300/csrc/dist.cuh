@@ -34,12 +34,13 @@ __device__ __forceinline__ bool box_item(unsigned lin, int3 lo, int3 ext, int gr
 
 // The 8 bricks of a chunk on the 4 voxel rows of brick row by in layer qz,
 // both directions.  A row of a chunk is one 32-bit word; the first voxel ahead
-// lies in it or in the next two (64 layers, the cap is 63).  FRESH: the mask
-// was written earlier in this launch, so it is not read through the
+// lies in it or in the next two (64 layers, the cap is 63).  The words of a
+// chunk whose coarse bit is clear are not read (coarse null: all are).  FRESH:
+// the mask was written earlier in this launch, so it is not read through the
 // non-coherent cache.
 template <bool FRESH>
-__device__ __forceinline__ void bdist_x_item(const unsigned long long* mask, unsigned char* __restrict__ xf,
-                                             const BrickGrid& b, int cx, int by, int qz) {
+__device__ __forceinline__ void bdist_x_item(const unsigned long long* mask, const unsigned long long* coarse,
+                                             unsigned char* __restrict__ xf, const BrickGrid& b, int cx, int by, int qz) {
     // r[k][y]: row y of chunk cx - 2 + k
     unsigned r[5][4];
 #pragma unroll
@@ -48,6 +49,10 @@ __device__ __forceinline__ void bdist_x_item(const unsigned long long* mask, uns
         for (int y = 0; y < 4; ++y) r[k][y] = 0u;
         const int c = cx - 2 + k;
         if (c < 0 || c >= b.CX) continue;
+        if (coarse) {
+            const unsigned ci = (unsigned)c + (unsigned)b.CX * ((unsigned)(by >> 3) + (unsigned)b.CY * (unsigned)(qz >> 5));
+            if (!((__ldg(coarse + (ci >> 6)) >> (ci & 63u)) & 1ull)) continue;
+        }
         const unsigned short* w = reinterpret_cast<const unsigned short*>(mask + brick_index(8 * c, by, qz >> 2, b.CX, b.CY)) + (qz & 3);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {

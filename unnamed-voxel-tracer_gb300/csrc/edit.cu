@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(512) k_pick_edit(WorldView w, unsigned long lo
     int cx, by, qz;
     if (box_item(threadIdx.x, make_int3(bx, y >> 2, z & ~3), make_int3(n, 1, 4), 8, make_int3(grid.GX, grid.GY, 4 * grid.GZ),
                  cx, by, qz))
-        bdist_x_item<true>(mask, xf, grid, cx, by, qz);
+        bdist_x_item<true>(mask, nullptr, xf, grid, cx, by, qz);
 }
 
 PickRay pick_ray(const vt_camera* cam) {

@@ -181,7 +181,8 @@ __global__ void __launch_bounds__(1024) k_dist_edit(const unsigned long long* co
 // z 804 us).  The x pass now finds first voxels with bit scans of 32-voxel row
 // words, and the y and z passes scan four bricks at a time (one 32-bit load,
 // 16-bit pair minima and maxima), the four shapes of a downward field in one
-// scan: x 42, y 108, z 126 us.
+// scan; bricks of chunks with open space ahead are not scanned: x 29, y 61, z 70 us
+// (42, 108, 126 with every brick scanned).
 // The y pass's fields: x direction xs, y direction ys (1: +y) and, for -y,
 // the box shape.
 constexpr int kYFields = 2 + 2 * kBoxShapes;
@@ -194,11 +195,11 @@ __device__ __forceinline__ int3 edit_origin(int3 lo, const int* d_cell, bool z_v
     return make_int3(lo.x + (d_cell[0] >> 2), lo.y + (d_cell[1] >> 2), lo.z + (z_voxels ? 4 * bz : bz));
 }
 
-__global__ void k_bdist_x(const unsigned long long* __restrict__ mask, unsigned char* __restrict__ xf, BrickGrid b,
-                          int3 lo, int3 ext) {
+__global__ void k_bdist_x(const unsigned long long* __restrict__ mask, const unsigned long long* __restrict__ coarse,
+                          unsigned char* __restrict__ xf, BrickGrid b, int3 lo, int3 ext) {
     int cx, by, qz;
     if (box_item(blockIdx.x * blockDim.x + threadIdx.x, lo, ext, 8, make_int3(b.GX, b.GY, b.GZ * 4), cx, by, qz))
-        bdist_x_item<false>(mask, xf, b, cx, by, qz);
+        bdist_x_item<false>(mask, coarse, xf, b, cx, by, qz);
 }
 
 // Four bytes (at most 63) as two pairs of 16-bit values with the byte on top:
@@ -300,12 +301,26 @@ __device__ __forceinline__ void scan_layers(const unsigned char* const* f, ptrdi
     }
 }
 
+// The chunk distances of the grid (up to date before the brick passes).  From
+// a chunk whose distance in an octant is 3 or more the two chunks ahead of it
+// on every axis are empty, 64 layers: every brick of it is at the cap, and its
+// scans are not run (the sky above a terrain).
+struct ChunkDist {
+    const unsigned char* d;
+    unsigned stride;
+    __device__ __forceinline__ bool far(const BrickGrid& b, unsigned oct, int bx, int by, int bz) const {
+        const unsigned ci = (unsigned)(bx >> 3) + (unsigned)b.CX * ((unsigned)(by >> 3) + (unsigned)b.CY * (unsigned)(bz >> 3));
+        return __ldg(d + oct * stride + ci) >= 3u;
+    }
+};
+constexpr unsigned kAllFar = (unsigned)(kVoxCap + 1) * 0x01010101u;
+
 // One thread: four bricks in x, one field (up) or the four shapes (down).
 // blockIdx.y: x direction, y direction << 1.  EDIT: a column group whose values
 // change is noted for the z pass.
 template <bool EDIT>
 __global__ void k_bdist_y(const unsigned char* __restrict__ xf, unsigned char* __restrict__ yf, BrickGrid b, int3 lo,
-                          int3 ext, int* __restrict__ d_cell) {
+                          int3 ext, int* __restrict__ d_cell, ChunkDist cd) {
     if (EDIT) {
         if (!d_cell[3]) return;
         lo = edit_origin(lo, d_cell, true);
@@ -321,21 +336,23 @@ __global__ void k_bdist_y(const unsigned char* __restrict__ xf, unsigned char* _
     const size_t field = (size_t)g.x * g.y * g.z, cell = (size_t)(4 * x4) + (size_t)g.x * ((size_t)by + (size_t)g.y * qz);
     const unsigned char* const in[1] = {near};
     bool changed = false;
-    auto store = [&](int f, Quad q) {
+    auto store = [&](int f, unsigned v) {
         unsigned* at = reinterpret_cast<unsigned*>(yf + (size_t)f * field + cell);
-        const unsigned v = quad_bytes(q);
         if (EDIT) changed = changed || *at != v;
         *at = v;
     };
+    // the scan stays in one layer of z, ahead in both z octants
+    const unsigned oct = (unsigned)xs | (fwd ? 2u : 0u);
+    const bool far = cd.far(b, oct, 4 * x4, by, qz >> 2) || cd.far(b, oct | 4u, 4 * x4, by, qz >> 2);
     if (fwd) {
         Quad q[1];
-        scan_layers<1, 1, EDIT>(in, b.GX, Y - 4 * by, q);
-        store(y_field(xs, 1, 0), q[0]);
+        if (!far) scan_layers<1, 1, EDIT>(in, b.GX, Y - 4 * by, q);
+        store(y_field(xs, 1, 0), far ? kAllFar : quad_bytes(q[0]));
     } else {
         Quad q[kBoxShapes];
-        scan_layers<1, kBoxShapes, EDIT>(in, -(ptrdiff_t)b.GX, 4 * by + 4, q);
+        if (!far) scan_layers<1, kBoxShapes, EDIT>(in, -(ptrdiff_t)b.GX, 4 * by + 4, q);
 #pragma unroll
-        for (int shape = 0; shape < kBoxShapes; ++shape) store(y_field(xs, 0, shape), q[shape]);
+        for (int shape = 0; shape < kBoxShapes; ++shape) store(y_field(xs, 0, shape), far ? kAllFar : quad_bytes(q[shape]));
     }
     if (EDIT && changed) d_cell[kEditColumns + (x4 - max(lo.x, 0) / 4) + kEditGroups * (by - lo.y)] = 1;
 }
@@ -344,7 +361,7 @@ __global__ void k_bdist_y(const unsigned char* __restrict__ xf, unsigned char* _
 // EDIT: only the column groups the y pass changed.
 template <bool EDIT>
 __global__ void k_bdist_z(const unsigned char* __restrict__ yf, unsigned char* __restrict__ out, BrickGrid b, int3 lo,
-                          int3 ext, const int* __restrict__ d_cell, size_t stride) {
+                          int3 ext, const int* __restrict__ d_cell, size_t stride, ChunkDist cd) {
     if (EDIT) {
         if (!d_cell[3]) return;
         lo = edit_origin(lo, d_cell, false);
@@ -361,7 +378,9 @@ __global__ void k_bdist_z(const unsigned char* __restrict__ yf, unsigned char* _
     const ptrdiff_t step = fwd ? (ptrdiff_t)layer : -(ptrdiff_t)layer;
     const int count = fwd ? Z - 4 * bz : 4 * bz + 4;
     unsigned res = 0u;
-    if (up) {
+    if (cd.far(b, v, 4 * x4, by, bz)) {
+        res = kAllFar;   // (shape 0 has the largest box)
+    } else if (up) {
         const unsigned char* const in[1] = {near + (size_t)y_field(xs, 1, 0) * yfield};
         Quad q[1];
         scan_layers<1, 1, true>(in, step, count, q);
@@ -435,12 +454,14 @@ size_t box_items(int3 ext, int group) { return (size_t)((ext.x + group - 1) / gr
 void brick_passes(vt_world* w, cudaStream_t st, const int3 lo[3], const int3 ext[3]) {
     const BrickGrid b = brick_grid(w);
     const size_t nb = w->nchunks * kBricksPerChunk;
+    const ChunkDist cd = {w->d_cdist, cdist_stride((unsigned)w->nchunks)};
     unsigned char* xf = w->d_dtmp;             // 2 fields of 16 bytes per brick
     unsigned char* yf = w->d_dtmp + 32 * nb;   // kYFields fields of 4 bytes per brick
-    k_bdist_x<<<dist_blocks(box_items(ext[0], 8)), kDistThreads, 0, st>>>(w->d_mask, xf, b, lo[0], ext[0]);
-    k_bdist_y<false><<<dim3(dist_blocks(box_items(ext[1], 4)), 4), kDistThreads, 0, st>>>(xf, yf, b, lo[1], ext[1], nullptr);
+    k_bdist_x<<<dist_blocks(box_items(ext[0], 8)), kDistThreads, 0, st>>>(w->d_mask, w->d_coarse, xf, b, lo[0], ext[0]);
+    k_bdist_y<false><<<dim3(dist_blocks(box_items(ext[1], 4)), 4), kDistThreads, 0, st>>>(xf, yf, b, lo[1], ext[1], nullptr,
+                                                                                            cd);
     k_bdist_z<false><<<dim3(dist_blocks(box_items(ext[2], 4)), 8), kDistThreads, 0, st>>>(yf, w->d_bdist, b, lo[2], ext[2],
-                                                                                          nullptr, nb);
+                                                                                          nullptr, nb, cd);
 }
 
 // The y and z passes around the voxel of a device-side edit (whose kernel ran
@@ -448,11 +469,12 @@ void brick_passes(vt_world* w, cudaStream_t st, const int3 lo[3], const int3 ext
 void edit_passes(vt_world* w, cudaStream_t st, const int3 lo[3], const int3 ext[3], int* d_cell) {
     const BrickGrid b = brick_grid(w);
     const size_t nb = w->nchunks * kBricksPerChunk;
+    const ChunkDist cd = {w->d_cdist, cdist_stride((unsigned)w->nchunks)};
     unsigned char* xf = w->d_dtmp;
     unsigned char* yf = w->d_dtmp + 32 * nb;
-    k_bdist_y<true><<<dim3((unsigned)((box_items(ext[1], 4) + 63) / 64), 4), 64, 0, st>>>(xf, yf, b, lo[1], ext[1], d_cell);
+    k_bdist_y<true><<<dim3((unsigned)((box_items(ext[1], 4) + 63) / 64), 4), 64, 0, st>>>(xf, yf, b, lo[1], ext[1], d_cell, cd);
     k_bdist_z<true><<<dim3((unsigned)((box_items(ext[2], 4) + 63) / 64), 8), 64, 0, st>>>(yf, w->d_bdist, b, lo[2], ext[2],
-                                                                                        d_cell, nb);
+                                                                                        d_cell, nb, cd);
 }
 
 // After the bricks of box [blo, blo + bext) changed occupancy only these
@@ -480,8 +502,8 @@ vt_status rebuild_distances(vt_world* w, cudaStream_t st) {
     const int3 o = make_int3(0, 0, 0);
     const int3 lo[3] = {o, o, o};
     const int3 ext[3] = {make_int3(GX, GY, 4 * GZ), make_int3(GX, GY, 4 * GZ), make_int3(GX, GY, GZ)};
+    chunk_passes(w, st, nullptr);   // before the brick passes, which read them
     brick_passes(w, st, lo, ext);
-    chunk_passes(w, st, nullptr);
     VT_CUDA(w->ctx, cudaGetLastError());
     w->dist_dirty = false;
     w->dist_box = false;
@@ -497,8 +519,8 @@ vt_status update_distances(vt_world* w, cudaStream_t st) {
     int3 lo[3], ext[3];
     edit_boxes(blo, bext, lo, ext);
     if (volume(ext[2]) >= w->nchunks * kBricksPerChunk / 2) return rebuild_distances(w, st);
+    chunk_passes(w, st, nullptr);   // before the brick passes, which read them
     brick_passes(w, st, lo, ext);
-    chunk_passes(w, st, nullptr);
     VT_CUDA(w->ctx, cudaGetLastError());
     w->dist_box = false;
     return VT_OK;
@@ -509,8 +531,8 @@ vt_status update_distances_at(vt_world* w, int* d_cell, cudaStream_t st) {
     if (s || w->dist_dirty) return s;
     int3 lo[3], ext[3];
     edit_boxes(make_int3(0, 0, 0), make_int3(1, 1, 1), lo, ext);
-    edit_passes(w, st, lo, ext, d_cell);
     chunk_passes(w, st, d_cell + kEditCoarse);
+    edit_passes(w, st, lo, ext, d_cell);
     VT_CUDA(w->ctx, cudaGetLastError());
     return VT_OK;
 }
