@@ -104,15 +104,16 @@ __global__ void __launch_bounds__(512) k_gen_chunks(WorldView w, unsigned long l
 // its error bound of the number; only then is the 64-bit value computed.
 // The lattice values a chunk needs (a few hundred) are hashed once into shared
 // memory, and the cave noise is interpolated along x once per lattice row.
-// The same world now takes 145 us.
+// The same world now takes 71 us.
 //
 // Error of the 32-bit values against the real ones, u = 2^-24: a lattice value
-// is in [-1, 1) (rounding u / 2), a weight smooth(t) is off by at most 4 u, an
-// interpolation a + (b - a) t adds 2 * 4 u for the weight and at most 2 u for
-// its rounding.  Two levels and a weighted mean of at most 16 octaves stay
-// below 32 u = 1.9e-6, three levels below 31 u, times 1.5 for the two octaves'
-// sum.  (The 64-bit values' own error is below 1e-14.)
-constexpr float kFbmError = 2.5e-6f, kCaveError = 4e-6f;
+// is in [-1, 1) (rounding u / 2); a weight, exact to 2^-28 before its one
+// rounding, is off by at most 0.6 u; an interpolation a + (b - a) t adds 1.2 u
+// for the weight and 1.5 u for its roundings.  Two levels: 6 u; the octaves'
+// sum (below 2) adds at most u an octave before the division by the
+// amplitudes' sum and 2 u in it; three levels: 8.6 u, times 1.5 for the two
+// octaves' sum, and 2 u more.  (The 64-bit values' own error is below 1e-14.)
+constexpr float kUlp = 0x1p-24f, kCaveError = 16.0f * kUlp;
 
 // gen::lattice rounded to 32 bits: the hash as a signed fraction.
 __device__ __forceinline__ float lattice32(uint64_t seed, int x, int y, int z) {
@@ -127,9 +128,10 @@ __device__ __forceinline__ float lattice32(uint64_t seed, int x, int y, int z) {
 // 2^-28, and the noise is continuous across the cells.
 __device__ __forceinline__ void lattice_coord(int g, long long f, int& cell, float& weight) {
     const long long x = (long long)g * f;
-    const float t = __uint2float_rn((unsigned)((unsigned long long)x >> 8)) * 0x1p-32f;
+    const unsigned t = (unsigned)((unsigned long long)x >> 8);   // the position in the cell, times 2^32
     cell = (int)(x >> 40);
-    weight = t * t * (3.0f - 2.0f * t);
+    // t t (3 - 2 t) in integers
+    weight = __uint2float_rn(__umulhi(__umulhi(t, t), 0xC0000000u - (t >> 1))) * 0x1p-30f;
 }
 
 __device__ __forceinline__ float lerp32(float a, float b, float t) { return __fmaf_rn(b - a, t, a); }
@@ -140,6 +142,8 @@ struct GenArgs {
     long long freq40, cave40;    // the frequencies, multiples of 2^-40
     uint64_t terrain_seed, cave_seed, leaf_seed;
     float norm;                  // 1 / (sum of the octaves' amplitudes)
+    float fbm_error;             // of the 32-bit fbm2
+    float ceiling;               // no cell at or above it but trees
     int water;
     // shared-memory layout of k_gen_tiles, in floats
     int height_side[16];         // most lattice points a chunk meets on an axis, per octave
@@ -159,7 +163,7 @@ __device__ __noinline__ bool cave_exact(const GenArgs* a, int x, int y, int z) {
 // clamps), or in 64 bits where that does not decide the floor.
 __device__ __forceinline__ int height_of(const GenArgs& a, float fbm, int x, int z) {
     const float v = __fmaf_rn(a.d.amplitude, fbm, a.d.base_height);
-    const float margin = fabsf(a.d.amplitude) * kFbmError + fabsf(v) * 0x1p-22f;
+    const float margin = fabsf(a.d.amplitude) * a.fbm_error + fabsf(v) * (4.0f * kUlp);
     const float lo = floorf(v - margin);
     if (!(lo == floorf(v + margin)) || !(fabsf(lo) < 1e6f)) return height_exact(&a.d, x, z);
     int h = (int)lo;
@@ -194,11 +198,14 @@ __device__ bool tree_site32(const GenArgs& a, int t, int* x, int* z, int* h) {
     return *h + 8 < a.d.dims[1];
 }
 
-// (two blocks per SM: 145 us on the cave world, one 366, three 154)
+// Bound: issue (63%) and the short phases between barriers.  Cells four in x
+// at a time from 16-byte table rows, a layer stored as it is done (71 us on the
+// 512x256x512 cave world; one cell at a time with the brick in registers 116 us);
+// chunks above every column are cleared at once.
 __global__ void __launch_bounds__(512, 2) k_gen_tiles(WorldView w, unsigned long long* mask, unsigned char* mats,
                                                    unsigned long long* coarse, const __grid_constant__ GenArgs a) {
-    extern __shared__ float s_gen[];
-    __shared__ int heights[32 * 32];
+    extern __shared__ __align__(16) float s_gen[];
+    __shared__ __align__(16) int heights[32 * 32];
     __shared__ float weight[16][2][32];       // [octave][axis][coordinate]; caves: [octave * 3 + axis][0]
     __shared__ unsigned char cell[16][2][32]; // lattice cell relative to the chunk's first
     __shared__ int first[16][2];              // the chunk's first lattice point
@@ -207,6 +214,16 @@ __global__ void __launch_bounds__(512, 2) k_gen_tiles(WorldView w, unsigned long
     const int cy = (int)((ci / (unsigned)w.cdim[0]) % (unsigned)w.cdim[1]);
     const int cz = (int)(ci / ((unsigned)w.cdim[0] * (unsigned)w.cdim[1]));
     const int tid = threadIdx.x;
+
+    // a chunk above the highest column (fbm is in [-1, 1]) and the water is air
+    if (cy > 0 && (float)(cy * 32) >= a.ceiling) {
+        uint4* dst = reinterpret_cast<uint4*>(mats + (size_t)ci * kChunkBytes);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dst[q * 512 + tid] = make_uint4(0u, 0u, 0u, 0u);
+        mask[ci * 512u + (unsigned)tid] = 0ull;
+        if (tid == 0) atomicAnd(coarse + (ci >> 6), ~(1ull << (ci & 63u)));
+        return;
+    }
 
     // ---- heights
     for (int i = tid; i < a.d.octaves * 64; i += 512) {
@@ -229,7 +246,7 @@ __global__ void __launch_bounds__(512, 2) k_gen_tiles(WorldView w, unsigned long
     __syncthreads();
     for (int c = tid; c < 32 * 32; c += 512) {
         const int lx = c & 31, lz = c >> 5, gx = cx * 32 + lx, gz = cz * 32 + lz;
-        int h = 0;
+        int h = -1;   // no column
         if (gx < w.dims[0] && gz < w.dims[2]) {
             float sum = 0.0f, amp = 1.0f;
             for (int o = 0, base = 0; o < a.d.octaves; ++o) {
@@ -248,7 +265,7 @@ __global__ void __launch_bounds__(512, 2) k_gen_tiles(WorldView w, unsigned long
 
     // ---- cave tables: per octave the lattice, then its rows along x (fixed
     // lattice y and z) interpolated at the chunk's 32 coordinates
-    float* rows = s_gen + a.cave_floats;
+    float* rows = s_gen + a.cave_floats;   // (16-byte aligned)
     if (a.d.caves) {
         for (int i = tid; i < 2 * 96; i += 512) {
             const int o = i / 96, axis = (i % 96) >> 5, k = i & 31, g0 = (axis == 0 ? cx : (axis == 1 ? cy : cz)) * 32;
@@ -282,78 +299,63 @@ __global__ void __launch_bounds__(512, 2) k_gen_tiles(WorldView w, unsigned long
         __syncthreads();
     }
 
-    // ---- the thread's brick
+    // ---- the thread's brick, a layer of 16 cells and one 16-byte store at a
+    // time; four cells in x share their loads
     const int bx = tid & 7, by = (tid >> 3) & 7, bz = tid >> 6;
-    const int gy0 = cy * 32 + by * 4;
-    unsigned packed[16];
-#pragma unroll
-    for (int q = 0; q < 16; ++q) packed[q] = 0u;
-    int top = 0;   // cells at or above it are air or water
-#pragma unroll
-    for (int c = 0; c < 16; ++c) top = max(top, heights[bx * 4 + (c & 3) + 32 * (bz * 4 + (c >> 2))]);
-    const float bound = 1.5f * a.d.cave_threshold;   // of noise + noise / 2
-    const float margin = kCaveError + 1e-6f * fabsf(bound);
-    if (gy0 < top || gy0 < a.water) {
-        const int n0 = a.cave_side[0], n1 = a.cave_side[1];
-#pragma unroll 1
-        for (int x = 0; x < 4; ++x) {
-            const int lx = bx * 4 + x, gx = cx * 32 + lx;
-#pragma unroll
-            for (int y = 0; y < 4; ++y) {
-                const int ly = by * 4 + y, gy = gy0 + y;
-                // the two octaves interpolated along x and y on the lattice
-                // planes around the z cell, kept while it lasts
-                float p0 = 0.0f, q0 = 0.0f, p1 = 0.0f, q1 = 0.0f;
-                int z0 = -1, z1 = -1;
-#pragma unroll
-                for (int z = 0; z < 4; ++z) {
-                    const int lz = bz * 4 + z, gz = cz * 32 + lz;
-                    const int h = heights[lx + 32 * lz];
-                    unsigned v = 0u;
-                    if (gx < w.dims[0] && gy < w.dims[1] && gz < w.dims[2]) {
-                        if (gy < h) {
-                            v = gy == h - 1 ? 1u : (gy >= h - 4 ? 2u : 3u);
-                            if (a.d.caves && gy > 0) {
-                                if (cell[2][0][lz] != z0) {
-                                    z0 = cell[2][0][lz];
-                                    const float* r = rows + 32 * (cell[1][0][ly] + n0 * z0) + lx;
-                                    const float s = weight[1][0][ly];
-                                    p0 = lerp32(r[0], r[32], s);
-                                    q0 = lerp32(r[32 * n0], r[32 * n0 + 32], s);
-                                }
-                                if (cell[5][0][lz] != z1) {
-                                    z1 = cell[5][0][lz];
-                                    const float* r = rows + 32 * (n0 * n0 + cell[4][0][ly] + n1 * z1) + lx;
-                                    const float s = weight[4][0][ly];
-                                    p1 = lerp32(r[0], r[32], s);
-                                    q1 = lerp32(r[32 * n1], r[32 * n1 + 32], s);
-                                }
-                                const float f = __fmaf_rn(0.5f, lerp32(p1, q1, weight[5][0][lz]), lerp32(p0, q0, weight[2][0][lz])) - bound;
-                                bool cave = f > 0.0f;
-                                if (fabsf(f) <= margin)
-                                    cave = cave_exact(&a, gx, gy, gz);
-                                if (cave) v = 0u;
-                            }
-                        } else if (gy < a.water) {
-                            v = 4u;
-                        }
-                    }
-                    packed[y + 4 * z] |= v << (8 * x);
-                }
-            }
-        }
-    }
-    unsigned long long m = 0ull;
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-        // bit per nonzero byte
-        const unsigned nz = ((packed[q] & 0x7F7F7F7Fu) + 0x7F7F7F7Fu | packed[q]) & 0x80808080u;
-        m |= (unsigned long long)((nz * 0x00204081u) >> 28) << (4 * q);
-    }
+    const int gy0 = cy * 32 + by * 4, water = min(a.water, w.dims[1]);
     const unsigned wi = ci * 512u + (unsigned)tid;
     uint4* dst = reinterpret_cast<uint4*>(mats + (size_t)wi * 64u);
+    const float bound = 1.5f * a.d.cave_threshold;   // of noise + noise / 2
+    const float margin = kCaveError + 4.0f * kUlp * fabsf(bound);
+    const int n0 = a.cave_side[0], n1 = a.cave_side[1];
+    unsigned long long m = 0ull;
+#pragma unroll 1
+    for (int z = 0; z < 4; ++z) {
+        const int lz = bz * 4 + z;
+        const int4 h4 = *reinterpret_cast<const int4*>(heights + bx * 4 + 32 * lz);
+        const int h[4] = {h4.x, h4.y, h4.z, h4.w};
+        const int top = max(max(h[0], h[1]), max(h[2], h[3]));
+        unsigned word[4] = {0u, 0u, 0u, 0u};
+        if (gy0 < top || gy0 < water) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) dst[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+            for (int y = 0; y < 4; ++y) {
+                const int gy = gy0 + y;
+                unsigned v[4];
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+                    v[x] = gy < h[x] ? (gy == h[x] - 1 ? 1u : (gy >= h[x] - 4 ? 2u : 3u)) : (gy < water && h[x] > 0 ? 4u : 0u);
+                if (a.d.caves && gy > 0 && gy < top) {
+                    const int ly = by * 4 + y;
+                    const float4* r0 = reinterpret_cast<const float4*>(rows + 32 * (cell[1][0][ly] + n0 * cell[2][0][lz])) + bx;
+                    const float4* r1 = reinterpret_cast<const float4*>(rows + 32 * (n0 * n0 + cell[4][0][ly] + n1 * cell[5][0][lz])) + bx;
+                    const float4 a00 = r0[0], a10 = r0[8], a01 = r0[8 * n0], a11 = r0[8 * n0 + 8];
+                    const float4 b00 = r1[0], b10 = r1[8], b01 = r1[8 * n1], b11 = r1[8 * n1 + 8];
+                    const float y0 = weight[1][0][ly], z0 = weight[2][0][lz], y1 = weight[4][0][ly], z1 = weight[5][0][lz];
+                    auto noise = [&](float p00, float p10, float p01, float p11, float q00, float q10, float q01, float q11) {
+                        const float p = lerp32(lerp32(p00, p10, y0), lerp32(p01, p11, y0), z0);
+                        const float q = lerp32(lerp32(q00, q10, y1), lerp32(q01, q11, y1), z1);
+                        return __fmaf_rn(0.5f, q, p) - bound;
+                    };
+                    const float f[4] = {noise(a00.x, a10.x, a01.x, a11.x, b00.x, b10.x, b01.x, b11.x),
+                                        noise(a00.y, a10.y, a01.y, a11.y, b00.y, b10.y, b01.y, b11.y),
+                                        noise(a00.z, a10.z, a01.z, a11.z, b00.z, b10.z, b01.z, b11.z),
+                                        noise(a00.w, a10.w, a01.w, a11.w, b00.w, b10.w, b01.w, b11.w)};
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        if (gy >= h[x]) continue;
+                        bool cave = f[x] > 0.0f;
+                        if (fabsf(f[x]) <= margin) cave = cave_exact(&a, cx * 32 + bx * 4 + x, gy, cz * 32 + lz);
+                        if (cave) v[x] = 0u;
+                    }
+                }
+                word[y] = v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24);
+                // bit per nonzero byte (materials below 128)
+                const unsigned nz = (word[y] + 0x7F7F7F7Fu) & 0x80808080u;
+                m |= (unsigned long long)((nz * 0x00204081u) >> 28) << (4 * y + 16 * z);
+            }
+        }
+        dst[z] = make_uint4(word[0], word[1], word[2], word[3]);
+    }
     mask[wi] = m;
     const int any = __syncthreads_or(m != 0ull);
     if (tid == 0) {
@@ -447,9 +449,12 @@ int gen_args(const vt_gen_desc& d, GenArgs& a) {
     a.cave_seed = gen::stream_seed(d.seed, gen::kCaves);
     a.leaf_seed = gen::stream_seed(d.seed, gen::kLeaves);
     a.water = (int)ceil((double)d.water_level);
+    const double top = std::fmax((double)d.base_height + std::fabs((double)d.amplitude) + 2.0, (double)a.water + 1.0);
+    a.ceiling = top < 1e6 ? (float)top + 1.0f : INFINITY;   // (NaN, too)
     double norm = 0.0, amp = 1.0;
     for (int o = 0; o < d.octaves; ++o, amp *= 0.5) norm += amp;
     a.norm = (float)(1.0 / norm);
+    a.fbm_error = (8.0f + (float)d.octaves) * kUlp;
     // 32 coordinates at frequency f meet at most floor(31 f) + 2 cells, one
     // more lattice points
     auto side = [](long long f40) { return (double)((31 * f40) >> 40) + 3.0; };
@@ -470,10 +475,10 @@ int gen_args(const vt_gen_desc& d, GenArgs& a) {
         caves += n * n * n;
         rows += n * n;
     }
-    const double floats = heights > caves + 32.0 * rows ? heights : caves + 32.0 * rows;
+    const double floats = heights > caves + 3.0 + 32.0 * rows ? heights : caves + 3.0 + 32.0 * rows;
     if (4.0 * floats > (double)kGenSmem) return 0;
     a.height_floats = (int)heights;
-    a.cave_floats = (int)caves;
+    a.cave_floats = ((int)caves + 3) / 4 * 4;
     a.cave_rows = (int)rows;
     return (int)floats * 4;
 }
