@@ -363,7 +363,7 @@ vt_status vt_brickmap_edit(vt_ctx* ctx, vt_brickmap* bm, const vt_camera* cam, i
  * Many scenes x cameras in one graph launch (no counterpart in the reference,
  * which renders one camera per frame, game.zig:232-256).  Under the default
  * tuning (VT_KERNEL_TILE) the graph holds one render launch per world (its
- * consecutive jobs, up to 256), whose grid covers the 16x16-pixel tiles of
+ * consecutive jobs, up to 256), whose grid covers the 16x8-pixel tiles of
  * all those jobs (the job table travels as the launch's parameters); under
  * VT_KERNEL_PER_JOB it holds one render launch per job on eight concurrent
  * chains; under VT_KERNEL_QUEUE one persistent kernel that pulls 16x16-pixel

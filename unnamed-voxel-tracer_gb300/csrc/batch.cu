@@ -5,7 +5,7 @@
 //
 //   tile (default)  the consecutive jobs of each world (up to kLaunchJobs
 //                   jobs and about 4 Mpixels) are ONE launch of k_render_jobs
-//                   whose grid covers every 16 x 16-pixel tile of all of
+//                   whose grid covers every 16 x 8-pixel tile of all of
 //                   them, on kBatchChains concurrent chains of the graph
 //                   (longest launch first, on the least loaded chain).  The launch's job table
 //                   (the world, the shared frame settings, each job's camera,
@@ -42,13 +42,16 @@ struct JobDesc {
 
 constexpr int kBatchBlock = 256;
 constexpr int kUnit = 16;  // pixels per unit side
+// The tile shape's block: 16 x 8 pixels (16 scenes, 40 cameras: 1213 us; 16 x 16
+// pixels 1252).
+constexpr int kTileBlock = 128, kTileH = kTileBlock / kUnit;
 constexpr int kBatchChains = 8;  // 4, 8, 16 and 32 chains measured within 1% on the 64-scene batch
 
 // ---------------------------------------------------------------- tile shape
 constexpr int kLaunchJobs = 256;
-// A launch holds at most this many 16 x 16 blocks (about 4 Mpixels) unless
+// A launch holds at most this many blocks (about 4 Mpixels) unless
 // one camera alone is larger: finer launches balance the graph's chains.
-constexpr unsigned kLaunchBlocks = 16384;
+constexpr unsigned kLaunchBlocks = 16384 * (256 / kTileBlock);
 
 // Per-job camera fields of a tile-shape launch.
 struct JobCam {
@@ -77,11 +80,11 @@ struct JobChunk {
 };
 static_assert(sizeof(JobChunk) <= 32764, "a kernel's parameters are limited to 32764 bytes");
 
-// One thread per pixel; the 256-thread block covers a 16 x 16 tile as eight
+// One thread per pixel; the 128-thread block covers a 16 x 8 tile as four
 // 8 x 4 warp tiles (the single-frame kernel's default shape), with the same
-// register cap (4 blocks per SM).
+// register cap (32 warps per SM).
 template <bool CHECKED, bool BOUNCE, bool LONG>
-__global__ void __launch_bounds__(kBatchBlock, 4) k_render_jobs(const __grid_constant__ JobChunk p, unsigned* status) {
+__global__ void __launch_bounds__(kTileBlock, 1024 / kTileBlock) k_render_jobs(const __grid_constant__ JobChunk p, unsigned* status) {
     const unsigned b = blockIdx.x;
     int lo = 0, hi = p.njobs - 1;
     while (lo < hi) {
@@ -104,16 +107,16 @@ __global__ void __launch_bounds__(kBatchBlock, 4) k_render_jobs(const __grid_con
     f.row_end = jc.height;
     f.screen = jc.screen;
     const unsigned local = b - p.first_block[lo];
-    const int x0 = (int)(local % jc.blocks_x) * kUnit, y0 = (int)(local / jc.blocks_x) * kUnit;
+    const int x0 = (int)(local % jc.blocks_x) * kUnit, y0 = (int)(local / jc.blocks_x) * kTileH;
     // screen coordinates: the frame's table, else once per block
-    __shared__ float s_col[3][kUnit], s_row[3][kUnit];
+    __shared__ float s_col[3][kUnit], s_row[3][kTileH];
     const bool table = f.screen != nullptr;
     if (!table) {
         if (threadIdx.x < kUnit) {
             s_col[0][threadIdx.x] = ray_u(f, x0 + (int)threadIdx.x);
             s_col[1][threadIdx.x] = centre_u(f, x0 + (int)threadIdx.x);
             s_col[2][threadIdx.x] = vignette_u(s_col[1][threadIdx.x]);
-        } else if (threadIdx.x >= 64 && threadIdx.x < 64 + kUnit) {
+        } else if (threadIdx.x >= 64 && threadIdx.x < 64 + kTileH) {
             s_row[0][threadIdx.x - 64] = ray_v(f, y0 + (int)threadIdx.x - 64);
             s_row[1][threadIdx.x - 64] = centre_v(f, y0 + (int)threadIdx.x - 64);
             s_row[2][threadIdx.x - 64] = vignette_v(s_row[1][threadIdx.x - 64]);
@@ -213,7 +216,7 @@ vt_status build_chunks(vt_batch* b) {
         vt_status s = screen_table(ctx, f, ctx->stream, true, &f.screen);
         if (s) return s;
         const unsigned long long job_blocks = (unsigned long long)((j.camera.width + kUnit - 1) / kUnit) *
-                                              (unsigned long long)((j.camera.height + kUnit - 1) / kUnit);
+                                              (unsigned long long)((j.camera.height + kTileH - 1) / kTileH);
         if (!c || c->njobs == kLaunchJobs || c->w.mask != j.world->d_mask ||
             (c->njobs > 0 && (unsigned long long)c->first_block[c->njobs] + job_blocks > kLaunchBlocks)) {
             b->chunks.emplace_back();
@@ -235,7 +238,7 @@ vt_status build_chunks(vt_batch* b) {
         jc.out = reinterpret_cast<uint4*>(j.d_out);
         jc.blocks_x = (unsigned)((j.camera.width + kUnit - 1) / kUnit);
         const unsigned long long nb =
-            (unsigned long long)jc.blocks_x * (unsigned long long)((j.camera.height + kUnit - 1) / kUnit);
+            (unsigned long long)jc.blocks_x * (unsigned long long)((j.camera.height + kTileH - 1) / kTileH);
         const unsigned long long end = (unsigned long long)c->first_block[n] + nb;
         if (end >= (1ull << 31)) return fail(ctx, VT_ERR_ARG, "batch launch too large (blocks >= 2^31)");
         c->first_block[n + 1] = (unsigned)end;
@@ -369,7 +372,7 @@ vt_status vt_batch_launch(vt_batch* b, vt_stream stream) {
                         auto k = checked ? k_render_jobs<true, true, true>
                                  : bounce ? (lng ? k_render_jobs<false, true, true> : k_render_jobs<false, true, false>)
                                           : (lng ? k_render_jobs<false, false, true> : k_render_jobs<false, false, false>);
-                        k<<<blocks, kBatchBlock, 0, chain[pc.second]>>>(ch, checked ? ctx->d_status : nullptr);
+                        k<<<blocks, kTileBlock, 0, chain[pc.second]>>>(ch, checked ? ctx->d_status : nullptr);
                     }
                 } else {
                     std::vector<double> wt(b->jobs.size());

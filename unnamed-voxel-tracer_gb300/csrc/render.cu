@@ -17,7 +17,11 @@ namespace vt {
 
 // 256-thread blocks; each warp traces a compact pixel tile so that its rays
 // start close together and share brick words in L1.
-constexpr int kBlock = 256;  // 128 measured the same with the register cap
+constexpr int kBlock = 256;
+// The default frame kernel's block without bounce rays: smaller blocks fill the
+// last wave better (1080p 103.4 -> 101.8 us, 640x360 12.7 -> 12.0); with bounce
+// rays 256 is faster (4K 1108 against 1124 us).
+constexpr int kSmallBlock = 128;
 constexpr size_t kMaxSharedCoarse = 48 * 1024;
 
 template <bool STATS>
@@ -35,28 +39,28 @@ __device__ __forceinline__ void flush_counters(PixelCounters& pc, unsigned long 
 // budget so that kOccBlocks blocks fit on an SM: 4 blocks (64 registers, 32
 // warps, no spills) measured 4% faster on a 1080p frame than 5 (48 registers
 // with spills) and 3 (uncapped, 67 registers).
-constexpr int kOccBlocks = 4 * 256 / kBlock;
-template <int TW>
+constexpr int kOccThreads = 4 * 256;
+template <int TW, int NB = kBlock>
 struct BlockTile {
     static constexpr int kW = TW < 16 ? 16 : TW;     // block tile width
     static constexpr int kWarpsX = kW / TW;
-    static constexpr int kH = (kBlock / 32 / kWarpsX) * (32 / TW);
-    static_assert(kW <= 64 && kH <= kBlock - 64, "the column and row tables are filled by distinct threads");
+    static constexpr int kH = (NB / 32 / kWarpsX) * (32 / TW);
+    static_assert(kW <= 64 && kH <= NB - 64, "the column and row tables are filled by distinct threads");
 };
 
 // SHARE: the lanes of a warp that look up the same brick word share one load
 // (Walker::brick_word).  BIN: deferred bounce rays are appended per block,
 // sorted by direction (stage_flush).
 template <bool STATS, bool CHECKED, bool SMEM, int TW, bool OCC, bool SHARE = false, bool BIN = false, bool BOUNCE = true,
-          bool LONG = true>
-__global__ void __launch_bounds__(kBlock, OCC ? kOccBlocks : 1) k_render(const __grid_constant__ WorldView w, const __grid_constant__ FrameParams f, uint4* __restrict__ out,
+          bool LONG = true, int NB = kBlock>
+__global__ void __launch_bounds__(NB, OCC ? kOccThreads / NB : 1) k_render(const __grid_constant__ WorldView w, const __grid_constant__ FrameParams f, uint4* __restrict__ out,
                                                                unsigned* status, unsigned long long* counters) {
     // shared copy of the coarse bits for the model traversal (STATS or
     // CHECKED); the production walk reads the chunk distances through L1,
     // which measured faster than staging all 8 octant fields per block
     extern __shared__ uint4 s_dyn[];
     unsigned long long* s_coarse = reinterpret_cast<unsigned long long*>(s_dyn);
-    using BT = BlockTile<TW>;
+    using BT = BlockTile<TW, NB>;
     // screen coordinates of the block's columns and rows, once per block
     // instead of four divisions per pixel
     __shared__ float s_col[3][BT::kW], s_row[3][BT::kH];
@@ -104,8 +108,13 @@ __global__ void __launch_bounds__(kBlock, OCC ? kOccBlocks : 1) k_render(const _
 }
 
 // Explicit ray list (production traversal); record.rgba is 0.
+// Bound: latency and issue (70%) at 9.5 lanes, the rays being unrelated; a
+// block waits for its longest ray, so blocks are two warps (a million rays:
+// 74.5 us in blocks of 256, 72.3 of 128, 71.6 of 64, 75.1 of 32; 64 with 16 to
+// 24 blocks per SM 70.7-72.7).  Lanes that take the next ray as theirs ends: 88 us.
+constexpr int kRayBlock = 64;
 template <bool LONG>
-__global__ void __launch_bounds__(kBlock) k_trace_rays(const __grid_constant__ WorldView w, const float* __restrict__ origins,
+__global__ void __launch_bounds__(kRayBlock, 16) k_trace_rays(const __grid_constant__ WorldView w, const float* __restrict__ origins,
                                                        const float* __restrict__ dirs, int n, int max_steps,
                                                        uint4* __restrict__ out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -521,11 +530,11 @@ vt_status launch_render(vt_ctx* ctx, const vt_world* world, const vt_camera* cam
             const bool bounce = (p->rays & VT_RAYS_BOUNCE) != 0, lng = long_steps(f);
             auto k = bounce ? (lng ? k_render<false, false, false, 8, true, false, false, true, true>
                                    : k_render<false, false, false, 8, true, false, false, true, false>)
-                            : (lng ? k_render<false, false, false, 8, true, false, false, false, true>
-                                   : k_render<false, false, false, 8, true, false, false, false, false>);
-            le = launch_kernel(k, dim3((cam->width + BlockTile<8>::kW - 1) / BlockTile<8>::kW,
-                                       (rows + BlockTile<8>::kH - 1) / BlockTile<8>::kH),
-                               dim3(kBlock), sm, stream, win, w, f, d_out, ctx->d_status, ctx->d_counters);
+                            : (lng ? k_render<false, false, false, 8, true, false, false, false, true, kSmallBlock>
+                                   : k_render<false, false, false, 8, true, false, false, false, false, kSmallBlock>);
+            const int th = bounce ? BlockTile<8>::kH : BlockTile<8, kSmallBlock>::kH;
+            le = launch_kernel(k, dim3((cam->width + BlockTile<8>::kW - 1) / BlockTile<8>::kW, (rows + th - 1) / th),
+                               dim3(bounce ? kBlock : kSmallBlock), sm, stream, win, w, f, d_out, ctx->d_status, ctx->d_counters);
         }
         else { VT_LAUNCH(false, false, false, 8, false); }
     }
@@ -677,7 +686,7 @@ vt_status vt_trace_rays(vt_ctx* ctx, const vt_world* world, const float* d_origi
         if (s) return s;
     }
     const WorldView w = world->view();
-    (max_steps > kChunkSteps ? k_trace_rays<true> : k_trace_rays<false>)<<<(n + kBlock - 1) / kBlock, kBlock, 0,
+    (max_steps > kChunkSteps ? k_trace_rays<true> : k_trace_rays<false>)<<<(n + kRayBlock - 1) / kRayBlock, kRayBlock, 0,
                                                                             (cudaStream_t)stream>>>(
         w, d_origins, d_dirs, n, max_steps, reinterpret_cast<uint4*>(d_out));
     VT_CUDA(ctx, cudaGetLastError());
