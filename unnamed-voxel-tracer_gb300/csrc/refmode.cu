@@ -37,7 +37,9 @@ vt_status parse_vox(const uint8_t* bytes, size_t n, std::vector<std::vector<uint
 namespace {
 
 constexpr int kModels = 32768;
-constexpr int kRefBlock = 256;
+// 16 x 8 pixels; 8 blocks per SM (1080p frame 620 us; uncapped 643, 16 x 16
+// pixels 651)
+constexpr int kRefBlock = 128;
 
 struct RefView {
     const unsigned* chunks;
@@ -332,20 +334,20 @@ __global__ void k_brickmap_edit(RefView w, unsigned* data, RefFrame f, int edit_
     if (idx < w.ndata) data[idx] = voxel;
 }
 
-__global__ void __launch_bounds__(kRefBlock) k_render_reference(RefView w, RefFrame f, uint4* __restrict__ out) {
+__global__ void __launch_bounds__(kRefBlock, 8) k_render_reference(RefView w, RefFrame f, uint4* __restrict__ out) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int px = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
-    const int py = blockIdx.y * 16 + (warp >> 1) * 4 + (lane >> 3);
+    const int py = blockIdx.y * (kRefBlock / 16) + (warp >> 1) * 4 + (lane >> 3);
     // The light's sky colour depends on the stored illumination alone, which
     // is the sun's direction or 0: computed once per block.
     __shared__ float s_sky[2][4];
-    if ((threadIdx.x & 127u) == 0u) {
+    if ((threadIdx.x & 31u) == 0u && threadIdx.x < 64u) {
         float il[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (threadIdx.x) {
             const float sun4[4] = {kSun[0], kSun[1], kSun[2], 0.3f};
             unpack8(pack8(sun4), il);
         }
-        sky_ref(il, s_sky[threadIdx.x >> 7]);
+        sky_ref(il, s_sky[threadIdx.x >> 5]);
     }
     __syncthreads();
     if (px >= f.width || py >= f.height) return;
@@ -569,7 +571,7 @@ vt_status vt_render_reference(vt_ctx* ctx, const vt_brickmap* bm, const vt_camer
     f.tan_half = tanf(cam->fov / 2.0f);  // primary.comp.glsl:36, on the host's libm
     f.width = cam->width;
     f.height = cam->height;
-    const dim3 grid((cam->width + 15) / 16, (cam->height + 15) / 16);
+    const dim3 grid((cam->width + 15) / 16, (cam->height + kRefBlock / 16 - 1) / (kRefBlock / 16));
     k_render_reference<<<grid, kRefBlock, 0, (cudaStream_t)stream>>>(view_of(bm), f, reinterpret_cast<uint4*>(d_out));
     VT_CUDA(ctx, cudaGetLastError());
     return VT_OK;
