@@ -42,8 +42,9 @@ struct JobDesc {
 
 constexpr int kBatchBlock = 256;
 constexpr int kUnit = 16;  // pixels per unit side
-// The tile shape's block: 16 x 8 pixels (16 scenes, 40 cameras: 1213 us; 16 x 16
-// pixels 1252).
+// The tile shape's block: 16 x 8 pixels, 9 blocks (36 warps, 56 registers) per
+// SM (16 scenes, 40 cameras: 1207 us; 8 blocks 1231, 10 1209, 16 x 16 pixels
+// 1252).
 constexpr int kTileBlock = 128, kTileH = kTileBlock / kUnit;
 constexpr int kBatchChains = 8;  // 4, 8, 16 and 32 chains measured within 1% on the 64-scene batch
 
@@ -82,9 +83,9 @@ static_assert(sizeof(JobChunk) <= 32764, "a kernel's parameters are limited to 3
 
 // One thread per pixel; the 128-thread block covers a 16 x 8 tile as four
 // 8 x 4 warp tiles (the single-frame kernel's default shape), with the same
-// register cap (32 warps per SM).
+// register cap (36 warps per SM).
 template <bool CHECKED, bool BOUNCE, bool LONG>
-__global__ void __launch_bounds__(kTileBlock, 1024 / kTileBlock) k_render_jobs(const __grid_constant__ JobChunk p, unsigned* status) {
+__global__ void __launch_bounds__(kTileBlock, 9) k_render_jobs(const __grid_constant__ JobChunk p, unsigned* status) {
     const unsigned b = blockIdx.x;
     int lo = 0, hi = p.njobs - 1;
     while (lo < hi) {

@@ -22,6 +22,10 @@ constexpr int kBlock = 256;
 // last wave better (1080p 103.4 -> 101.8 us, 640x360 12.7 -> 12.0); with bounce
 // rays 256 is faster (4K 1108 against 1124 us).
 constexpr int kSmallBlock = 128;
+// Its blocks per SM, 36 warps of 56 registers (8: 101.5 us, 10: 101.6, 11: 105.5,
+// 9: 100.2).
+constexpr int kSmallBlocks = 9;
+
 constexpr size_t kMaxSharedCoarse = 48 * 1024;
 
 template <bool STATS>
@@ -35,10 +39,9 @@ __device__ __forceinline__ void flush_counters(PixelCounters& pc, unsigned long 
 }
 
 // One thread per pixel.  A warp covers a TW x (32 / TW) pixel tile; the
-// 256-thread block covers max(16, TW) pixels across.  OCC caps the register
-// budget so that kOccBlocks blocks fit on an SM: 4 blocks (64 registers, 32
-// warps, no spills) measured 4% faster on a 1080p frame than 5 (48 registers
-// with spills) and 3 (uncapped, 67 registers).
+// NB-thread block covers max(16, TW) pixels across.  OCC caps the register
+// budget so that kOccThreads threads (64 registers, 32 warps) fit on an SM, or
+// kSmallBlocks small blocks.
 constexpr int kOccThreads = 4 * 256;
 template <int TW, int NB = kBlock>
 struct BlockTile {
@@ -53,8 +56,9 @@ struct BlockTile {
 // sorted by direction (stage_flush).
 template <bool STATS, bool CHECKED, bool SMEM, int TW, bool OCC, bool SHARE = false, bool BIN = false, bool BOUNCE = true,
           bool LONG = true, int NB = kBlock>
-__global__ void __launch_bounds__(NB, OCC ? kOccThreads / NB : 1) k_render(const __grid_constant__ WorldView w, const __grid_constant__ FrameParams f, uint4* __restrict__ out,
-                                                               unsigned* status, unsigned long long* counters) {
+__global__ void __launch_bounds__(NB, OCC ? (NB == kSmallBlock ? kSmallBlocks : kOccThreads / NB) : 1)
+    k_render(const __grid_constant__ WorldView w, const __grid_constant__ FrameParams f, uint4* __restrict__ out,
+             unsigned* status, unsigned long long* counters) {
     // shared copy of the coarse bits for the model traversal (STATS or
     // CHECKED); the production walk reads the chunk distances through L1,
     // which measured faster than staging all 8 octant fields per block

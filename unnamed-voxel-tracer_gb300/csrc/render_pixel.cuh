@@ -73,7 +73,6 @@ __device__ __forceinline__ bool trace_sun(const WorldView& w, const FrameParams&
             fw.b[i] = r.oinv[i];
             fw.o[i] = __fmaf_rn(so[i], f.sun_side[i], -0.25f);
             fw.nk[i] = __fmaf_rn(magic_floor(so[i]) - kMagic, f.sun_side[i], f.sun_off[i]);
-            fw.tm[i] = __fmaf_rn(fw.nk[i], fw.a[i], fw.b[i]);
             x[i] = __fmaf_rn(f.sun_exit[i], fw.a[i], fw.b[i]);
         }
         fw.texit = fminf(fminf(x[0], x[1]), x[2]);
@@ -105,7 +104,7 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
     TraceHit h;
     TraceCounters cnt;
     constexpr bool kForward = !STATS && !CHECKED && !SHARE;
-    const bool hit = kForward && (f.cam_inside || near_origin(r.o)) && ordinary_inv(r.inv)
+    const bool hit = kForward && (f.cam_inside || near_origin(r.o)) && ordinary_unit(r.inv)
                          ? trace_primary<LONG>(w, f, r, h)
                          : trace_any<STATS, CHECKED, true, false, SHARE, LONG>(w, coarse, cd, r, f.max_steps, h, cnt, status);
     if (STATS) {

@@ -728,12 +728,17 @@ __host__ __device__ __forceinline__ bool ordinary_inv(const float inv[3]) {
     return a <= 0x1p100f && b <= 0x1p100f && c <= 0x1p100f && a >= 0x1p-100f && b >= 0x1p-100f && c >= 0x1p-100f;
 }
 
+// The same for a direction of length about 1, whose reciprocals are about 1 or
+// more.
+__device__ __forceinline__ bool ordinary_unit(const float inv[3]) {
+    return fabsf(inv[0]) <= 0x1p100f && fabsf(inv[1]) <= 0x1p100f && fabsf(inv[2]) <= 0x1p100f;
+}
+
 struct FwdWalk {
     float d[3], o[3];  // |direction|; mirrored origin less a quarter
     float a[3], b[3];  // plane time of k: fma(k, a, b)
     int m[3];          // 0, or -1 where the axis is mirrored
     float nk[3];       // next plane per axis
-    float tm[3];       // its crossing time
     float t;           // entry time of the current cell
     float texit;       // earliest exit plane time of the grid
     float limit;       // sum of nk at which the step limit is reached
@@ -767,7 +772,6 @@ struct FwdWalk {
             a[i] = fabsf(r.inv[i]);
             b[i] = r.oinv[i];
             nk[i] = sign ? -c[i] : c[i] + 1.0f;
-            tm[i] = __fmaf_rn(nk[i], a[i], b[i]);
             x[i] = __fmaf_rn(sign ? 0.0f : __int2float_rn(w.dims[i]), a[i], b[i]);
         }
         texit = fminf(fminf(x[0], x[1]), x[2]);
@@ -828,6 +832,9 @@ struct FwdWalk {
             // tie) crosses another plane first and the brick is looked up again
             const float tb = fminf(fminf(__fmaf_rn(far[0], a[0], b[0]), __fmaf_rn(far[1], a[1], b[1])),
                                    __fmaf_rn(far[2], a[2], b[2]));
+            float tm[3];   // the next planes' crossing times
+#pragma unroll
+            for (int i = 0; i < 3; ++i) tm[i] = __fmaf_rn(nk[i], a[i], b[i]);
             for (;;) {
                 VT_STEP_HOOK(2);
                 vb = ((unsigned)float_bits(vf) ^ flip) & 63u;
@@ -886,8 +893,6 @@ struct FwdWalk {
             nk[0] = fmaxf(p0, nk[0]);
             nk[1] = fmaxf(p1, nk[1]);
             nk[2] = fmaxf(p2, nk[2]);
-#pragma unroll
-            for (int i = 0; i < 3; ++i) tm[i] = __fmaf_rn(nk[i], a[i], b[i]);
         }
         if ((nk[0] + nk[1]) + nk[2] >= limit || t >= texit) {
             if ((nk[0] + nk[1]) + nk[2] >= limit || outside(w)) return kMiss;
