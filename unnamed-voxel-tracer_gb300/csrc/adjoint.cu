@@ -31,8 +31,8 @@ struct AdjArgs {
     WorldView w;
     const float* pal;
     const float* alb;
-    float sun_d[3], sun_inv[3];   // the shadow rays' direction as traced, and its reciprocal (FrameParams)
-    float sun_raw[3];             // as given (entity boxes)
+    SunWalk sun;                  // the shadow rays
+    float sun_raw[3];             // the sun as given (entity boxes)
     float sun_n[3], inv_len;
     float ka, kd;
     int shadow_steps;
@@ -95,10 +95,10 @@ __device__ __forceinline__ float warp_sum4(unsigned lane, float a, float b, floa
 // 166 -> 130 us against one tile per block, a sum over the warp per value and
 // tile, and the general walk inlined beside the forward one.  GENERAL: long
 // step limits, or a sun direction the forward walk does not take (trace_fast).
-// Register caps: 7 and 6 blocks per SM, the fastest of 4-8 (36 and 40
-// registers, a few bytes spilled).
+// Register caps: 6 blocks per SM forward (40 registers) and 5 backward (48), an
+// iteration 239.5 us; 7 and 6 242.4, 5 and 6 244.0, 6 and 4 247.
 template <bool BWD, bool GENERAL>
-__global__ void __launch_bounds__(kAdjBlock, BWD ? 6 : 7) k_shade_views(const __grid_constant__ ViewsArgs va) {
+__global__ void __launch_bounds__(kAdjBlock, BWD ? 5 : 6) k_shade_views(const __grid_constant__ ViewsArgs va) {
     const AdjArgs& a = va.a;
     const ViewP& V = va.v[blockIdx.z];
     __shared__ float s_gpal[BWD ? 768 : 1], s_acc[4];   // palette gradient; loss and sun
@@ -160,11 +160,16 @@ __global__ void __launch_bounds__(kAdjBlock, BWD ? 6 : 7) k_shade_views(const __
                 if (a.vis_in) {
                     lit = a.vis_in[p] != 0;
                 } else {
-                    PRay rs;
-                    pray_init_dir(rs, so, a.sun_d, a.sun_inv);
-                    TraceHit hs;
-                    lit = !(GENERAL ? trace_fast<false, true, true>(a.w, a.w.cdist, rs, a.shadow_steps, hs)
-                                    : trace_ordinary<false, false>(a.w, rs, a.shadow_steps, hs)) &&
+                    bool blocked;
+                    if (GENERAL) {
+                        PRay rs;
+                        pray_init_dir(rs, so, a.sun.d, a.sun.inv);
+                        TraceHit hs;
+                        blocked = trace_fast<false, true, true>(a.w, a.w.cdist, rs, a.shadow_steps, hs);
+                    } else {
+                        blocked = trace_sun<false>(a.w, a.sun, so, a.shadow_steps);
+                    }
+                    lit = !blocked &&
                           !(a.w.n_entities > 0 && entity_occluded(a.w, so, a.sun_raw));
                 }
                 ndl_raw = dot3(nrm, a.sun_n);
@@ -273,10 +278,9 @@ vt_status prepare_shade(vt_ctx* ctx, const vt_world* world, const vt_shade_input
     a.alb = in->d_albedo;
     for (int j = 0; j < 3; ++j) {
         a.sun_raw[j] = in->sun[j];
-        a.sun_d[j] = f.sun_d[j];
-        a.sun_inv[j] = f.sun_inv[j];
         a.sun_n[j] = f.sun_n[j];
     }
+    a.sun = sun_walk(f, a.w);
     a.inv_len = 1.0f / sqrtf(len2);
     a.ka = in->ambient;
     a.kd = in->diffuse;
@@ -319,7 +323,7 @@ vt_status launch_shade_views(vt_ctx* ctx, const vt_world* world, int32_t n, cons
         s = shade_sums(ctx, st, &a.sums, &used);
         if (s) return s;
     }
-    const bool general = a.shadow_steps > kChunkSteps || !ordinary_inv(a.sun_inv);
+    const bool general = a.shadow_steps > kChunkSteps || !ordinary_inv(a.sun.inv);
     auto k = bwd ? (general ? k_shade_views<true, true> : k_shade_views<true, false>)
                  : (general ? k_shade_views<false, true> : k_shade_views<false, false>);
     ViewsArgs va;

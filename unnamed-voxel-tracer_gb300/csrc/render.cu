@@ -332,27 +332,34 @@ FrameParams make_frame(const vt_camera* cam, const vt_params* p) {
     return f;
 }
 
-void walk_constants(FrameParams& f, const WorldView& w) {
-    f.cam_inside = near_origin(f.pos) ? 1 : 0;
-    for (int j = 0; j < 3; ++j) {
-        f.in_hi[j] = (float)(w.dims[j] - 1);
-        if (!(f.pos[j] >= 1.0f && f.pos[j] <= f.in_hi[j])) f.cam_inside = 0;
-    }
-    for (int j = 0; j < 3; ++j) f.cam_c[j] = f.cam_inside ? floorf(f.pos[j]) : 0.0f;
+SunWalk sun_walk(const FrameParams& f, const WorldView& w) {
+    SunWalk s;
     unsigned oct = 0;
-    f.sun_flip = 0;
+    s.flip = 0;
     for (int j = 0; j < 3; ++j) {
         const bool up = f.sun_d[j] > 0.0f;
-        f.sun_m[j] = up ? 0 : -1;
-        f.sun_side[j] = up ? 1.0f : -1.0f;
-        f.sun_off[j] = up ? 1.0f : 0.0f;
-        f.sun_ad[j] = fabsf(f.sun_d[j]);
-        f.sun_ai[j] = fabsf(f.sun_inv[j]);
-        f.sun_exit[j] = up ? (float)w.dims[j] : 0.0f;
+        s.d[j] = f.sun_d[j];
+        s.inv[j] = f.sun_inv[j];
+        s.m[j] = up ? 0 : -1;
+        s.side[j] = up ? 1.0f : -1.0f;
+        s.off[j] = up ? 1.0f : 0.0f;
+        s.ad[j] = fabsf(f.sun_d[j]);
+        s.ai[j] = fabsf(f.sun_inv[j]);
+        s.exit[j] = up ? (float)w.dims[j] : 0.0f;
+        s.in_hi[j] = (float)(w.dims[j] - 1);
         if (up) oct |= 1u << j;
-        else f.sun_flip |= 3u << (2 * j);
+        else s.flip |= 3u << (2 * j);
     }
-    f.sun_field = oct * w.nwords;
+    s.field = oct * w.nwords;
+    return s;
+}
+
+void walk_constants(FrameParams& f, const WorldView& w) {
+    f.cam_inside = near_origin(f.pos) ? 1 : 0;
+    for (int j = 0; j < 3; ++j)
+        if (!(f.pos[j] >= 1.0f && f.pos[j] <= (float)(w.dims[j] - 1))) f.cam_inside = 0;
+    for (int j = 0; j < 3; ++j) f.cam_c[j] = f.cam_inside ? floorf(f.pos[j]) : 0.0f;
+    f.sunw = sun_walk(f, w);
 }
 
 vt_status check_frame_args(vt_ctx* ctx, const vt_world* world, const vt_camera* cam, const vt_params* p) {

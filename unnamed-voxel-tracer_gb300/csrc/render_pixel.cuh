@@ -49,42 +49,6 @@ __device__ __forceinline__ bool trace_primary(const WorldView& w, const FramePar
     return go && fw.finish<true, LONG>(w, r, h);
 }
 
-// The shadow ray from so: the fields of its walk that depend on the sun alone
-// are the frame's (walk_constants), and an origin at least one cell inside
-// the grid starts in its own cell (pray_start).
-template <bool LONG>
-__device__ __forceinline__ bool trace_sun(const WorldView& w, const FrameParams& f, const float so[3]) {
-    PRay r;
-    pray_init_dir(r, so, f.sun_d, f.sun_inv);
-    TraceHit h;
-    FwdWalk fw;
-    const bool inside = so[0] >= 1.0f && so[1] >= 1.0f && so[2] >= 1.0f && so[0] <= f.in_hi[0] && so[1] <= f.in_hi[1] &&
-                        so[2] <= f.in_hi[2];
-    bool go = true;
-    if (inside) {
-        if (f.shadow_max_steps <= 0) return false;
-        fw.t = 0.0f;
-        float x[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            fw.m[i] = f.sun_m[i];
-            fw.d[i] = f.sun_ad[i];
-            fw.a[i] = f.sun_ai[i];
-            fw.b[i] = r.oinv[i];
-            fw.o[i] = __fmaf_rn(so[i], f.sun_side[i], -0.25f);
-            fw.nk[i] = __fmaf_rn(magic_floor(so[i]) - kMagic, f.sun_side[i], f.sun_off[i]);
-            x[i] = __fmaf_rn(f.sun_exit[i], fw.a[i], fw.b[i]);
-        }
-        fw.texit = fminf(fminf(x[0], x[1]), x[2]);
-        fw.limit = ((fw.nk[0] + fw.nk[1]) + fw.nk[2]) + __int2float_rn(min(f.shadow_max_steps, 1 << 20));
-        fw.flip = f.sun_flip;
-        fw.field = f.sun_field;
-    } else {
-        go = fw.start(w, r, f.shadow_max_steps);
-    }
-    return go && fw.finish<false, LONG>(w, r, h);
-}
-
 // uv: the pixel's screen coordinates (pixel_uv(f, px, py); the frame kernel
 // reads them from the frame's screen table or its per-block tables).
 // BIN: a deferred bounce ray is staged in the block's shared memory for the
@@ -137,7 +101,7 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
         bool shadowed = false;
         if (f.rays & VT_RAYS_SHADOW) {
             if (kForward && (!LONG || ordinary_inv(f.sun_inv))) {
-                shadowed = trace_sun<LONG>(w, f, so);
+                shadowed = trace_sun<LONG>(w, f.sunw, so, f.shadow_max_steps);
             } else {
                 PRay rs;
                 pray_init_dir(rs, so, f.sun_d, f.sun_inv);

@@ -33,17 +33,11 @@ struct FrameParams {
     float lit_a;        // illumination alpha 0.3 stored in RGBA8
     float sun_d[3];     // the shadow rays' direction as traced (a zero component made 0.001, map.glsl:85-90)
     float sun_inv[3];   // its correctly rounded reciprocal
-    // of the frame's world (walk_constants): where the camera's rays start,
-    // and the shadow rays' fields of FwdWalk, the same for all of them
+    // of the frame's world (walk_constants): where the camera's rays start, and
+    // the shadow rays' walk
     int cam_inside;     // the camera is near and at least one cell inside the grid:
     float cam_c[3];     // its cell
-    float in_hi[3];     // the grid's sides less one
-    int sun_m[3];       // 0, or -1 where it moves down the axis
-    float sun_side[3];  // 1, or -1 where the shadow ray moves down the axis
-    float sun_off[3];   // 1 or 0: the plane after cell c is sun_side * c + sun_off
-    float sun_ad[3], sun_ai[3];  // |sun_d|, |sun_inv|
-    float sun_exit[3];  // the grid's last plane, mirrored
-    unsigned sun_flip, sun_field;
+    SunWalk sunw;
     float cross_r2;     // the largest x with sqrt(x) <= 0.002 (crosshair radius test without a square root)
     int row0, row_end;  // rows [row0, row_end) of the image this launch renders
     void* bounce_head;       // non-null: bounce rays are queued here (BounceHead), not traced inline
@@ -350,6 +344,8 @@ FrameParams make_frame(const vt_camera* cam, const vt_params* p);
 // The constants that depend on the frame's world too (host side; after the
 // camera's and frame_constants).
 void walk_constants(FrameParams& f, const WorldView& w);
+// SunWalk of f's sun (after frame_constants) in w.
+SunWalk sun_walk(const FrameParams& f, const WorldView& w);
 
 // The per-frame constants of FrameParams (host side).
 inline void frame_constants(FrameParams& f) {

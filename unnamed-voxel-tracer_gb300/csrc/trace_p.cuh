@@ -938,6 +938,42 @@ __device__ __forceinline__ bool trace_ordinary(const WorldView& w, const PRay& r
     return fw.start(w, r, max_steps) && fw.finish<MAT, LONG>(w, r, h);
 }
 
+// Whether the shadow ray from so is blocked (a sun that passes ordinary_inv):
+// the fields of its walk that depend on the sun alone are given, and an origin
+// at least one cell inside the grid starts in its own cell (pray_start).
+template <bool LONG>
+__device__ __forceinline__ bool trace_sun(const WorldView& w, const SunWalk& sun, const float so[3], int max_steps) {
+    PRay r;
+    pray_init_dir(r, so, sun.d, sun.inv);
+    TraceHit h;
+    FwdWalk fw;
+    const bool inside = so[0] >= 1.0f && so[1] >= 1.0f && so[2] >= 1.0f && so[0] <= sun.in_hi[0] &&
+                        so[1] <= sun.in_hi[1] && so[2] <= sun.in_hi[2];
+    bool go = true;
+    if (inside) {
+        if (max_steps <= 0) return false;
+        fw.t = 0.0f;
+        float x[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            fw.m[i] = sun.m[i];
+            fw.d[i] = sun.ad[i];
+            fw.a[i] = sun.ai[i];
+            fw.b[i] = r.oinv[i];
+            fw.o[i] = __fmaf_rn(so[i], sun.side[i], -0.25f);
+            fw.nk[i] = __fmaf_rn(magic_floor(so[i]) - kMagic, sun.side[i], sun.off[i]);
+            x[i] = __fmaf_rn(sun.exit[i], fw.a[i], fw.b[i]);
+        }
+        fw.texit = fminf(fminf(x[0], x[1]), x[2]);
+        fw.limit = ((fw.nk[0] + fw.nk[1]) + fw.nk[2]) + __int2float_rn(min(max_steps, 1 << 20));
+        fw.flip = sun.flip;
+        fw.field = sun.field;
+    } else {
+        go = fw.start(w, r, max_steps);
+    }
+    return go && fw.finish<false, LONG>(w, r, h);
+}
+
 // Traces one ray to its end.  NEAR: the origin passes near_origin; SHARE:
 // brick words shared between the lanes of a warp (Walker only); LONG: step
 // limits above kChunkSteps (chunk jumps; without them only speed is lost).

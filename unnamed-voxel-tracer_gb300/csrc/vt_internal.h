@@ -42,6 +42,19 @@ struct WorldView {
     unsigned cstride;                   // bytes per chunk-distance field (nchunks rounded up to 16)
 };
 
+// The fields of the shadow rays' forward walk (FwdWalk) that depend on the sun
+// and the world alone.
+struct SunWalk {
+    float d[3], inv[3];   // the direction as traced (a zero component made 0.001, map.glsl:85-90), its reciprocal
+    int m[3];             // 0, or -1 where the ray moves down the axis
+    float side[3];        // 1, or -1 there
+    float off[3];         // 1, or 0 there: the plane after cell c is side * c + off
+    float ad[3], ai[3];   // |d|, |inv|
+    float exit[3];        // the grid's last plane, mirrored
+    float in_hi[3];       // the grid's sides less one
+    unsigned flip, field;
+};
+
 // Cap of the chunk distances: a stored value d >= 1 promises that every
 // chunk within radius d - 1 ahead is empty.
 constexpr int kDistCap = 15;
