@@ -328,7 +328,8 @@ vt_status launch_shade_views(vt_ctx* ctx, const vt_world* world, int32_t n, cons
                  : (general ? k_shade_views<false, true> : k_shade_views<false, false>);
     ViewsArgs va;
     std::memset(&va, 0, sizeof(va));
-    for (int v0 = 0; v0 < n; v0 += kMaxViews) {
+    cudaError_t e = cudaSuccess;
+    for (int v0 = 0; v0 < n && e == cudaSuccess; v0 += kMaxViews) {
         const int nv = n - v0 < kMaxViews ? n - v0 : kMaxViews;
         int gw = 0, gh = 0;
         size_t tiles = 0;
@@ -356,14 +357,14 @@ vt_status launch_shade_views(vt_ctx* ctx, const vt_world* world, int32_t n, cons
         va.a = a;
         const dim3 grid((gw + 16 * a.tiles - 1) / (16 * a.tiles), (gh + 15) / 16, nv);
         k<<<grid, kAdjBlock, 0, st>>>(va);
-        VT_CUDA(ctx, cudaGetLastError());
+        e = cudaGetLastError();
     }
-    if (a.sums) {
+    if (a.sums) {   // (after a failed launch too: the region is left zero)
         k_shade_sums<<<1, kAdjBlock, 0, st>>>(a);
-        VT_CUDA(ctx, cudaGetLastError());
-        VT_CUDA(ctx, cudaEventRecord(used, st));
+        const cudaError_t es = cudaGetLastError(), er = cudaEventRecord(used, st);
+        if (e == cudaSuccess) e = es != cudaSuccess ? es : er;
     }
-    return VT_OK;
+    return e == cudaSuccess ? VT_OK : check_cuda(ctx, e, "shading launch");
 }
 
 }  // namespace

@@ -104,10 +104,7 @@ __global__ void __launch_bounds__(512) k_set_voxel(WorldView w, unsigned long lo
 // `stride` bytes apart.  The pass covers the whole chunk grid.
 // The window's reads are independent and all in flight at once.
 __device__ __forceinline__ void dist_cell(const unsigned long long* coarse, const unsigned char* in, unsigned char* out,
-                                          int axis, int CX, int CY, int CZ, size_t stride, unsigned v, unsigned lin) {
-    const bool fwd = ((v >> axis) & 1u) != 0u;
-    if (axis > 0) in += (size_t)(v & ((1u << axis) - 1u)) * stride;
-    out += (size_t)v * stride;
+                                          int axis, bool fwd, int CX, int CY, int CZ, unsigned lin) {
     const unsigned p[3] = {lin % (unsigned)CX, (lin / (unsigned)CX) % (unsigned)CY, lin / ((unsigned)CX * (unsigned)CY)};
     const int u = (int)(axis == 0 ? p[0] : (axis == 1 ? p[1] : p[2])), g = axis == 0 ? CX : (axis == 1 ? CY : CZ);
     const int step = (axis == 0 ? 1 : (axis == 1 ? CX : CX * CY)) * (fwd ? 1 : -1);
@@ -132,23 +129,30 @@ __device__ __forceinline__ void dist_cell(const unsigned long long* coarse, cons
 __global__ void k_dist_pass(const unsigned long long* coarse, const unsigned char* in, unsigned char* out, int axis,
                             int CX, int CY, int CZ, size_t stride, const int* d_changed) {
     if (d_changed && !*d_changed) return;
-    const unsigned lin = blockIdx.x * blockDim.x + threadIdx.x;
-    if (lin < (unsigned)CX * (unsigned)CY * (unsigned)CZ) dist_cell(coarse, in, out, axis, CX, CY, CZ, stride, blockIdx.y, lin);
+    const unsigned v = blockIdx.y, lin = blockIdx.x * blockDim.x + threadIdx.x;
+    if (lin >= (unsigned)CX * (unsigned)CY * (unsigned)CZ) return;
+    if (axis > 0) in += (size_t)(v & ((1u << axis) - 1u)) * stride;
+    dist_cell(coarse, in, out + (size_t)v * stride, axis, ((v >> axis) & 1u) != 0u, CX, CY, CZ, lin);
 }
 
-// The three passes after a device-side edit of a small grid as one block, one
-// launch instead of three that mostly find nothing to do.
-__global__ void __launch_bounds__(1024) k_dist_edit(const unsigned long long* coarse, unsigned char* fx, unsigned char* fy,
-                                                    unsigned char* out, int CX, int CY, int CZ, size_t stride,
-                                                    const int* d_changed) {
-    if (!*d_changed) return;
-    const unsigned n = (unsigned)CX * (unsigned)CY * (unsigned)CZ;
-    for (int axis = 0; axis < 3; ++axis) {
-        const unsigned char* in = axis == 1 ? fx : fy;
-        unsigned char* to = axis == 0 ? fx : (axis == 1 ? fy : out);
-        for (unsigned i = threadIdx.x; i < (n << (axis + 1)); i += 1024u) dist_cell(coarse, in, to, axis, CX, CY, CZ, stride, i / n, i % n);
-        __syncthreads();
-    }
+// The three passes of a small grid in one launch, a block per octant (output
+// field), which keeps its own x and y results in shared memory.  Bound: the
+// latency of a few dependent rounds of loads.  2048 chunks: 9.1 us against 9.2
+// in three launches and the gaps between them; after an edit that changed a
+// coarse bit 9.3 us against 36 as one block for all octants, after one that
+// changed none (the rule for single voxels) 2.7 against 8.
+constexpr int kSmallChunks = 4096;
+__global__ void __launch_bounds__(1024) k_dist_small(const unsigned long long* coarse, unsigned char* out, int CX, int CY,
+                                                     int CZ, size_t stride, const int* d_changed) {
+    if (d_changed && !*d_changed) return;
+    __shared__ unsigned char fx[kSmallChunks], fy[kSmallChunks];
+    const unsigned n = (unsigned)CX * (unsigned)CY * (unsigned)CZ, v = blockIdx.x;
+    for (unsigned i = threadIdx.x; i < n; i += 1024u) dist_cell(coarse, nullptr, fx, 0, (v & 1u) != 0u, CX, CY, CZ, i);
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < n; i += 1024u) dist_cell(nullptr, fx, fy, 1, (v & 2u) != 0u, CX, CY, CZ, i);
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < n; i += 1024u)
+        dist_cell(nullptr, fy, out + (size_t)v * stride, 2, (v & 4u) != 0u, CX, CY, CZ, i);
 }
 
 // Brick level, in voxels.  With vertical weight w = 2^shape, brick b has
@@ -420,19 +424,17 @@ size_t volume(int3 e) { return (size_t)e.x * e.y * e.z; }
 
 // The chunk level over the whole chunk grid (at most a few tens of thousands
 // of cells: cheap enough to redo after any edit, and skipped on the device
-// after an edit that changed no coarse bit, the rule for single voxels): x into 2 fields of tmp, y
-// into the 4 fields after them, z into the 8 output fields.
+// after an edit that changed no coarse bit); of a larger grid x into 2 fields
+// of tmp, y into the 4 fields after them, z into the 8 output fields.
 void chunk_passes(vt_world* w, cudaStream_t st, const int* d_changed) {
     const int CX = w->cdim[0], CY = w->cdim[1], CZ = w->cdim[2];
     const size_t stride = cdist_stride((unsigned)w->nchunks);
-    unsigned char* fx = w->d_ctmp;
-    unsigned char* fy = w->d_ctmp + 2 * stride;
-    // (2048 chunks in one block: 15 us when a coarse bit changed against 9, 2.7
-    // against 8 when none did)
-    if (d_changed && w->nchunks <= 4096) {
-        k_dist_edit<<<1, 1024, 0, st>>>(w->d_coarse, fx, fy, w->d_cdist, CX, CY, CZ, stride, d_changed);
+    if (w->nchunks <= kSmallChunks) {
+        k_dist_small<<<8, 1024, 0, st>>>(w->d_coarse, w->d_cdist, CX, CY, CZ, stride, d_changed);
         return;
     }
+    unsigned char* fx = w->d_ctmp;
+    unsigned char* fy = w->d_ctmp + 2 * stride;
     const unsigned nb = dist_blocks(w->nchunks);
     k_dist_pass<<<dim3(nb, 2), kDistThreads, 0, st>>>(w->d_coarse, nullptr, fx, 0, CX, CY, CZ, stride, d_changed);
     k_dist_pass<<<dim3(nb, 4), kDistThreads, 0, st>>>(w->d_coarse, fx, fy, 1, CX, CY, CZ, stride, d_changed);
