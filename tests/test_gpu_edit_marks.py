@@ -1,6 +1,6 @@
 """Device-side edits whose distance updates are cut down (x pass in the edit's
 block, z pass only over column groups the y pass changed, chunk passes only
-when a coarse bit changed, one block or three launches by grid size): after
+when a coarse bit changed, one or three launches by grid size): after
 every edit the distances equal a fresh upload's."""
 import numpy as np
 import pytest
@@ -19,7 +19,7 @@ def same_as_fresh(vt, ctx, w, dims):
         f.close()
 
 
-# the last has more chunks than the one-block chunk passes take
+# the last has more chunks than the one-launch chunk passes take
 @pytest.mark.parametrize("dims", [(150, 70, 140), (33, 200, 35), (700, 64, 3072)])
 def test_edits_against_fresh_uploads(vt, ctx, dims):
     X, Y, Z = dims

@@ -91,9 +91,11 @@ __device__ __forceinline__ float warp_sum4(unsigned lane, float a, float b, floa
 // the shadow walks; the backward one adds the loss and gradients, per thread
 // over the block's tiles for the loss and the sun, in shared memory for the
 // palette, so that a block clears, sums and flushes them once.
-// Bound: issue slots (77-80%).  16 views of 512x512: forward 101 us, backward
-// 166 -> 130 us against one tile per block, a sum over the warp per value and
-// tile, and the general walk inlined beside the forward one.  GENERAL: long
+// Bound: issue slots (forward 81%, backward 73% with its albedo atomics waiting
+// for L2).  16 views of 512x512: forward 92 us, backward 121 us (166 with one
+// tile per block, a sum over the warp per value and tile, and the general walk
+// inlined beside the forward one; 101 and 130 with the sun's walk constants per
+// ray).  GENERAL: long
 // step limits, or a sun direction the forward walk does not take (trace_fast).
 // Register caps: 6 blocks per SM forward (40 registers) and 5 backward (48), an
 // iteration 239.5 us; 7 and 6 242.4, 5 and 6 244.0, 6 and 4 247.

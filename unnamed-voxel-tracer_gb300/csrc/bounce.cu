@@ -13,7 +13,8 @@ constexpr int kBounceBlock = 256;
 // a warp takes new rays from the queue once this many of its lanes are idle
 // (tuning bounce_refill), and a busy lane makes kActions iterations of the walk
 // between two refill checks: 12 and 3 are fastest of 4-16 and 1-4 with the
-// forward walk (4K cave frame 1145 us; 8 and 2: 1182, 16 and 4: 1146)
+// forward walk (4K cave frame as first measured 1145 us; 8 and 2: 1182, 16 and
+// 4: 1146; refill alone, now: 12 1120 us, 4 1141, 8 1138, 16 1118)
 constexpr int kRefill = 12;
 constexpr int kActions = 3;
 
@@ -67,7 +68,7 @@ __device__ __forceinline__ void open_pixel(uint4* out, unsigned pixel, unsigned 
 // Bound: issue slots (76%) at 12 lanes an instruction, the lanes of a warp
 // being in different phases of unrelated walks; the register cap (4 blocks of
 // 64 registers; uncapped 96) hides the lookups' latency.  7 M rays of a 4K
-// cave frame: 614 us.  Measured slower: setting 32 rays up at a time in shared
+// cave frame: 601 us.  Measured against 614 then, slower: setting 32 rays up at a time in shared
 // memory for idle lanes to take (727 us: the copies cost more instructions
 // than the set-ups at few lanes), one code path for jumps and unit steps (568 us
 // here, but 11% slower on a 1021x577 frame whose queue is short).
