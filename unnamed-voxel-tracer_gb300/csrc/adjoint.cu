@@ -12,10 +12,10 @@
 // the hit exactly as the render kernel does (same origin arithmetic, same
 // traversal), instead of being stored between passes.  The backward kernel is
 // the forward kernel plus the loss and gradient epilogue, one thread per
-// pixel of up to four tiles.  Palette gradients are summed per warp over the
-// lanes that share a material (the warp walks its distinct materials), per
-// block in shared memory, then once per block with global atomics; albedo
-// gradients go to global memory with one atomic per pixel.
+// pixel.  Palette gradients are summed per warp over the lanes that share a
+// material (the warp walks its distinct materials), per block in shared memory,
+// then once per block with global atomics; albedo gradients go to global memory
+// with one atomic per pixel.
 #include <cstring>
 
 #include "shade.cuh"
@@ -36,7 +36,6 @@ struct AdjArgs {
     float sun_n[3], inv_len;
     float ka, kd;
     int shadow_steps;
-    int tiles;                    // 16x16-pixel tiles a block shades, side by side
     const unsigned char* vis_in;
     unsigned char* vis_out;
     float* loss;
@@ -59,7 +58,6 @@ __device__ __forceinline__ float* grad_sum(const AdjArgs& a, int i) {
 // Several views of one world in one launch (blockIdx.z = view): one launch
 // instead of one per view, whose tails would leave the GPU partly idle.
 constexpr int kMaxViews = 16;
-constexpr int kMaxTiles = 4;
 struct ViewP {
     float pos[3];
     float view[16];
@@ -87,31 +85,44 @@ __device__ __forceinline__ float warp_sum4(unsigned lane, float a, float b, floa
     return r;
 }
 
-// One block: a.tiles tiles of 16x16 pixels in a row.  The forward kernel is
-// the shadow walks; the backward one adds the loss and gradients, per thread
-// over the block's tiles for the loss and the sun, in shared memory for the
-// palette, so that a block clears, sums and flushes them once.
-// Bound: issue slots (forward 81%, backward 73% with its albedo atomics waiting
-// for L2).  16 views of 512x512: forward 92 us, backward 121 us (166 with one
-// tile per block, a sum over the warp per value and tile, and the general walk
-// inlined beside the forward one; 101 and 130 with the sun's walk constants per
-// ray).  GENERAL: long
-// step limits, or a sun direction the forward walk does not take (trace_fast).
-// Register caps: 6 blocks per SM forward (40 registers) and 5 backward (48), an
-// iteration 239.5 us; 7 and 6 242.4, 5 and 6 244.0, 6 and 4 247.
+// One block: 16x16 pixels.  The forward kernel is the shadow walks; the
+// backward one adds the loss and gradients.
+//
+// A block shades one tile, and blocks start in the order of the views and of
+// the tiles in a view: a voxel's albedo gradient is then summed in about that
+// order, as by one call per view.  Blocks of four tiles side by side, which
+// clear and flush their sums once for four, take 241 us an iteration instead of
+// 258, but keep three views of 512x512 in flight at once: a voxel that fills
+// much of several views gets 1e4 to 1e5 float addends, whose rounding goes one
+// way within a binade, and the gradients of such scenes came out up to 4.6e-4
+// from one call per view, where two runs of either differ by up to 9e-5.
+//
+// Bound: issue slots (forward 81%, backward with its albedo atomics waiting for
+// L2).  An iteration on 16 views of 512x512 took 339 us with the general walk,
+// a sum over the warp per value and float atomics for every sum; now 258.
+// Register caps: 6 blocks per SM (40 registers); backward with 5 269 us, with 7
+// 250, but 2% slower on one view of 1920x1080; forward with 5 2% slower.
+// GENERAL: long step limits, or a sun direction the forward walk does not take
+// (trace_fast).
 template <bool BWD, bool GENERAL>
-__global__ void __launch_bounds__(kAdjBlock, BWD ? 5 : 6) k_shade_views(const __grid_constant__ ViewsArgs va) {
+__global__ void __launch_bounds__(kAdjBlock, 6) k_shade_views(const __grid_constant__ ViewsArgs va) {
     const AdjArgs& a = va.a;
     const ViewP& V = va.v[blockIdx.z];
     __shared__ float s_gpal[BWD ? 768 : 1], s_acc[4];   // palette gradient; loss and sun
-    __shared__ float s_col[16 * kMaxTiles], s_row[16];  // ray UVs (shade.cuh, ray_u and ray_v)
-    const int x0 = (int)blockIdx.x * 16 * a.tiles, y0 = (int)blockIdx.y * 16;
+    __shared__ float s_col[16], s_row[16];              // ray UVs (shade.cuh, ray_u and ray_v)
+    const int x0 = (int)blockIdx.x * 16, y0 = (int)blockIdx.y * 16;
     if (x0 >= V.width || y0 >= V.height) return;  // the view is smaller
+    const int warp = threadIdx.x >> 5;
+    const unsigned lane = threadIdx.x & 31u;
+    const int lx = (warp & 1) * 8 + (int)(lane & 7u), ly = (warp >> 1) * 4 + (int)(lane >> 3);
+    const int px = x0 + lx, py = y0 + ly;
+    const bool inside = px < V.width && py < V.height;
+    const size_t p = inside ? (size_t)py * V.width + px : 0;
     if (BWD) {
         for (int i = threadIdx.x; i < 768; i += kAdjBlock) s_gpal[i] = 0.0f;
         if (threadIdx.x < 4) s_acc[threadIdx.x] = 0.0f;
     }
-    if (threadIdx.x < 16 * a.tiles) {
+    if (threadIdx.x < 16) {
         const float u = (((float)(x0 + (int)threadIdx.x) / (float)V.width) * 2.0f) - 1.0f;
         s_col[threadIdx.x] = u * V.tan_half_fov;
     } else if (threadIdx.x >= 128 && threadIdx.x < 144) {
@@ -121,117 +132,107 @@ __global__ void __launch_bounds__(kAdjBlock, BWD ? 5 : 6) k_shade_views(const __
         s_row[threadIdx.x - 128] = v * V.tan_half_fov;
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5;
-    const unsigned lane = threadIdx.x & 31u;
-    const int lx = (warp & 1) * 8 + (int)(lane & 7u), ly = (warp >> 1) * 4 + (int)(lane >> 3);
     float lossv = 0.0f, gsun[3] = {0.0f, 0.0f, 0.0f};
-    for (int tile = 0; tile < a.tiles; ++tile) {
-        const int px = x0 + 16 * tile + lx, py = y0 + ly;
-        if (x0 + 16 * tile >= V.width) break;
-        const bool inside = px < V.width && py < V.height;
-        const size_t p = inside ? (size_t)py * V.width + px : 0;
-        bool hit = false;
-        int m = 0;
-        unsigned v = 0;
-        float c[3] = {0.0f, 0.0f, 0.0f}, shade = 0.0f, albv = 1.0f, ndl_raw = 0.0f, nrm[3] = {0.0f, 0.0f, 0.0f};
-        bool lit = false;
-        if (inside) {
-            const uint4 rec = V.hits[p];
-            hit = ((rec.w >> 16) & VT_HIT_PRIMARY) != 0;
-            if (hit) {
-                v = rec.x;
-                const float t = __uint_as_float(rec.y);
-                const unsigned face = rec.w & 0xFFu;
-                m = (int)((rec.w >> 8) & 0xFFu);
-                const int axis = (int)(face >> 1);
-                const bool pos = (face & 1u) == 0u;
-                // the primary ray (primary_ray_uv) and the shadow origin
-                const float u = s_col[16 * tile + lx], w = s_row[ly];
-                float q[3], so[3];
-#pragma unroll
-                for (int j = 0; j < 3; ++j) q[j] = ((u * V.view[j] + w * V.view[4 + j]) + V.view[8 + j]) + V.view[12 + j];
-                const float len = __fsqrt_rn((q[0] * q[0] + q[1] * q[1]) + q[2] * q[2]);
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    float d = __fdiv_rn(q[j], len);
-                    if (d == 0.0f) d = 0.001f;   // map.glsl:85-90
-                    nrm[j] = (j == axis) ? (pos ? -1.0f : 1.0f) : 0.0f;
-                    so[j] = __fmaf_rn(d, t, V.pos[j]);
-                    if (j == axis) so[j] = so[j] + nrm[j] * 0.001f;
-                }
-                if (a.vis_in) {
-                    lit = a.vis_in[p] != 0;
-                } else {
-                    bool blocked;
-                    if (GENERAL) {
-                        PRay rs;
-                        pray_init_dir(rs, so, a.sun.d, a.sun.inv);
-                        TraceHit hs;
-                        blocked = trace_fast<false, true, true>(a.w, a.w.cdist, rs, a.shadow_steps, hs);
-                    } else {
-                        blocked = trace_sun<false>(a.w, a.sun, so, a.shadow_steps);
-                    }
-                    lit = !blocked &&
-                          !(a.w.n_entities > 0 && entity_occluded(a.w, so, a.sun_raw));
-                }
-                ndl_raw = dot3(nrm, a.sun_n);
-                const float ndl = ndl_raw > 0.0f ? ndl_raw : 0.0f;
-                shade = a.ka + a.kd * ndl * (lit ? 1.0f : 0.0f);
-                albv = a.alb ? __ldg(a.alb + v) : 1.0f;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) c[k] = (__ldg(a.pal + 3 * m + k) * albv) * shade;
-            }
-        }
-        if (!BWD) {
-            if (inside) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) V.rgb[3 * p + k] = c[k];
-                if (a.vis_out) a.vis_out[p] = (unsigned char)(hit && lit ? 1 : 0);
-            }
-            continue;
-        }
-
-        // ---- loss and gradients
-        float g[3] = {0.0f, 0.0f, 0.0f};
-        if (inside) {
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float diff = c[k] - __ldg(V.target + 3 * p + k);
-                g[k] = 2.0f * diff;
-                lossv += diff * diff;
-            }
-        }
-        float gp[3] = {0.0f, 0.0f, 0.0f};
+    bool hit = false;
+    int m = 0;
+    unsigned v = 0;
+    float c[3] = {0.0f, 0.0f, 0.0f}, shade = 0.0f, albv = 1.0f, ndl_raw = 0.0f, nrm[3] = {0.0f, 0.0f, 0.0f};
+    bool lit = false;
+    if (inside) {
+        const uint4 rec = V.hits[p];
+        hit = ((rec.w >> 16) & VT_HIT_PRIMARY) != 0;
         if (hit) {
-            float ga = 0.0f, gb = 0.0f;
+            v = rec.x;
+            const float t = __uint_as_float(rec.y);
+            const unsigned face = rec.w & 0xFFu;
+            m = (int)((rec.w >> 8) & 0xFFu);
+            const int axis = (int)(face >> 1);
+            const bool pos = (face & 1u) == 0u;
+            // the primary ray (primary_ray_uv) and the shadow origin
+            const float u = s_col[lx], w = s_row[ly];
+            float q[3], so[3];
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float pk = __ldg(a.pal + 3 * m + k);
-                gp[k] = g[k] * albv * shade;
-                ga += g[k] * pk * shade;
-                gb += g[k] * pk * albv;
-            }
-            if (lit && ndl_raw > 0.0f) {
-                const float coef = gb * a.kd * a.inv_len;
+            for (int j = 0; j < 3; ++j) q[j] = ((u * V.view[j] + w * V.view[4 + j]) + V.view[8 + j]) + V.view[12 + j];
+            const float len = __fsqrt_rn((q[0] * q[0] + q[1] * q[1]) + q[2] * q[2]);
 #pragma unroll
-                for (int k = 0; k < 3; ++k) gsun[k] += coef * (nrm[k] - ndl_raw * a.sun_n[k]);
+            for (int j = 0; j < 3; ++j) {
+                float d = __fdiv_rn(q[j], len);
+                if (d == 0.0f) d = 0.001f;   // map.glsl:85-90
+                nrm[j] = (j == axis) ? (pos ? -1.0f : 1.0f) : 0.0f;
+                so[j] = __fmaf_rn(d, t, V.pos[j]);
+                if (j == axis) so[j] = so[j] + nrm[j] * 0.001f;
             }
-            // albedo: one global atomic per hit pixel (voxels differ across
-            // most of a warp; the L2 absorbs the few repeats)
-            if (a.galb) atomicAdd(a.galb + v, ga);
-        }
-        // palette: one shared-memory atomic per (warp, material, channel).
-        // The warp walks its distinct materials (few per warp), no divergence.
-        unsigned todo = __ballot_sync(0xFFFFFFFFu, hit);
-        while (todo) {
-            const int key = __shfl_sync(0xFFFFFFFFu, m, __ffs(todo) - 1);
-            const bool mine = hit && m == key;
-            todo &= ~__ballot_sync(0xFFFFFFFFu, mine);
-            const float s = warp_sum4(lane, mine ? gp[0] : 0.0f, mine ? gp[1] : 0.0f, mine ? gp[2] : 0.0f, 0.0f);
-            if ((lane & 7u) == 0u && lane < 24u) atomicAdd(s_gpal + 3 * key + (lane >> 3), s);
+            if (a.vis_in) {
+                lit = a.vis_in[p] != 0;
+            } else {
+                bool blocked;
+                if (GENERAL) {
+                    PRay rs;
+                    pray_init_dir(rs, so, a.sun.d, a.sun.inv);
+                    TraceHit hs;
+                    blocked = trace_fast<false, true, true>(a.w, a.w.cdist, rs, a.shadow_steps, hs);
+                } else {
+                    blocked = trace_sun<false>(a.w, a.sun, so, a.shadow_steps);
+                }
+                lit = !blocked &&
+                      !(a.w.n_entities > 0 && entity_occluded(a.w, so, a.sun_raw));
+            }
+            ndl_raw = dot3(nrm, a.sun_n);
+            const float ndl = ndl_raw > 0.0f ? ndl_raw : 0.0f;
+            shade = a.ka + a.kd * ndl * (lit ? 1.0f : 0.0f);
+            albv = a.alb ? __ldg(a.alb + v) : 1.0f;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) c[k] = (__ldg(a.pal + 3 * m + k) * albv) * shade;
         }
     }
-    if (!BWD) return;
+    if (!BWD) {
+        if (inside) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) V.rgb[3 * p + k] = c[k];
+            if (a.vis_out) a.vis_out[p] = (unsigned char)(hit && lit ? 1 : 0);
+        }
+        return;
+    }
+
+    // ---- loss and gradients
+    float g[3] = {0.0f, 0.0f, 0.0f};
+    if (inside) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float diff = c[k] - __ldg(V.target + 3 * p + k);
+            g[k] = 2.0f * diff;
+            lossv += diff * diff;
+        }
+    }
+    float gp[3] = {0.0f, 0.0f, 0.0f};
+    if (hit) {
+        float ga = 0.0f, gb = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float pk = __ldg(a.pal + 3 * m + k);
+            gp[k] = g[k] * albv * shade;
+            ga += g[k] * pk * shade;
+            gb += g[k] * pk * albv;
+        }
+        if (lit && ndl_raw > 0.0f) {
+            const float coef = gb * a.kd * a.inv_len;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) gsun[k] += coef * (nrm[k] - ndl_raw * a.sun_n[k]);
+        }
+        // albedo: one global atomic per hit pixel (voxels differ across
+        // most of a warp; the L2 absorbs the few repeats)
+        if (a.galb) atomicAdd(a.galb + v, ga);
+    }
+    // palette: one shared-memory atomic per (warp, material, channel).
+    // The warp walks its distinct materials (few per warp), no divergence.
+    unsigned todo = __ballot_sync(0xFFFFFFFFu, hit);
+    while (todo) {
+        const int key = __shfl_sync(0xFFFFFFFFu, m, __ffs(todo) - 1);
+        const bool mine = hit && m == key;
+        todo &= ~__ballot_sync(0xFFFFFFFFu, mine);
+        const float s = warp_sum4(lane, mine ? gp[0] : 0.0f, mine ? gp[1] : 0.0f, mine ? gp[2] : 0.0f, 0.0f);
+        if ((lane & 7u) == 0u && lane < 24u) atomicAdd(s_gpal + 3 * key + (lane >> 3), s);
+    }
     {
         const float s = warp_sum4(lane, lossv, gsun[0], gsun[1], gsun[2]);
         if ((lane & 7u) == 0u) atomicAdd(s_acc + (lane >> 3), s);
@@ -334,7 +335,6 @@ vt_status launch_shade_views(vt_ctx* ctx, const vt_world* world, int32_t n, cons
     for (int v0 = 0; v0 < n && e == cudaSuccess; v0 += kMaxViews) {
         const int nv = n - v0 < kMaxViews ? n - v0 : kMaxViews;
         int gw = 0, gh = 0;
-        size_t tiles = 0;
         for (int i = 0; i < nv; ++i) {
             const vt_camera& c = cams[v0 + i];
             ViewP& V = va.v[i];
@@ -348,16 +348,9 @@ vt_status launch_shade_views(vt_ctx* ctx, const vt_world* world, int32_t n, cons
             V.rgb = bwd ? nullptr : d_rgb[v0 + i];
             gw = c.width > gw ? c.width : gw;
             gh = c.height > gh ? c.height : gh;
-            tiles += (size_t)((c.width + 15) / 16) * (size_t)((c.height + 15) / 16);
         }
-        // A backward block's clearing and flushing is shared by up to four
-        // tiles (16 views of 512x512: 1 tile 280 us an iteration, 2 and 4 256
-        // us; the forward kernel has nothing to share and is slower), as long
-        // as the launch keeps 24 blocks per SM, four waves.
-        a.tiles = 1;
-        while (bwd && a.tiles < kMaxTiles && tiles / (size_t)(2 * a.tiles) >= (size_t)(24 * ctx->sm_count)) a.tiles *= 2;
         va.a = a;
-        const dim3 grid((gw + 16 * a.tiles - 1) / (16 * a.tiles), (gh + 15) / 16, nv);
+        const dim3 grid((gw + 15) / 16, (gh + 15) / 16, nv);
         k<<<grid, kAdjBlock, 0, st>>>(va);
         e = cudaGetLastError();
     }
