@@ -1,0 +1,65 @@
+"""Every walk ends and reads inside its world, whatever the camera holds: the
+frame's pixel compiled as host C++ (host/walk_ends.cpp) under
+a limit of walk steps far above what any ray of these worlds takes, its world
+reads checked.  What the records say is compared with the unit-step oracle."""
+import ctypes as C
+import subprocess
+
+import numpy as np
+import pytest
+
+from test_host_trace import HERE, cuda_include, ht  # noqa: F401
+
+SRC = HERE / "host" / "walk_ends.cpp"
+OUT = HERE / "host" / "_build" / "libwalk_ends.so"
+DIMS = (64, 70, 61)
+LIMIT = 100000
+
+
+@pytest.fixture(scope="module")
+def we(ht):  # noqa: F811
+    deps = [SRC, HERE.parent / "include" / "vt.h"] + sorted((HERE.parent / "unnamed-voxel-tracer_gb300" / "csrc").glob("*.cuh")) + \
+        sorted((HERE.parent / "unnamed-voxel-tracer_gb300" / "csrc").glob("*.h"))
+    if not OUT.exists() or any(d.stat().st_mtime > OUT.stat().st_mtime for d in deps):
+        OUT.parent.mkdir(exist_ok=True)
+        subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fPIC", "-shared", "-I", cuda_include(),
+                        str(SRC), "-o", str(OUT)], check=True)
+    return C.CDLL(str(OUT))
+
+
+@pytest.fixture(scope="module")
+def world(ht, vtlib):  # noqa: F811
+    """Dims, voxels and distance fields of a small cave world."""
+    mats = vtlib.gen_world(vtlib.gen_desc(DIMS, scale=0.5, seed=7, trees=12, caves=True))
+    nch = int(np.prod([(d + 31) // 32 for d in DIMS]))
+    brick, chunk = np.zeros(8 * nch * 512, np.uint8), np.zeros(8 * nch, np.uint8)
+    dims = (C.c_int32 * 3)(*DIMS)
+    ht.ht_distances.argtypes = [C.POINTER(C.c_int32), C.c_void_p, C.c_void_p, C.c_void_p]
+    ht.ht_distances(dims, mats.ctypes.data, brick.ctypes.data, chunk.ctypes.data)
+    return dims, mats, brick, chunk
+
+
+@pytest.mark.parametrize("pos", [(30.5, 55.5, 30.5), (-40.0, 60.0, -30.0), (3e5, 2e5, 4e5)])
+@pytest.mark.parametrize("scale", [1.0, 1e-12, 1e-19, 1e-22, 3e-23, 1e-23, 1e-25, 1e-30, 1e-38, 1e-44, 0.0, 1e15, 1e19,
+                                   1e25, 1e38])
+def test_frames_of_scaled_views(we, oracle, vtlib, world, pos, scale):
+    """A view whose rows are so small (or large) that a direction's squared
+    length leaves the float range: components of the normalised direction are
+    infinite, NaN, or all zero (replaced by 0.001)."""
+    dims, mats, brick, chunk = world
+    W, H = 24, 17
+    cam = vtlib.Camera(pos=pos, yaw=0.7, pitch=-0.5, fov=1.3, width=W, height=H).as_uniform_data()
+    with np.errstate(over="ignore", under="ignore"):
+        view = (np.array(list(cam.view), np.float32) * np.float32(scale)).astype(np.float32)
+    cam.view = (C.c_float * 16)(*view)
+    out = np.zeros((H * W, 2), np.uint8)
+    we.we_frame.argtypes = [C.POINTER(C.c_int32)] + [C.c_void_p] * 5 + [C.c_float] + [C.c_int32] * 3 + [C.c_int64, C.c_void_p]
+    p = np.array(pos, np.float32)
+    we.we_frame(dims, mats.ctypes.data, brick.ctypes.data, chunk.ctypes.data, p.ctypes.data, view.ctypes.data,
+                cam.tan_half_fov, W, H, 512, LIMIT, out.ctypes.data)
+    assert np.all(out[:, 0] == 0), (np.bincount(out[:, 0]), "pixels that ended, did not end, read out of range")
+    params = vtlib.default_params(rays=vtlib.RAYS_PRIMARY, shade=vtlib.SHADE_NONE)
+    ref, _ = oracle.render(oracle.OracleWorld(mats), vtlib.default_palette(), cam, params, threads=4)
+    assert np.array_equal(out[:, 1], ref["flags"])
+    if scale == 1.0 and pos[0] == 30.5:
+        assert np.count_nonzero(out[:, 1]) > 100

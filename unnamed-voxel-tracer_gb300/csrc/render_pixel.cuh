@@ -68,7 +68,7 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
     TraceHit h;
     TraceCounters cnt;
     constexpr bool kForward = !STATS && !CHECKED && !SHARE;
-    const bool hit = kForward && (f.cam_inside || near_origin(r.o)) && ordinary_unit(r.inv)
+    const bool hit = kForward && (f.cam_inside || near_origin(r.o)) && ordinary_inv(r.inv)
                          ? trace_primary<LONG>(w, f, r, h)
                          : trace_any<STATS, CHECKED, true, false, SHARE, LONG>(w, coarse, cd, r, f.max_steps, h, cnt, status);
     if (STATS) {

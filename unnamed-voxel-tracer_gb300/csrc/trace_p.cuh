@@ -724,16 +724,14 @@ __device__ __forceinline__ float magic_brick(float n) {
 constexpr int kChunkSteps = 1024;
 
 // A ray the forward walk takes: near origin, and reciprocals in
-// [2^-100, 2^100] in magnitude (so no plane time overflows or is NaN).
+// [2^-100, 2^100] in magnitude (so no plane time overflows or is NaN, and every
+// plane is crossed later than the one before: with a reciprocal of 0, of an
+// infinite component, all plane times of an axis are one and a jump need not
+// move).  A normalised direction is tested too: it is infinite where its squared
+// length underflowed.
 __host__ __device__ __forceinline__ bool ordinary_inv(const float inv[3]) {
     const float a = fabsf(inv[0]), b = fabsf(inv[1]), c = fabsf(inv[2]);
     return a <= 0x1p100f && b <= 0x1p100f && c <= 0x1p100f && a >= 0x1p-100f && b >= 0x1p-100f && c >= 0x1p-100f;
-}
-
-// The same for a direction of length about 1, whose reciprocals are about 1 or
-// more.
-__device__ __forceinline__ bool ordinary_unit(const float inv[3]) {
-    return fabsf(inv[0]) <= 0x1p100f && fabsf(inv[1]) <= 0x1p100f && fabsf(inv[2]) <= 0x1p100f;
 }
 
 struct FwdWalk {
