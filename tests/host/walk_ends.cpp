@@ -1,7 +1,7 @@
-// Test-only: the frame's pixel (render_pixel.cuh) compiled as host C++, run
-// under a limit of walk steps and with every world read checked against its
-// array, so that a walk that would not end, or would read outside its world, is
-// found without a GPU.
+// Test-only: the frame's pixel (render_pixel.cuh) and the shadow walk
+// (trace_p.cuh) compiled as host C++, each run under a limit of walk steps and
+// with every world read checked against its array, so that a walk that would
+// not end, or would read outside its world, is found without a GPU.
 #include <math.h>
 #include <stdint.h>
 #include <string.h>
@@ -119,6 +119,30 @@ struct HostWorld {
     }
 };
 
+// Sun fields of the shadow walk (as sun_walk makes them for a frame).
+vt::SunWalk sun_fields(const float sun[3], const vt::WorldView& w) {
+    vt::SunWalk s;
+    unsigned oct = 0;
+    s.flip = 0;
+    for (int j = 0; j < 3; ++j) {
+        const float d = sun[j] == 0.0f ? 0.001f : sun[j];
+        const bool up = d > 0.0f;
+        s.d[j] = d;
+        s.inv[j] = 1.0f / d;
+        s.m[j] = up ? 0 : -1;
+        s.side[j] = up ? 1.0f : -1.0f;
+        s.off[j] = up ? 1.0f : 0.0f;
+        s.ad[j] = fabsf(d);
+        s.ai[j] = fabsf(s.inv[j]);
+        s.exit[j] = up ? (float)w.dims[j] : 0.0f;
+        s.in_hi[j] = (float)(w.dims[j] - 1);
+        if (up) oct |= 1u << j;
+        else s.flip |= 3u << (2 * j);
+    }
+    s.field = oct * w.nwords;
+    return s;
+}
+
 }  // namespace
 
 enum { kEnded = 0, kEndless = 1, kOutOfRange = 2 };
@@ -163,4 +187,42 @@ extern "C" void we_frame(const int32_t dims[3], const uint8_t* dense, const uint
                 o[0] = (uint8_t)fault_of(e);
             }
         }
+}
+
+// Shadow rays from n start points: per point {how the shading kernels' walk
+// ended, whether it is blocked, the same of trace_fast, the same of the general
+// walk, which takes any origin}.
+extern "C" void we_shadow(const int32_t dims[3], const uint8_t* dense, const uint8_t* brick, const uint8_t* chunk,
+                          const float sun[3], const float* origins, int64_t n, int32_t max_steps, int64_t limit,
+                          uint8_t* out) {
+    HostWorld hw(dims, dense, brick, chunk);
+    const vt::SunWalk s = sun_fields(sun, hw.w);
+    for (int64_t i = 0; i < n; ++i) {
+        const float* so = origins + 3 * i;
+        vt::PRay r;
+        vt::pray_init_dir(r, so, s.d, s.inv);
+        for (int k = 0; k < 3; ++k) {
+            uint8_t* o = out + 6 * i + 2 * k;
+            o[0] = kEnded;
+            o[1] = 0;
+            steps_left = limit;
+            vt::TraceHit h;
+            try {
+                if (k == 0) {
+                    o[1] = vt::trace_sun<false>(hw.w, s, so, max_steps);
+                } else if (k == 1) {
+                    o[1] = vt::trace_fast<false, true, true>(hw.w, hw.w.cdist, r, max_steps, h);
+                } else {
+                    vt::Walker wk;
+                    int st = vt::Walker::kMiss;
+                    if (wk.start_ray(hw.w, r, max_steps))
+                        while ((st = wk.step<false, true, true>(hw.w, hw.w.cdist, h)) == vt::Walker::kMore) {
+                        }
+                    o[1] = st == vt::Walker::kHit;
+                }
+            } catch (const WalkFault& e) {
+                o[0] = (uint8_t)fault_of(e);
+            }
+        }
+    }
 }

@@ -1,5 +1,5 @@
-"""Every walk ends and reads inside its world, whatever the camera holds: the
-frame's pixel compiled as host C++ (host/walk_ends.cpp) under
+"""Every walk ends and reads inside its world, whatever the camera or the hit
+records hold: the frame's pixel compiled as host C++ (host/walk_ends.cpp) under
 a limit of walk steps far above what any ray of these worlds takes, its world
 reads checked.  What the records say is compared with the unit-step oracle."""
 import ctypes as C
@@ -63,3 +63,31 @@ def test_frames_of_scaled_views(we, oracle, vtlib, world, pos, scale):
     assert np.array_equal(out[:, 1], ref["flags"])
     if scale == 1.0 and pos[0] == 30.5:
         assert np.count_nonzero(out[:, 1]) > 100
+
+
+@pytest.mark.parametrize("sun", [(0.6, 0.5, 0.3), (-0.6, -0.5, -0.3), (0.3, -0.9, 0.0), (-1e12, 2e12, 5e11)])
+def test_shadow_rays_from_any_point(we, world, sun):
+    """Points the shading kernels make from hit records that no frame of this
+    world wrote (any t): far away on the line into the world, infinite, NaN."""
+    dims, mats, brick, chunk = world
+    rng = np.random.default_rng(3)
+    n = 20000
+    d = np.array(sun, np.float64)
+    d[d == 0] = 0.001
+    d /= np.linalg.norm(d)
+    inside = rng.uniform([0, 0, 0], DIMS, (n, 3))
+    back = np.where(rng.random(n) < 0.2, 0.0, 2.0 ** rng.uniform(-3, 40, n))
+    o = (inside - d * back[:, None]).astype(np.float32)
+    o[::50, 0] = np.inf
+    o[1::50, 1] = -np.inf
+    o[2::50] = np.nan
+    o[3::50, 2] = np.float32(3e38)
+    o[4::50] = np.sign(-d).astype(np.float32) * np.float32(1e30)
+    s = np.array(sun, np.float32)
+    out = np.zeros((n, 3, 2), np.uint8)
+    we.we_shadow.argtypes = [C.POINTER(C.c_int32)] + [C.c_void_p] * 5 + [C.c_int64, C.c_int32, C.c_int64, C.c_void_p]
+    we.we_shadow(dims, mats.ctypes.data, brick.ctypes.data, chunk.ctypes.data, s.ctypes.data, o.ctypes.data, n, 512,
+                 LIMIT, out.ctypes.data)
+    assert np.all(out[:, :, 0] == 0), [np.bincount(out[:, k, 0]) for k in range(3)]
+    assert np.array_equal(out[:, 0, 1], out[:, 2, 1]) and np.array_equal(out[:, 1, 1], out[:, 2, 1])
+    assert 1000 < np.count_nonzero(out[:, 2, 1]) < n - 1000

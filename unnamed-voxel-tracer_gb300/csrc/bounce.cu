@@ -36,15 +36,15 @@ struct Walk<true, LONG> {
     }
 };
 
-// The forward walk; a ray it does not take (a reciprocal out of its range) is
-// traced to its end by Walker at the start.
+// The forward walk; a ray it does not take (a reciprocal out of its range, a far
+// origin) is traced to its end by Walker at the start.
 template <bool LONG>
 struct Walk<false, LONG> {
     FwdWalk fw;
     __device__ __forceinline__ int start(const WorldView& w, const float o[3], const float d[3], int steps) {
         PRay r;
         pray_init(r, o, d);
-        if (ordinary_inv(r.inv)) return fw.start(w, r, steps) ? Walker::kMore : Walker::kMiss;
+        if (ordinary_inv(r.inv) && near_origin(o)) return fw.start(w, r, steps) ? Walker::kMore : Walker::kMiss;
         TraceHit h;
         return trace_fast<false, true, true>(w, w.cdist, r, steps, h) ? Walker::kHit : Walker::kMiss;
     }

@@ -724,11 +724,15 @@ __device__ __forceinline__ float magic_brick(float n) {
 constexpr int kChunkSteps = 1024;
 
 // A ray the forward walk takes: near origin, and reciprocals in
-// [2^-100, 2^100] in magnitude (so no plane time overflows or is NaN, and every
-// plane is crossed later than the one before: with a reciprocal of 0, of an
-// infinite component, all plane times of an axis are one and a jump need not
-// move).  A normalised direction is tested too: it is infinite where its squared
-// length underflowed.
+// [2^-100, 2^100] in magnitude, so no plane time overflows or is NaN.  For such a
+// ray every step moves on and stays in the grid's padded box: in an occupied
+// brick it crosses planes one by one up to the brick's far face; a jump ends at
+// the time of its exit plane K, where the position is within 3/16 of a cell of
+// K, so that plane K is the last one crossed on that axis (step).  With a far
+// origin the position is not that exact, and with a reciprocal of 0 (an infinite
+// component) all plane times of an axis are one: a jump may then stay where it is
+// or end anywhere.  So every caller tests both, a normalised direction too: it is
+// infinite where its squared length underflowed.
 __host__ __device__ __forceinline__ bool ordinary_inv(const float inv[3]) {
     const float a = fabsf(inv[0]), b = fabsf(inv[1]), c = fabsf(inv[2]);
     return a <= 0x1p100f && b <= 0x1p100f && c <= 0x1p100f && a >= 0x1p-100f && b >= 0x1p-100f && c >= 0x1p-100f;
@@ -938,9 +942,25 @@ __device__ __forceinline__ bool trace_ordinary(const WorldView& w, const PRay& r
     return fw.start(w, r, max_steps) && fw.finish<MAT, LONG>(w, r, h);
 }
 
+// Walker to the ray's end.
+template <bool MAT, bool RUN, bool NEAR, bool SHARE>
+__device__ __forceinline__ bool walk_general(const WorldView& w, const unsigned char* cdist, const PRay& r, int max_steps,
+                                             TraceHit& h) {
+    int s;
+    Walker wk;
+    if (!wk.start_ray(w, r, max_steps)) return false;
+    while ((s = wk.step<MAT, RUN, NEAR, SHARE>(w, cdist, h)) == Walker::kMore) {
+    }
+    return s == Walker::kHit;
+}
+
 // Whether the shadow ray from so is blocked (a sun that passes ordinary_inv):
 // the fields of its walk that depend on the sun alone are given, and an origin
-// at least one cell inside the grid starts in its own cell (pray_start).
+// at least one cell inside the grid starts in its own cell (pray_start).  so may be
+// anywhere, or not a number, where it comes from a caller's hit records or a
+// camera at 2^40; Walker takes such a ray, as it takes any (the test and its code
+// cost 0.3% of a 4K frame with bounce rays, nothing measurable elsewhere; a call
+// out of line 5%).
 template <bool LONG>
 __device__ __forceinline__ bool trace_sun(const WorldView& w, const SunWalk& sun, const float so[3], int max_steps) {
     PRay r;
@@ -968,25 +988,24 @@ __device__ __forceinline__ bool trace_sun(const WorldView& w, const SunWalk& sun
         fw.limit = ((fw.nk[0] + fw.nk[1]) + fw.nk[2]) + __int2float_rn(min(max_steps, 1 << 20));
         fw.flip = sun.flip;
         fw.field = sun.field;
-    } else {
+    } else if (near_origin(so)) {
         go = fw.start(w, r, max_steps);
+    } else {
+        return walk_general<false, true, true, false>(w, w.cdist, r, max_steps, h);
     }
     return go && fw.finish<false, LONG>(w, r, h);
 }
 
-// Traces one ray to its end.  NEAR: the origin passes near_origin; SHARE:
-// brick words shared between the lanes of a warp (Walker only); LONG: step
-// limits above kChunkSteps (chunk jumps; without them only speed is lost).
+// Traces one ray to its end: by the forward walk if it is one that walk takes.
+// NEAR: the origin passes near_origin, or a plane search off by more than one
+// cell will do; SHARE: brick words shared between the lanes of a warp (Walker
+// only); LONG: step limits above kChunkSteps (chunk jumps; without them only
+// speed is lost).
 template <bool MAT, bool RUN = true, bool NEAR = false, bool SHARE = false, bool LONG = true>
 __device__ __forceinline__ bool trace_fast(const WorldView& w, const unsigned char* cdist, const PRay& r,
                                            int max_steps, TraceHit& h) {
-    if (NEAR && RUN && !SHARE && ordinary_inv(r.inv)) return trace_ordinary<MAT, LONG>(w, r, max_steps, h);
-    int s;
-    Walker wk;
-    if (!wk.start_ray(w, r, max_steps)) return false;
-    while ((s = wk.step<MAT, RUN, NEAR, SHARE>(w, cdist, h)) == Walker::kMore) {
-    }
-    return s == Walker::kHit;
+    if (NEAR && RUN && !SHARE && ordinary_inv(r.inv) && near_origin(r.o)) return trace_ordinary<MAT, LONG>(w, r, max_steps, h);
+    return walk_general<MAT, RUN, NEAR, SHARE>(w, cdist, r, max_steps, h);
 }
 
 }  // namespace vt
