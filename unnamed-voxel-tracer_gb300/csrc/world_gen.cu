@@ -107,12 +107,15 @@ __global__ void __launch_bounds__(512) k_gen_chunks(WorldView w, unsigned long l
 // The same world now takes 71 us.
 //
 // Error of the 32-bit values against the real ones, u = 2^-24: a lattice value
-// is in [-1, 1) (rounding u / 2); a weight, exact to 2^-28 before its one
-// rounding, is off by at most 0.6 u; an interpolation a + (b - a) t adds 1.2 u
-// for the weight and 1.5 u for its roundings.  Two levels: 6 u; the octaves'
-// sum (below 2) adds at most u an octave before the division by the
-// amplitudes' sum and 2 u in it; three levels: 8.6 u, times 1.5 for the two
-// octaves' sum, and 2 u more.  (The 64-bit values' own error is below 1e-14.)
+// is in [-1, 1) (rounding u / 2); a position is off by at most 2^-28
+// (lattice_coord), a weight, whose slope is at most 1.5, by 0.14 u before its one
+// rounding and 0.64 u in all; an interpolation a + (b - a) t adds 1.28 u for the
+// weight and 1.5 u for its roundings.  Two levels: 6.1 u; the octaves' sum (below
+// 2) adds at most u an octave after the first, the division by the amplitudes'
+// sum 1.5 u: below 8 u and u an octave.  Three levels: 8.9 u, times 1.5 for the
+// two octaves' sum, and 1 u in it: 14.4 u.  Largest found near coordinate 8191,
+// 9 million values: caves 4.9 u, heights 4.6 u.  (The 64-bit values' own error is
+// below 1e-14.)
 constexpr float kUlp = 0x1p-24f, kCaveError = 16.0f * kUlp;
 
 // gen::lattice rounded to 32 bits: the hash as a signed fraction.
@@ -124,8 +127,9 @@ __device__ __forceinline__ float lattice32(uint64_t seed, int x, int y, int z) {
 }
 
 // Lattice cell and interpolation weight of coordinate g (below 2^13) at a
-// frequency (below 2^2) held as a multiple of 2^-40: the position is exact to
-// 2^-28, and the noise is continuous across the cells.
+// frequency (below 2^2) rounded to a multiple of 2^-40 (fixed40): the position is
+// off by at most 2^13 * 2^-41 = 2^-28, and the noise is continuous across the
+// cells.
 __device__ __forceinline__ void lattice_coord(int g, long long f, int& cell, float& weight) {
     const long long x = (long long)g * f;
     const unsigned t = (unsigned)((unsigned long long)x >> 8);   // the position in the cell, times 2^32
@@ -139,7 +143,8 @@ __device__ __forceinline__ float lerp32(float a, float b, float t) { return __fm
 struct GenArgs {
     vt_gen_desc d;
     double cave_freq;            // 1 / cave_period
-    long long freq40, cave40;    // the frequencies, multiples of 2^-40
+    long long height40[16];      // the octaves' frequencies, multiples of 2^-40; [0] 0: heights in 64 bits
+    long long cave40[2];
     uint64_t terrain_seed, cave_seed, leaf_seed;
     float norm;                  // 1 / (sum of the octaves' amplitudes)
     float fbm_error;             // of the 32-bit fbm2
@@ -147,9 +152,8 @@ struct GenArgs {
     int water;
     // shared-memory layout of k_gen_tiles, in floats
     int height_side[16];         // most lattice points a chunk meets on an axis, per octave
-    int height_floats;
     int cave_side[2];
-    int cave_floats, cave_rows;  // lattice values; rows interpolated along x (32 values each)
+    int cave_floats;             // lattice values; the rows interpolated along x follow them
 };
 
 // The 64-bit decisions, out of line: inlined they cost the kernels registers
@@ -173,20 +177,18 @@ __device__ __forceinline__ int height_of(const GenArgs& a, float fbm, int x, int
 
 // gen::height_at of one column without tables.
 __device__ int height_at32(const GenArgs& a, int x, int z) {
-    if (!a.freq40) return height_exact(&a.d, x, z);
-    long long f = a.freq40;
+    if (!a.height40[0]) return height_exact(&a.d, x, z);
     float sum = 0.0f, amp = 1.0f;
     for (int o = 0; o < a.d.octaves; ++o) {
         int cx, cz;
         float sx, sz;
-        lattice_coord(x, f, cx, sx);
-        lattice_coord(z, f, cz, sz);
+        lattice_coord(x, a.height40[o], cx, sx);
+        lattice_coord(z, a.height40[o], cz, sz);
         const uint64_t seed = a.terrain_seed + (uint64_t)o * gen::kOctaveSalt;
         const float p = lerp32(lattice32(seed, cx, 0, cz), lattice32(seed, cx + 1, 0, cz), sx);
         const float q = lerp32(lattice32(seed, cx, 0, cz + 1), lattice32(seed, cx + 1, 0, cz + 1), sx);
         sum += amp * lerp32(p, q, sz);
         amp *= 0.5f;
-        f *= 2;
     }
     return height_of(a, sum * a.norm, x, z);
 }
@@ -230,7 +232,7 @@ __global__ void __launch_bounds__(512, 2) k_gen_tiles(WorldView w, unsigned long
         const int o = i >> 6, axis = (i >> 5) & 1, k = i & 31, g0 = (axis ? cz : cx) * 32;
         int c;
         float s;
-        lattice_coord(g0 + k, a.freq40 << o, c, s);
+        lattice_coord(g0 + k, a.height40[o], c, s);
         const int c0 = __shfl_sync(0xFFFFFFFFu, c, 0);   // k is the lane
         weight[o][axis][k] = s;
         cell[o][axis][k] = (unsigned char)(c - c0);
@@ -271,7 +273,7 @@ __global__ void __launch_bounds__(512, 2) k_gen_tiles(WorldView w, unsigned long
             const int o = i / 96, axis = (i % 96) >> 5, k = i & 31, g0 = (axis == 0 ? cx : (axis == 1 ? cy : cz)) * 32;
             int c;
             float s;
-            lattice_coord(g0 + k, a.cave40 << o, c, s);
+            lattice_coord(g0 + k, a.cave40[o], c, s);
             const int c0 = __shfl_sync(0xFFFFFFFFu, c, 0);
             weight[o * 3 + axis][0][k] = s;
             cell[o * 3 + axis][0][k] = (unsigned char)(c - c0);
@@ -458,28 +460,27 @@ int gen_args(const vt_gen_desc& d, GenArgs& a) {
     // 32 coordinates at frequency f meet at most floor(31 f) + 2 cells, one
     // more lattice points
     auto side = [](long long f40) { return (double)((31 * f40) >> 40) + 3.0; };
+    auto fixed40 = [](double f, int octave) { return llrint(f * (double)(1 << octave) * 0x1p40); };
     const double finest = freq * (double)(1 << (d.octaves - 1));
     if (!(finest < 2.0)) return 0;
-    a.freq40 = (long long)(freq * 0x1p40);
+    for (int o = 0; o < d.octaves; ++o) a.height40[o] = fixed40(freq, o);
     if (d.caves && !(a.cave_freq < 1.0)) return 0;
-    a.cave40 = d.caves ? (long long)(a.cave_freq * 0x1p40) : 0;
+    for (int o = 0; o < 2 && d.caves; ++o) a.cave40[o] = fixed40(a.cave_freq, o);
     double heights = 0.0, caves = 0.0, rows = 0.0;
     for (int o = 0; o < d.octaves; ++o) {
-        const double n = side(a.freq40 << o);
+        const double n = side(a.height40[o]);
         a.height_side[o] = (int)n;
         heights += n * n;
     }
     for (int o = 0; o < 2 && d.caves; ++o) {
-        const double n = side(a.cave40 << o);
+        const double n = side(a.cave40[o]);
         a.cave_side[o] = (int)n;
         caves += n * n * n;
         rows += n * n;
     }
     const double floats = heights > caves + 3.0 + 32.0 * rows ? heights : caves + 3.0 + 32.0 * rows;
     if (4.0 * floats > (double)kGenSmem) return 0;
-    a.height_floats = (int)heights;
     a.cave_floats = ((int)caves + 3) / 4 * 4;
-    a.cave_rows = (int)rows;
     return (int)floats * 4;
 }
 
