@@ -602,13 +602,24 @@ vt_status vt_render_host(vt_ctx* ctx, const vt_world* world, const vt_camera* ca
     // Pinned host memory is mapped into the device's address space: the
     // kernel stores the records straight into it over the host link, with no
     // staging copy (1080p: 244 us per frame end to end against 288 us for the
-    // band pipeline below, kernel alone 210 us).
+    // band pipeline below, kernel alone 210 us).  The deferred bounce pass
+    // rewrites 5 bytes of the pixels whose ray leaves, in an order of its own,
+    // which over the link costs more than the copy of the whole frame: such
+    // frames are rendered in device memory and copied (1080p cave frame 456 us
+    // against 636).
     {
         cudaPointerAttributes pa;
         if (cudaPointerGetAttributes(&pa, h_out) == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer) {
-            s = launch_render(ctx, world, cam, params, reinterpret_cast<uint4*>(pa.devicePointer), ctx->stream, false,
-                              0, -1, true);
+            void* d_frame = nullptr;
+            if ((params->rays & VT_RAYS_BOUNCE) && (params->flags & VT_FLAG_CHECKED) == 0 &&
+                ctx->tuning.kernel != VT_KERNEL_QUEUE && ctx_scratch(ctx, bytes, &d_frame) != VT_OK) {
+                cudaGetLastError();   // no room for the staging frame: straight into the host's
+                d_frame = nullptr;
+            }
+            s = launch_render(ctx, world, cam, params, reinterpret_cast<uint4*>(d_frame ? d_frame : pa.devicePointer),
+                              ctx->stream, false, 0, -1, true);
             if (s) return s;
+            if (d_frame) VT_CUDA(ctx, cudaMemcpyAsync(h_out, d_frame, bytes, cudaMemcpyDeviceToHost, ctx->stream));
             return vt_sync(ctx, ctx->stream);
         }
         cudaGetLastError();  // a pageable pointer is not an error
