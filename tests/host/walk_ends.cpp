@@ -209,7 +209,7 @@ extern "C" void we_shadow(const int32_t dims[3], const uint8_t* dense, const uin
             vt::TraceHit h;
             try {
                 if (k == 0) {
-                    o[1] = vt::trace_sun<false>(hw.w, s, so, max_steps);
+                    o[1] = vt::trace_sun(hw.w, s, so, max_steps);
                 } else if (k == 1) {
                     o[1] = vt::trace_fast<false, true, true>(hw.w, hw.w.cdist, r, max_steps, h);
                 } else {

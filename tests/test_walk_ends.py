@@ -27,16 +27,32 @@ def we(ht):  # noqa: F811
     return C.CDLL(str(OUT))
 
 
-@pytest.fixture(scope="module")
-def world(ht, vtlib):  # noqa: F811
-    """Dims, voxels and distance fields of a small cave world."""
-    mats = vtlib.gen_world(vtlib.gen_desc(DIMS, scale=0.5, seed=7, trees=12, caves=True))
-    nch = int(np.prod([(d + 31) // 32 for d in DIMS]))
+def with_distances(ht, mats):  # noqa: F811
+    """Dims, voxels and distance fields of a world."""
+    dims = mats.shape[::-1]
+    nch = int(np.prod([(d + 31) // 32 for d in dims]))
     brick, chunk = np.zeros(8 * nch * 512, np.uint8), np.zeros(8 * nch, np.uint8)
-    dims = (C.c_int32 * 3)(*DIMS)
+    dims = (C.c_int32 * 3)(*dims)
     ht.ht_distances.argtypes = [C.POINTER(C.c_int32), C.c_void_p, C.c_void_p, C.c_void_p]
     ht.ht_distances(dims, mats.ctypes.data, brick.ctypes.data, chunk.ctypes.data)
     return dims, mats, brick, chunk
+
+
+@pytest.fixture(scope="module")
+def world(ht, vtlib):  # noqa: F811
+    """A small cave world."""
+    return with_distances(ht, vtlib.gen_world(vtlib.gen_desc(DIMS, scale=0.5, seed=7, trees=12, caves=True)))
+
+
+def trace_frame(we, world, pos, view, tan_half_fov, W, H, max_steps, limit):
+    """Per pixel of a frame's primary rays {how the walk ended, the record's flags}."""
+    out = np.zeros((H * W, 2), np.uint8)
+    we.we_frame.argtypes = [C.POINTER(C.c_int32)] + [C.c_void_p] * 5 + [C.c_float] + [C.c_int32] * 3 + [C.c_int64, C.c_void_p]
+    p = np.array(pos, np.float32)
+    dims, mats, brick, chunk = world
+    we.we_frame(dims, mats.ctypes.data, brick.ctypes.data, chunk.ctypes.data, p.ctypes.data, view.ctypes.data,
+                tan_half_fov, W, H, max_steps, limit, out.ctypes.data)
+    return out
 
 
 @pytest.mark.parametrize("pos", [(30.5, 55.5, 30.5), (-40.0, 60.0, -30.0), (3e5, 2e5, 4e5)])
@@ -46,20 +62,15 @@ def test_frames_of_scaled_views(we, oracle, vtlib, world, pos, scale):
     """A view whose rows are so small (or large) that a direction's squared
     length leaves the float range: components of the normalised direction are
     infinite, NaN, or all zero (replaced by 0.001)."""
-    dims, mats, brick, chunk = world
     W, H = 24, 17
     cam = vtlib.Camera(pos=pos, yaw=0.7, pitch=-0.5, fov=1.3, width=W, height=H).as_uniform_data()
     with np.errstate(over="ignore", under="ignore"):
         view = (np.array(list(cam.view), np.float32) * np.float32(scale)).astype(np.float32)
     cam.view = (C.c_float * 16)(*view)
-    out = np.zeros((H * W, 2), np.uint8)
-    we.we_frame.argtypes = [C.POINTER(C.c_int32)] + [C.c_void_p] * 5 + [C.c_float] + [C.c_int32] * 3 + [C.c_int64, C.c_void_p]
-    p = np.array(pos, np.float32)
-    we.we_frame(dims, mats.ctypes.data, brick.ctypes.data, chunk.ctypes.data, p.ctypes.data, view.ctypes.data,
-                cam.tan_half_fov, W, H, 512, LIMIT, out.ctypes.data)
+    out = trace_frame(we, world, pos, view, cam.tan_half_fov, W, H, 512, LIMIT)
     assert np.all(out[:, 0] == 0), (np.bincount(out[:, 0]), "pixels that ended, did not end, read out of range")
     params = vtlib.default_params(rays=vtlib.RAYS_PRIMARY, shade=vtlib.SHADE_NONE)
-    ref, _ = oracle.render(oracle.OracleWorld(mats), vtlib.default_palette(), cam, params, threads=4)
+    ref, _ = oracle.render(oracle.OracleWorld(world[1]), vtlib.default_palette(), cam, params, threads=4)
     assert np.array_equal(out[:, 1], ref["flags"])
     if scale == 1.0 and pos[0] == 30.5:
         assert np.count_nonzero(out[:, 1]) > 100
@@ -91,3 +102,16 @@ def test_shadow_rays_from_any_point(we, world, sun):
     assert np.all(out[:, :, 0] == 0), [np.bincount(out[:, k, 0]) for k in range(3)]
     assert np.array_equal(out[:, 0, 1], out[:, 2, 1]) and np.array_equal(out[:, 1, 1], out[:, 2, 1])
     assert 1000 < np.count_nonzero(out[:, 2, 1]) < n - 1000
+
+
+@pytest.mark.parametrize("max_steps", [620, 1024, 1025])
+def test_open_space_takes_few_jumps(we, ht, vtlib, max_steps):  # noqa: F811
+    """Rays through 594 empty cells of a grid of 2 x 2 x 19 chunks: two jumps out
+    of boxes of empty chunks (nine of the brick distances' 66 cells), whatever
+    the step limit."""
+    open_world = with_distances(ht, np.zeros((600, 64, 64), np.uint8))
+    pos = (32.5, 32.5, 5.5)
+    cam = vtlib.Camera(pos=pos, fov=0.05, width=8, height=8).as_uniform_data()
+    view = np.array(list(cam.view), np.float32)
+    out = trace_frame(we, open_world, pos, view, cam.tan_half_fov, 8, 8, max_steps, 3)
+    assert np.all(out == 0), np.bincount(out[:, 0])

@@ -84,7 +84,7 @@ static_assert(sizeof(JobChunk) <= 32764, "a kernel's parameters are limited to 3
 // One thread per pixel; the 128-thread block covers a 16 x 8 tile as four
 // 8 x 4 warp tiles (the single-frame kernel's default shape), with the same
 // register cap (36 warps per SM).
-template <bool CHECKED, bool BOUNCE, bool LONG>
+template <bool CHECKED, bool BOUNCE, bool ANYSUN>
 __global__ void __launch_bounds__(kTileBlock, 9) k_render_jobs(const __grid_constant__ JobChunk p, unsigned* status) {
     const unsigned b = blockIdx.x;
     int lo = 0, hi = p.njobs - 1;
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kTileBlock, 9) k_render_jobs(const __grid_cons
         uv.gv = s_row[2][ly];
     }
     PixelCounters pc;
-    const uint4 rec = render_pixel<false, CHECKED, CoarseGlobal, false, false, BOUNCE, LONG>(p.w, CoarseGlobal{p.w.coarse}, p.w.cdist, f, px, py, uv, status, pc);
+    const uint4 rec = render_pixel<false, CHECKED, CoarseGlobal, false, false, BOUNCE, ANYSUN>(p.w, CoarseGlobal{p.w.coarse}, p.w.cdist, f, px, py, uv, status, pc);
     p.cam[lo].out[(size_t)py * f.width + px] = rec;
 }
 
@@ -369,10 +369,10 @@ vt_status vt_batch_launch(vt_batch* b, vt_stream stream) {
                     for (const auto& pc : chain_plan(wt)) {
                         const JobChunk& ch = b->chunks[pc.first];
                         const unsigned blocks = ch.first_block[ch.njobs];
-                        const bool bounce = (b->params.rays & VT_RAYS_BOUNCE) != 0, lng = long_steps(ch.f);
+                        const bool bounce = (b->params.rays & VT_RAYS_BOUNCE) != 0, anysun = !ordinary_sun(ch.f);
                         auto k = checked ? k_render_jobs<true, true, true>
-                                 : bounce ? (lng ? k_render_jobs<false, true, true> : k_render_jobs<false, true, false>)
-                                          : (lng ? k_render_jobs<false, false, true> : k_render_jobs<false, false, false>);
+                                 : bounce ? (anysun ? k_render_jobs<false, true, true> : k_render_jobs<false, true, false>)
+                                          : (anysun ? k_render_jobs<false, false, true> : k_render_jobs<false, false, false>);
                         k<<<blocks, kTileBlock, 0, chain[pc.second]>>>(ch, checked ? ctx->d_status : nullptr);
                     }
                 } else {

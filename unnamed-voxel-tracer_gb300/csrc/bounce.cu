@@ -20,12 +20,12 @@ constexpr int kActions = 3;
 
 // The walk of one lane.  Both start a ray (kMore: under way; kHit or kMiss: it
 // is done already) and advance it by one step.
-template <bool FLAT, bool LONG>
+template <bool FLAT>
 struct Walk;
 
 // Walker::step_flat (one code path for jumps and unit steps).
-template <bool LONG>
-struct Walk<true, LONG> {
+template <>
+struct Walk<true> {
     Walker wk;
     __device__ __forceinline__ int start(const WorldView& w, const float o[3], const float d[3], int steps) {
         return wk.start(w, o, d, steps) ? Walker::kMore : Walker::kMiss;
@@ -38,8 +38,8 @@ struct Walk<true, LONG> {
 
 // The forward walk; a ray it does not take (a reciprocal out of its range, a far
 // origin) is traced to its end by Walker at the start.
-template <bool LONG>
-struct Walk<false, LONG> {
+template <>
+struct Walk<false> {
     FwdWalk fw;
     __device__ __forceinline__ int start(const WorldView& w, const float o[3], const float d[3], int steps) {
         PRay r;
@@ -50,7 +50,7 @@ struct Walk<false, LONG> {
     }
     __device__ __forceinline__ int step(const WorldView& w) {
         unsigned wi, vb;
-        return fw.template step<LONG>(w, wi, vb);
+        return fw.step(w, wi, vb);
     }
 };
 
@@ -72,7 +72,7 @@ __device__ __forceinline__ void open_pixel(uint4* out, unsigned pixel, unsigned 
 // memory for idle lanes to take (727 us: the copies cost more instructions
 // than the set-ups at few lanes), one code path for jumps and unit steps (568 us
 // here, but 11% slower on a 1021x577 frame whose queue is short).
-template <bool FLAT, bool LONG>
+template <bool FLAT>
 __global__ void __launch_bounds__(kBounceBlock, 4) k_bounce_trace(WorldView w, const BounceHead* __restrict__ heads,
                                                                const BounceTail* __restrict__ tails,
                                                                const unsigned* __restrict__ counters,
@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kBounceBlock, 4) k_bounce_trace(WorldView w, c
     const unsigned total = counters[0];
     const unsigned lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
-    Walk<FLAT, LONG> wk;
+    Walk<FLAT> wk;
     bool busy = false;
     unsigned job = 0;
     for (;;) {
@@ -134,21 +134,19 @@ vt_status bounce_buffers(vt_ctx* ctx, size_t pixels) {
 
 vt_status launch_bounce(vt_ctx* ctx, const vt_world* world, const FrameParams& f, uint4* d_out, cudaStream_t st) {
     const WorldView w = world->view();
-    const bool flat = ctx->tuning.bounce_walk == 1, lng = f.bounce_max_steps > kChunkSteps;
+    const int flat = ctx->tuning.bounce_walk == 1 ? 1 : 0;
     const int refill = ctx->tuning.bounce_refill > 0 ? ctx->tuning.bounce_refill : kRefill;
-    auto k = flat ? (lng ? k_bounce_trace<true, true> : k_bounce_trace<true, false>)
-                  : (lng ? k_bounce_trace<false, true> : k_bounce_trace<false, false>);
-    const int v = (flat ? 2 : 0) + (lng ? 1 : 0);
-    if (ctx->bounce_blocks[v] == 0) {
+    auto k = flat ? k_bounce_trace<true> : k_bounce_trace<false>;
+    if (ctx->bounce_blocks[flat] == 0) {
         int nb = 0;
         VT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, kBounceBlock, 0));
-        ctx->bounce_blocks[v] = ctx->sm_count * (nb > 0 ? nb : 1);
+        ctx->bounce_blocks[flat] = ctx->sm_count * (nb > 0 ? nb : 1);
     }
     cudaAccessPolicyWindow win_storage;
     const cudaAccessPolicyWindow* win = nullptr;  // L2 window over the brick words (tuning l2_persist)
     vt_status s = l2_policy(ctx, world, &win_storage, &win);
     if (s) return s;
-    VT_CUDA(ctx, launch_kernel(k, dim3(ctx->bounce_blocks[v]), dim3(kBounceBlock), 0, st, win, w,
+    VT_CUDA(ctx, launch_kernel(k, dim3(ctx->bounce_blocks[flat]), dim3(kBounceBlock), 0, st, win, w,
                                (const BounceHead*)ctx->d_bounce_head, (const BounceTail*)ctx->d_bounce_tail,
                                (const unsigned*)ctx->d_bounce_ctr, ctx->d_bounce_ctr + 1, d_out, f.bounce_max_steps,
                                refill));

@@ -55,7 +55,7 @@ struct BlockTile {
 // (Walker::brick_word).  BIN: deferred bounce rays are appended per block,
 // sorted by direction (stage_flush).
 template <bool STATS, bool CHECKED, bool SMEM, int TW, bool OCC, bool SHARE = false, bool BIN = false, bool BOUNCE = true,
-          bool LONG = true, int NB = kBlock>
+          bool ANYSUN = true, int NB = kBlock>
 __global__ void __launch_bounds__(NB, OCC ? (NB == kSmallBlock ? kSmallBlocks : kOccThreads / NB) : 1)
     k_render(const __grid_constant__ WorldView w, const __grid_constant__ FrameParams f, uint4* __restrict__ out,
              unsigned* status, unsigned long long* counters) {
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(NB, OCC ? (NB == kSmallBlock ? kSmallBlocks : 
         }
         uint4 rec;
         if (SMEM) rec = render_pixel<STATS, CHECKED>(w, CoarseShared{s_coarse}, w.cdist, f, px, py, uv, status, pc);
-        else rec = render_pixel<STATS, CHECKED, CoarseGlobal, SHARE, BIN, BOUNCE, LONG>(w, CoarseGlobal{w.coarse}, w.cdist, f, px,
+        else rec = render_pixel<STATS, CHECKED, CoarseGlobal, SHARE, BIN, BOUNCE, ANYSUN>(w, CoarseGlobal{w.coarse}, w.cdist, f, px,
                                                                           py, uv, status, pc);
         out[(size_t)py * f.width + px] = rec;
     }
@@ -117,7 +117,6 @@ __global__ void __launch_bounds__(NB, OCC ? (NB == kSmallBlock ? kSmallBlocks : 
 // 74.5 us in blocks of 256, 72.3 of 128, 71.6 of 64, 75.1 of 32; 64 with 16 to
 // 24 blocks per SM 70.7-72.7).  Lanes that take the next ray as theirs ends: 88 us.
 constexpr int kRayBlock = 64;
-template <bool LONG>
 __global__ void __launch_bounds__(kRayBlock, 16) k_trace_rays(const __grid_constant__ WorldView w, const float* __restrict__ origins,
                                                        const float* __restrict__ dirs, int n, int max_steps,
                                                        uint4* __restrict__ out) {
@@ -132,7 +131,7 @@ __global__ void __launch_bounds__(kRayBlock, 16) k_trace_rays(const __grid_const
     PRay r;
     pray_init(r, o, d);
     TraceHit h;
-    const bool hit = near_origin(r.o) ? trace_fast<true, true, true, false, LONG>(w, w.cdist, r, max_steps, h)
+    const bool hit = near_origin(r.o) ? trace_fast<true, true, true>(w, w.cdist, r, max_steps, h)
                                       : trace_fast<true, true, false>(w, w.cdist, r, max_steps, h);
     if (hit) {
         const int e = h.axis;
@@ -538,10 +537,10 @@ vt_status launch_render(vt_ctx* ctx, const vt_world* world, const vt_camera* cam
                                          dim3(kBlock), sm, stream, win, w, f, d_out, ctx->d_status, ctx->d_counters); }
         else if (tu.occupancy && tu.share_bricks) { VT_LAUNCH_X(false, false, false, 8, true, true); }
         else if (tu.occupancy) {
-            const bool bounce = (p->rays & VT_RAYS_BOUNCE) != 0, lng = long_steps(f);
-            auto k = bounce ? (lng ? k_render<false, false, false, 8, true, false, false, true, true>
+            const bool bounce = (p->rays & VT_RAYS_BOUNCE) != 0, anysun = !ordinary_sun(f);
+            auto k = bounce ? (anysun ? k_render<false, false, false, 8, true, false, false, true, true>
                                    : k_render<false, false, false, 8, true, false, false, true, false>)
-                            : (lng ? k_render<false, false, false, 8, true, false, false, false, true, kSmallBlock>
+                            : (anysun ? k_render<false, false, false, 8, true, false, false, false, true, kSmallBlock>
                                    : k_render<false, false, false, 8, true, false, false, false, false, kSmallBlock>);
             const int th = bounce ? BlockTile<8>::kH : BlockTile<8, kSmallBlock>::kH;
             le = launch_kernel(k, dim3((cam->width + BlockTile<8>::kW - 1) / BlockTile<8>::kW, (rows + th - 1) / th),
@@ -708,8 +707,7 @@ vt_status vt_trace_rays(vt_ctx* ctx, const vt_world* world, const float* d_origi
         if (s) return s;
     }
     const WorldView w = world->view();
-    (max_steps > kChunkSteps ? k_trace_rays<true> : k_trace_rays<false>)<<<(n + kRayBlock - 1) / kRayBlock, kRayBlock, 0,
-                                                                            (cudaStream_t)stream>>>(
+    k_trace_rays<<<(n + kRayBlock - 1) / kRayBlock, kRayBlock, 0, (cudaStream_t)stream>>>(
         w, d_origins, d_dirs, n, max_steps, reinterpret_cast<uint4*>(d_out));
     VT_CUDA(ctx, cudaGetLastError());
     return note_status_writer(ctx, (cudaStream_t)stream);

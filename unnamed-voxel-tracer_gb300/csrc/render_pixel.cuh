@@ -9,11 +9,8 @@
 
 namespace vt {
 
-// Whether some ray kind of the frame may walk far enough for chunk jumps to
-// pay, or the sun's direction is not one the forward walk takes.
-inline bool long_steps(const FrameParams& f) {
-    return f.max_steps > kChunkSteps || f.shadow_max_steps > kChunkSteps || f.bounce_max_steps > kChunkSteps || !ordinary_inv(f.sun_inv);
-}
+// Whether the sun's direction is one the forward walk takes.
+inline bool ordinary_sun(const FrameParams& f) { return ordinary_inv(f.sun_inv); }
 
 struct PixelCounters {
     unsigned v[kNumCounters];
@@ -25,18 +22,17 @@ struct PixelCounters {
 // NEAR: the caller knows the origin passes near_origin (secondary rays start
 // on a hit inside the grid); otherwise the primary ray checks it once.
 // SHARE: brick words shared between the lanes of a warp (Walker::brick_word).
-template <bool STATS, bool CHECKED, bool MAT, bool NEAR, bool SHARE, bool LONG, class Coarse>
+template <bool STATS, bool CHECKED, bool MAT, bool NEAR, bool SHARE, class Coarse>
 __device__ __forceinline__ bool trace_any(const WorldView& w, const Coarse& coarse, const unsigned char* cd,
                                           const PRay& r, int max_steps, TraceHit& h, TraceCounters& cnt,
                                           unsigned* status) {
     if (STATS || CHECKED) return trace_p<STATS, CHECKED, MAT>(w, coarse, r, max_steps, h, cnt, status);
-    if (NEAR || near_origin(r.o)) return trace_fast<MAT, true, true, SHARE, LONG>(w, cd, r, max_steps, h);
-    return trace_fast<MAT, true, false, SHARE, LONG>(w, cd, r, max_steps, h);
+    if (NEAR || near_origin(r.o)) return trace_fast<MAT, true, true, SHARE>(w, cd, r, max_steps, h);
+    return trace_fast<MAT, true, false, SHARE>(w, cd, r, max_steps, h);
 }
 
 // The primary ray of a frame whose camera is inside the grid: its cell is the
 // frame's (walk_constants).
-template <bool LONG>
 __device__ __forceinline__ bool trace_primary(const WorldView& w, const FrameParams& f, const PRay& r, TraceHit& h) {
     FwdWalk fw;
     bool go;
@@ -46,7 +42,7 @@ __device__ __forceinline__ bool trace_primary(const WorldView& w, const FramePar
     } else {
         go = fw.start(w, r, f.max_steps);
     }
-    return go && fw.finish<true, LONG>(w, r, h);
+    return go && fw.finish<true>(w, r, h);
 }
 
 // uv: the pixel's screen coordinates (pixel_uv(f, px, py); the frame kernel
@@ -54,10 +50,10 @@ __device__ __forceinline__ bool trace_primary(const WorldView& w, const FramePar
 // BIN: a deferred bounce ray is staged in the block's shared memory for the
 // block's direction-sorted append (stage_flush) instead of appended at once.
 // BOUNCE: false leaves the bounce rays' code out (frames without them: the
-// kernel's registers and code then serve the walk alone).  LONG: a ray kind's
-// step limit is above kChunkSteps (trace_fast).
+// kernel's registers and code then serve the walk alone).  ANYSUN: the sun may be
+// one the forward walk does not take (ordinary_sun).
 template <bool STATS, bool CHECKED, class Coarse, bool SHARE = false, bool BIN = false, bool BOUNCE = true,
-          bool LONG = true>
+          bool ANYSUN = true>
 __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& coarse, const unsigned char* cd,
                                               const FrameParams& f, int px, int py, const PixelUV& uv,
                                               unsigned* status, PixelCounters& pc) {
@@ -69,8 +65,8 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
     TraceCounters cnt;
     constexpr bool kForward = !STATS && !CHECKED && !SHARE;
     const bool hit = kForward && (f.cam_inside || near_origin(r.o)) && ordinary_inv(r.inv)
-                         ? trace_primary<LONG>(w, f, r, h)
-                         : trace_any<STATS, CHECKED, true, false, SHARE, LONG>(w, coarse, cd, r, f.max_steps, h, cnt, status);
+                         ? trace_primary(w, f, r, h)
+                         : trace_any<STATS, CHECKED, true, false, SHARE>(w, coarse, cd, r, f.max_steps, h, cnt, status);
     if (STATS) {
         pc.v[0] += 1;
         pc.v[9] += 16;
@@ -100,13 +96,13 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
         }
         bool shadowed = false;
         if (f.rays & VT_RAYS_SHADOW) {
-            if (kForward && (!LONG || ordinary_inv(f.sun_inv))) {
-                shadowed = trace_sun<LONG>(w, f.sunw, so, f.shadow_max_steps);
+            if (kForward && (!ANYSUN || ordinary_inv(f.sun_inv))) {
+                shadowed = trace_sun(w, f.sunw, so, f.shadow_max_steps);
             } else {
                 PRay rs;
                 pray_init_dir(rs, so, f.sun_d, f.sun_inv);
                 TraceHit hs;
-                shadowed = trace_any<STATS, CHECKED, false, true, SHARE, LONG>(w, coarse, cd, rs, f.shadow_max_steps, hs, cnt, status);
+                shadowed = trace_any<STATS, CHECKED, false, true, SHARE>(w, coarse, cd, rs, f.shadow_max_steps, hs, cnt, status);
             }
             if (shadowed) flags |= VT_HIT_SHADOWED;
             if (STATS) {
@@ -139,7 +135,7 @@ __device__ __forceinline__ uint4 render_pixel(const WorldView& w, const Coarse& 
             PRay rb;
             pray_init(rb, so, bdir);
             TraceHit hb;
-            const bool bh = trace_any<STATS, CHECKED, false, true, SHARE, LONG>(w, coarse, cd, rb, f.bounce_max_steps, hb, cnt, status);
+            const bool bh = trace_any<STATS, CHECKED, false, true, SHARE>(w, coarse, cd, rb, f.bounce_max_steps, hb, cnt, status);
             if (bh) flags |= VT_HIT_BOUNCE;
             bounce_open = !bh;
             if (STATS) {

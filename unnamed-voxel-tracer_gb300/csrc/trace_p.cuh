@@ -667,8 +667,7 @@ struct Walker {
 //     are the planes compared.  Inside a brick nothing is checked: cells past
 //     the grid's sides in a partly filled brick or chunk are empty;
 //   - the brick distance is read first (0: occupied, then the brick's word is
-//     read), and the chunk distance only for long step limits where the
-//     brick's is at its cap (kChunkSteps).
+//     read), and the chunk distance only where the brick's is at its cap.
 // Bound: compares, selects and integer logic share one half-rate pipe, which
 // bounds the frame kernel with the issue slots; adds and fused multiply-adds
 // do not use it, hence the arithmetic on magic floats.  1080p terrain frame,
@@ -697,6 +696,16 @@ __device__ __forceinline__ float bits_float(int i) {
     return x;
 #endif
 }
+// 32 u + 32 for a plane n = 32 u + 1 .. 32 u + 32: the far face of the next
+// plane's chunk, by a sum with 1.5 * 2^28 (spacing 32) rounded up.
+__device__ __forceinline__ float chunk_face(float n) {
+#ifdef __CUDA_ARCH__
+    constexpr float kMagic32 = 402653184.0f;
+    return __fadd_ru(n, kMagic32) - kMagic32;
+#else
+    return 32.0f * ceilf(n * 0.03125f);
+#endif
+}
 // kMagic + floor(p), |p| < 2^22: the sum rounded down.
 __device__ __forceinline__ float magic_floor(float p) {
 #ifdef __CUDA_ARCH__
@@ -714,14 +723,6 @@ __device__ __forceinline__ float magic_brick(float n) {
     return (kMagic4 - 4.0f) + 4.0f * ceilf(n * 0.25f);
 #endif
 }
-
-// Kernels whose rays have a step limit above this are compiled with chunk
-// jumps.  A brick jump already crosses up to 66 cells, and a chunk jump has to
-// cross more (distance 3 or above) to pay for its lookup: with limits of 512
-// the walk without them is faster (as first measured: 1080p frame 109 against
-// 111 us, 16-scene batch 1318 against 1343 us); a walk of thousands of empty cells needs up to
-// 7 times fewer jumps with them.
-constexpr int kChunkSteps = 1024;
 
 // A ray the forward walk takes: near origin, and reciprocals in
 // [2^-100, 2^100] in magnitude, so no plane time overflows or is NaN.  For such a
@@ -812,7 +813,6 @@ struct FwdWalk {
 
     // One iteration: a jump out of an empty box, or the unit steps of one
     // visit to an occupied brick.  On a hit wi and vb are its brick and voxel.
-    template <bool CHUNK>
     __device__ __forceinline__ int step(const WorldView& w, unsigned& wi, unsigned& vb) {
         // the brick: magic float and real coordinate per axis, far face
         float rb[3], far[3];
@@ -868,13 +868,18 @@ struct FwdWalk {
             float up = __int2float_rn(layers >> (s >> 6));
             VT_STEP_HOOK(1);
             float K0 = far[0] + across, K1 = far[1] + up, K2 = far[2] + across;
-            if (CHUNK && layers == kVoxCap) {
-                const int dc = w.cdist[((m[0] ? 0u : 1u) | (m[1] ? 0u : 2u) | (m[2] ? 0u : 4u)) * w.cstride + (wi >> 9)];
-                if (dc > 2) {
-                    const int ahead = 8 * dc - 8;   // bricks beyond the chunk's last
-                    K0 = __int2float_rn(4 * (((float_bits(rb[0]) | 7) - 0x4C400000) + ahead + 1));
-                    K1 = __int2float_rn(4 * (((float_bits(rb[1]) | 7) - 0x4C400000) + ahead + 1));
-                    K2 = __int2float_rn(4 * (((float_bits(rb[2]) | 7) - 0x4C400000) + ahead + 1));
+            if (layers == kVoxCap) {
+                // The chunk distance may go on (without it a frame of open space
+                // takes up to twice as long: 3840x2160 from the middle of an empty
+                // 1024x512x1024 world 269 us against 137; its code costs frames
+                // that see none of it up to 3%).  field = octant * nwords and
+                // nwords = 512 nchunks, so its index is the brick's over 512.
+                const unsigned dc = __ldg(w.cdist + ((field + wi) >> 9));
+                if (dc > 2u) {
+                    const float ahead = __fmaf_rn(bits_float((int)(dc | 0x4B000000u)), 32.0f, -32.0f * 8388609.0f);   // 32 (dc - 1)
+                    K0 = chunk_face(nk[0]) + ahead;
+                    K1 = chunk_face(nk[1]) + ahead;
+                    K2 = chunk_face(nk[2]) + ahead;
                 }
             }
             const float t0 = __fmaf_rn(K0, a[0], b[0]), t1 = __fmaf_rn(K1, a[1], b[1]), t2 = __fmaf_rn(K2, a[2], b[2]);
@@ -916,11 +921,11 @@ struct FwdWalk {
     }
 
     // Walks to the ray's end.
-    template <bool MAT, bool LONG>
+    template <bool MAT>
     __device__ __forceinline__ bool finish(const WorldView& w, const PRay& r, TraceHit& h) {
         unsigned wi = 0, vb = 0;
         int s;
-        while ((s = step<LONG>(w, wi, vb)) == kMore) {
+        while ((s = step(w, wi, vb)) == kMore) {
         }
 #ifdef __CUDA_ARCH__
         // The loop's exits meet here: without this the compiler sends the
@@ -936,10 +941,10 @@ struct FwdWalk {
 };
 
 // Traces a ray that passes near_origin and ordinary_inv to its end.
-template <bool MAT, bool LONG>
+template <bool MAT>
 __device__ __forceinline__ bool trace_ordinary(const WorldView& w, const PRay& r, int max_steps, TraceHit& h) {
     FwdWalk fw;
-    return fw.start(w, r, max_steps) && fw.finish<MAT, LONG>(w, r, h);
+    return fw.start(w, r, max_steps) && fw.finish<MAT>(w, r, h);
 }
 
 // Walker to the ray's end.
@@ -961,7 +966,6 @@ __device__ __forceinline__ bool walk_general(const WorldView& w, const unsigned 
 // camera at 2^40; Walker takes such a ray, as it takes any (the test and its code
 // cost 0.3% of a 4K frame with bounce rays, nothing measurable elsewhere; a call
 // out of line 5%).
-template <bool LONG>
 __device__ __forceinline__ bool trace_sun(const WorldView& w, const SunWalk& sun, const float so[3], int max_steps) {
     PRay r;
     pray_init_dir(r, so, sun.d, sun.inv);
@@ -993,18 +997,17 @@ __device__ __forceinline__ bool trace_sun(const WorldView& w, const SunWalk& sun
     } else {
         return walk_general<false, true, true, false>(w, w.cdist, r, max_steps, h);
     }
-    return go && fw.finish<false, LONG>(w, r, h);
+    return go && fw.finish<false>(w, r, h);
 }
 
 // Traces one ray to its end: by the forward walk if it is one that walk takes.
 // NEAR: the origin passes near_origin, or a plane search off by more than one
 // cell will do; SHARE: brick words shared between the lanes of a warp (Walker
-// only); LONG: step limits above kChunkSteps (chunk jumps; without them only
-// speed is lost).
-template <bool MAT, bool RUN = true, bool NEAR = false, bool SHARE = false, bool LONG = true>
+// only).
+template <bool MAT, bool RUN = true, bool NEAR = false, bool SHARE = false>
 __device__ __forceinline__ bool trace_fast(const WorldView& w, const unsigned char* cdist, const PRay& r,
                                            int max_steps, TraceHit& h) {
-    if (NEAR && RUN && !SHARE && ordinary_inv(r.inv) && near_origin(r.o)) return trace_ordinary<MAT, LONG>(w, r, max_steps, h);
+    if (NEAR && RUN && !SHARE && ordinary_inv(r.inv) && near_origin(r.o)) return trace_ordinary<MAT>(w, r, max_steps, h);
     return walk_general<MAT, RUN, NEAR, SHARE>(w, cdist, r, max_steps, h);
 }
 

@@ -39,7 +39,7 @@ struct WorldView {
     unsigned nwords;                    // number of brick words
     unsigned ncoarse;                   // number of coarse words
     unsigned nchunks;
-    unsigned cstride;                   // bytes per chunk-distance field (nchunks rounded up to 16)
+    unsigned cstride;                   // bytes per chunk-distance field
 };
 
 // The fields of the shadow rays' forward walk (FwdWalk) that depend on the sun
@@ -77,7 +77,9 @@ constexpr int kVoxCap = 62;
 // primary rays above the ground) see the open space in front of them instead
 // of the terrain they came from.
 constexpr int kOctants = 8;
-__host__ __device__ inline unsigned cdist_stride(unsigned nchunks) { return (nchunks + 15u) / 16u * 16u; }
+// Bytes per chunk-distance field: packed, so that an entry's index is that of
+// its bricks' distances over 512.
+__host__ __device__ inline unsigned cdist_stride(unsigned nchunks) { return nchunks; }
 // The brick field of an octant whose rays move down (-y) picks, per brick, the
 // shape of its empty box: vertical weight w = 2^shape, shape 0..3, s = min
 // over occupied voxels of max(dx, w*dy, dz), a box of s-1 layers across and
@@ -172,7 +174,7 @@ struct vt_ctx {
     // screen tables of the frame sizes rendered so far (see screen_table)
     vt::ScreenTable screen[vt::kScreenTables];
     int n_screen = 0;
-    int bounce_blocks[4] = {0, 0, 0, 0};  // resident blocks of the bounce walk kernels (brick-run, one-path; short, long step limits)
+    int bounce_blocks[2] = {0, 0};     // resident blocks of the bounce walk kernels (brick-run, one-path)
 };
 
 namespace vt {
