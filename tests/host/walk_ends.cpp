@@ -149,11 +149,11 @@ enum { kEnded = 0, kEndless = 1, kOutOfRange = 2 };
 
 static int fault_of(const WalkFault& e) { return strcmp(e.what(), "endless") ? kOutOfRange : kEndless; }
 
-// Primary rays of a width x height frame (16 floats of view, row major): per
-// pixel {how the walk ended, the record's flags}.
+// Primary and shadow rays of a width x height frame (16 floats of view, row
+// major): per pixel {how the walks ended, the record's flags}.
 extern "C" void we_frame(const int32_t dims[3], const uint8_t* dense, const uint8_t* brick, const uint8_t* chunk,
                          const float pos[3], const float view[16], float tan_half_fov, int32_t width, int32_t height,
-                         int32_t max_steps, int64_t limit, uint8_t* out) {
+                         const float sun[3], int32_t max_steps, int64_t limit, uint8_t* out) {
     HostWorld hw(dims, dense, brick, chunk);
     vt::FrameParams f;
     memset(&f, 0, sizeof(f));
@@ -169,9 +169,16 @@ extern "C" void we_frame(const int32_t dims[3], const uint8_t* dense, const uint
     f.width = width;
     f.height = height;
     f.row_end = height;
-    f.max_steps = max_steps;
-    f.rays = VT_RAYS_PRIMARY;
+    f.max_steps = f.shadow_max_steps = max_steps;
+    f.sunw = sun_fields(sun, hw.w);
+    for (int j = 0; j < 3; ++j) {
+        f.sun[j] = sun[j];
+        f.sun_d[j] = f.sunw.d[j];
+        f.sun_inv[j] = f.sunw.inv[j];
+    }
+    f.rays = VT_RAYS_PRIMARY | VT_RAYS_SHADOW;
     f.shade = VT_SHADE_NONE;
+    const bool any = vt::any_shadow(f);
     for (int y = 0; y < height; ++y)
         for (int x = 0; x < width; ++x) {
             uint8_t* o = out + 2 * ((size_t)y * width + x);
@@ -180,8 +187,9 @@ extern "C" void we_frame(const int32_t dims[3], const uint8_t* dense, const uint
             steps_left = limit;
             try {
                 vt::PixelCounters pc;
-                const uint4 r = vt::render_pixel<false, false, vt::CoarseGlobal, false, false, false, false>(
-                    hw.w, vt::CoarseGlobal{nullptr}, hw.w.cdist, f, x, y, vt::pixel_uv(f, x, y), nullptr, pc);
+                auto pixel = any ? vt::render_pixel<false, false, vt::CoarseGlobal, false, false, false, true>
+                                 : vt::render_pixel<false, false, vt::CoarseGlobal, false, false, false, false>;
+                const uint4 r = pixel(hw.w, vt::CoarseGlobal{nullptr}, hw.w.cdist, f, x, y, vt::pixel_uv(f, x, y), nullptr, pc);
                 o[1] = (uint8_t)(r.w >> 16);
             } catch (const WalkFault& e) {
                 o[0] = (uint8_t)fault_of(e);
@@ -209,7 +217,7 @@ extern "C" void we_shadow(const int32_t dims[3], const uint8_t* dense, const uin
             vt::TraceHit h;
             try {
                 if (k == 0) {
-                    o[1] = vt::trace_sun(hw.w, s, so, max_steps);
+                    o[1] = vt::trace_sun<true>(hw.w, s, so, max_steps);
                 } else if (k == 1) {
                     o[1] = vt::trace_fast<false, true, true>(hw.w, hw.w.cdist, r, max_steps, h);
                 } else {

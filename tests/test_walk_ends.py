@@ -44,14 +44,17 @@ def world(ht, vtlib):  # noqa: F811
     return with_distances(ht, vtlib.gen_world(vtlib.gen_desc(DIMS, scale=0.5, seed=7, trees=12, caves=True)))
 
 
+SUN = (0.4, 0.8, -0.3)
+
+
 def trace_frame(we, world, pos, view, tan_half_fov, W, H, max_steps, limit):
-    """Per pixel of a frame's primary rays {how the walk ended, the record's flags}."""
+    """Per pixel of a frame's primary and shadow rays {how the walks ended, the record's flags}."""
     out = np.zeros((H * W, 2), np.uint8)
-    we.we_frame.argtypes = [C.POINTER(C.c_int32)] + [C.c_void_p] * 5 + [C.c_float] + [C.c_int32] * 3 + [C.c_int64, C.c_void_p]
-    p = np.array(pos, np.float32)
+    we.we_frame.argtypes = [C.POINTER(C.c_int32)] + [C.c_void_p] * 5 + [C.c_float] + [C.c_int32] * 2 + [C.c_void_p, C.c_int32, C.c_int64, C.c_void_p]
+    p, sun = np.array(pos, np.float32), np.array(SUN, np.float32)
     dims, mats, brick, chunk = world
     we.we_frame(dims, mats.ctypes.data, brick.ctypes.data, chunk.ctypes.data, p.ctypes.data, view.ctypes.data,
-                tan_half_fov, W, H, max_steps, limit, out.ctypes.data)
+                tan_half_fov, W, H, sun.ctypes.data, max_steps, limit, out.ctypes.data)
     return out
 
 
@@ -69,10 +72,35 @@ def test_frames_of_scaled_views(we, oracle, vtlib, world, pos, scale):
     cam.view = (C.c_float * 16)(*view)
     out = trace_frame(we, world, pos, view, cam.tan_half_fov, W, H, 512, LIMIT)
     assert np.all(out[:, 0] == 0), (np.bincount(out[:, 0]), "pixels that ended, did not end, read out of range")
-    params = vtlib.default_params(rays=vtlib.RAYS_PRIMARY, shade=vtlib.SHADE_NONE)
+    params = vtlib.default_params(rays=vtlib.RAYS_PRIMARY | vtlib.RAYS_SHADOW, shade=vtlib.SHADE_NONE, sun_dir=SUN)
     ref, _ = oracle.render(oracle.OracleWorld(world[1]), vtlib.default_palette(), cam, params, threads=4)
     assert np.array_equal(out[:, 1], ref["flags"])
     if scale == 1.0 and pos[0] == 30.5:
+        assert np.count_nonzero(out[:, 1]) > 100 and np.any(out[:, 1] & vtlib.HIT_SHADOWED)
+
+
+@pytest.mark.parametrize("exponent", [12, 19, 19.95, 20.1, 21, 24, 30, 36, 42, 46, 60])
+def test_frames_of_far_cameras(we, oracle, vtlib, world, exponent):
+    """Cameras at 2^exponent cells on a diagonal, looking at the world: on both
+    sides of the bound of near origins, and where plane times run together."""
+    W, H = 31, 29
+    away = np.array([0.6, 0.62, 0.5])
+    pos = np.float32(np.array(DIMS) / 2 + away / np.linalg.norm(away) * 2.0 ** exponent)
+    f = (np.array(DIMS) / 2 - pos.astype(np.float64))
+    f /= np.linalg.norm(f)
+    r = np.cross([0.0, 1.0, 0.0], f)
+    r /= np.linalg.norm(r)
+    view = np.zeros((4, 4), np.float32)
+    view[0, :3], view[1, :3], view[2, :3] = r, np.cross(f, r), f
+    cam = vtlib.Camera(pos=pos, fov=1.0, width=W, height=H).as_uniform_data()
+    cam.view = (C.c_float * 16)(*view.reshape(-1))
+    cam.tan_half_fov = min(1.0, 60.0 * 2.0 ** -exponent)
+    out = trace_frame(we, world, pos, view.reshape(-1), cam.tan_half_fov, W, H, 512, LIMIT)
+    assert np.all(out[:, 0] == 0), np.bincount(out[:, 0])
+    params = vtlib.default_params(rays=vtlib.RAYS_PRIMARY | vtlib.RAYS_SHADOW, shade=vtlib.SHADE_NONE, sun_dir=SUN)
+    ref, _ = oracle.render(oracle.OracleWorld(world[1]), vtlib.default_palette(), cam, params, threads=4)
+    assert np.array_equal(out[:, 1], ref["flags"])
+    if exponent < 20:
         assert np.count_nonzero(out[:, 1]) > 100
 
 

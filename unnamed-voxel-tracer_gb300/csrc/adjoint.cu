@@ -102,8 +102,8 @@ __device__ __forceinline__ float warp_sum4(unsigned lane, float a, float b, floa
 // a sum over the warp per value and float atomics for every sum; now 258.
 // Register caps: 6 blocks per SM (40 registers); backward with 5 269 us, with 7
 // 250, but 2% slower on one view of 1920x1080; forward with 5 2% slower.
-// ANYSUN: a sun direction the forward walk does not take (trace_fast).
-template <bool BWD, bool ANYSUN>
+// ANY: a sun direction the forward walk does not take (trace_fast).
+template <bool BWD, bool ANY>
 __global__ void __launch_bounds__(kAdjBlock, 6) k_shade_views(const __grid_constant__ ViewsArgs va) {
     const AdjArgs& a = va.a;
     const ViewP& V = va.v[blockIdx.z];
@@ -165,13 +165,13 @@ __global__ void __launch_bounds__(kAdjBlock, 6) k_shade_views(const __grid_const
                 lit = a.vis_in[p] != 0;
             } else {
                 bool blocked;
-                if (ANYSUN) {
+                if (ANY) {
                     PRay rs;
                     pray_init_dir(rs, so, a.sun.d, a.sun.inv);
                     TraceHit hs;
                     blocked = trace_fast<false, true, true>(a.w, a.w.cdist, rs, a.shadow_steps, hs);
                 } else {
-                    blocked = trace_sun(a.w, a.sun, so, a.shadow_steps);
+                    blocked = trace_sun<true>(a.w, a.sun, so, a.shadow_steps);
                 }
                 lit = !blocked &&
                       !(a.w.n_entities > 0 && entity_occluded(a.w, so, a.sun_raw));
@@ -325,9 +325,9 @@ vt_status launch_shade_views(vt_ctx* ctx, const vt_world* world, int32_t n, cons
         s = shade_sums(ctx, st, &a.sums, &used);
         if (s) return s;
     }
-    const bool anysun = !ordinary_inv(a.sun.inv);
-    auto k = bwd ? (anysun ? k_shade_views<true, true> : k_shade_views<true, false>)
-                 : (anysun ? k_shade_views<false, true> : k_shade_views<false, false>);
+    const bool any = !ordinary_inv(a.sun.inv);
+    auto k = bwd ? (any ? k_shade_views<true, true> : k_shade_views<true, false>)
+                 : (any ? k_shade_views<false, true> : k_shade_views<false, false>);
     ViewsArgs va;
     std::memset(&va, 0, sizeof(va));
     cudaError_t e = cudaSuccess;

@@ -84,7 +84,7 @@ static_assert(sizeof(JobChunk) <= 32764, "a kernel's parameters are limited to 3
 // One thread per pixel; the 128-thread block covers a 16 x 8 tile as four
 // 8 x 4 warp tiles (the single-frame kernel's default shape), with the same
 // register cap (36 warps per SM).
-template <bool CHECKED, bool BOUNCE, bool ANYSUN>
+template <bool CHECKED, bool BOUNCE, bool ANY>
 __global__ void __launch_bounds__(kTileBlock, 9) k_render_jobs(const __grid_constant__ JobChunk p, unsigned* status) {
     const unsigned b = blockIdx.x;
     int lo = 0, hi = p.njobs - 1;
@@ -140,11 +140,12 @@ __global__ void __launch_bounds__(kTileBlock, 9) k_render_jobs(const __grid_cons
         uv.gv = s_row[2][ly];
     }
     PixelCounters pc;
-    const uint4 rec = render_pixel<false, CHECKED, CoarseGlobal, false, false, BOUNCE, ANYSUN>(p.w, CoarseGlobal{p.w.coarse}, p.w.cdist, f, px, py, uv, status, pc);
+    const uint4 rec = render_pixel<false, CHECKED, CoarseGlobal, false, false, BOUNCE, ANY>(p.w, CoarseGlobal{p.w.coarse}, p.w.cdist, f, px, py, uv, status, pc);
     p.cam[lo].out[(size_t)py * f.width + px] = rec;
 }
 
 // --------------------------------------------------------------- queue shape
+template <bool ANY>
 __global__ void __launch_bounds__(kBatchBlock, 3) k_render_batch(const JobDesc* __restrict__ jobs, int njobs,
                                                                  unsigned total_units, unsigned* __restrict__ counter) {
     const unsigned lane = threadIdx.x & 31u;
@@ -172,8 +173,8 @@ __global__ void __launch_bounds__(kBatchBlock, 3) k_render_batch(const JobDesc* 
             if (px < f.width && py < f.height) {
                 PixelCounters pc;
                 J.out[(size_t)py * f.width + px] =
-                    render_pixel<false, false>(w, CoarseGlobal{w.coarse}, w.cdist, f, px, py, pixel_uv(f, px, py),
-                                               nullptr, pc);
+                    render_pixel<false, false, CoarseGlobal, false, false, true, ANY>(
+                        w, CoarseGlobal{w.coarse}, w.cdist, f, px, py, pixel_uv(f, px, py), nullptr, pc);
             }
         }
     }
@@ -194,6 +195,7 @@ struct vt_batch {
     unsigned total_units = 0;
     unsigned long long pixels = 0;
     unsigned blocks = 0;
+    bool any = false;   // some job needs kernels for any shadow ray (any_shadow)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
@@ -292,6 +294,7 @@ vt_status vt_batch_create(vt_ctx* ctx, const vt_job* jobs, int32_t n, const vt_p
         d.w = j.world->view();
         d.f = make_frame(&j.camera, params);
         walk_constants(d.f, d.w);
+        b->any = b->any || any_shadow(d.f);
         d.out = reinterpret_cast<uint4*>(j.d_out);
         d.first_unit = (unsigned)units;
         d.units_x = (unsigned)((j.camera.width + kUnit - 1) / kUnit);
@@ -313,7 +316,7 @@ vt_status vt_batch_create(vt_ctx* ctx, const vt_job* jobs, int32_t n, const vt_p
         return check_cuda(ctx, e, "batch upload");
     }
     int per_sm = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_render_batch, kBatchBlock, 0)) != cudaSuccess) {
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->any ? k_render_batch<true> : k_render_batch<false>, kBatchBlock, 0)) != cudaSuccess) {
         vt_batch_destroy(b);
         return check_cuda(ctx, e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     }
@@ -357,7 +360,8 @@ vt_status vt_batch_launch(vt_batch* b, vt_stream stream) {
         if (e == cudaSuccess) {
             if (shape == VT_KERNEL_QUEUE) {
                 cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned), cap);
-                k_render_batch<<<b->blocks, kBatchBlock, 0, cap>>>(b->d_jobs, b->njobs, b->total_units, b->d_counter);
+                (b->any ? k_render_batch<true> : k_render_batch<false>)<<<b->blocks, kBatchBlock, 0, cap>>>(
+                    b->d_jobs, b->njobs, b->total_units, b->d_counter);
             } else {
                 // fork chains off the capture stream, launches longest first on
                 // the least loaded chain (chain_plan), join
@@ -369,10 +373,10 @@ vt_status vt_batch_launch(vt_batch* b, vt_stream stream) {
                     for (const auto& pc : chain_plan(wt)) {
                         const JobChunk& ch = b->chunks[pc.first];
                         const unsigned blocks = ch.first_block[ch.njobs];
-                        const bool bounce = (b->params.rays & VT_RAYS_BOUNCE) != 0, anysun = !ordinary_sun(ch.f);
+                        const bool bounce = (b->params.rays & VT_RAYS_BOUNCE) != 0, any = b->any;
                         auto k = checked ? k_render_jobs<true, true, true>
-                                 : bounce ? (anysun ? k_render_jobs<false, true, true> : k_render_jobs<false, true, false>)
-                                          : (anysun ? k_render_jobs<false, false, true> : k_render_jobs<false, false, false>);
+                                 : bounce ? (any ? k_render_jobs<false, true, true> : k_render_jobs<false, true, false>)
+                                          : (any ? k_render_jobs<false, false, true> : k_render_jobs<false, false, false>);
                         k<<<blocks, kTileBlock, 0, chain[pc.second]>>>(ch, checked ? ctx->d_status : nullptr);
                     }
                 } else {

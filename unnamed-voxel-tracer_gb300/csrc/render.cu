@@ -55,7 +55,7 @@ struct BlockTile {
 // (Walker::brick_word).  BIN: deferred bounce rays are appended per block,
 // sorted by direction (stage_flush).
 template <bool STATS, bool CHECKED, bool SMEM, int TW, bool OCC, bool SHARE = false, bool BIN = false, bool BOUNCE = true,
-          bool ANYSUN = true, int NB = kBlock>
+          bool ANY = true, int NB = kBlock>
 __global__ void __launch_bounds__(NB, OCC ? (NB == kSmallBlock ? kSmallBlocks : kOccThreads / NB) : 1)
     k_render(const __grid_constant__ WorldView w, const __grid_constant__ FrameParams f, uint4* __restrict__ out,
              unsigned* status, unsigned long long* counters) {
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(NB, OCC ? (NB == kSmallBlock ? kSmallBlocks : 
         }
         uint4 rec;
         if (SMEM) rec = render_pixel<STATS, CHECKED>(w, CoarseShared{s_coarse}, w.cdist, f, px, py, uv, status, pc);
-        else rec = render_pixel<STATS, CHECKED, CoarseGlobal, SHARE, BIN, BOUNCE, ANYSUN>(w, CoarseGlobal{w.coarse}, w.cdist, f, px,
+        else rec = render_pixel<STATS, CHECKED, CoarseGlobal, SHARE, BIN, BOUNCE, ANY>(w, CoarseGlobal{w.coarse}, w.cdist, f, px,
                                                                           py, uv, status, pc);
         out[(size_t)py * f.width + px] = rec;
     }
@@ -537,10 +537,10 @@ vt_status launch_render(vt_ctx* ctx, const vt_world* world, const vt_camera* cam
                                          dim3(kBlock), sm, stream, win, w, f, d_out, ctx->d_status, ctx->d_counters); }
         else if (tu.occupancy && tu.share_bricks) { VT_LAUNCH_X(false, false, false, 8, true, true); }
         else if (tu.occupancy) {
-            const bool bounce = (p->rays & VT_RAYS_BOUNCE) != 0, anysun = !ordinary_sun(f);
-            auto k = bounce ? (anysun ? k_render<false, false, false, 8, true, false, false, true, true>
+            const bool bounce = (p->rays & VT_RAYS_BOUNCE) != 0, any = any_shadow(f);
+            auto k = bounce ? (any ? k_render<false, false, false, 8, true, false, false, true, true>
                                    : k_render<false, false, false, 8, true, false, false, true, false>)
-                            : (anysun ? k_render<false, false, false, 8, true, false, false, false, true, kSmallBlock>
+                            : (any ? k_render<false, false, false, 8, true, false, false, false, true, kSmallBlock>
                                    : k_render<false, false, false, 8, true, false, false, false, false, kSmallBlock>);
             const int th = bounce ? BlockTile<8>::kH : BlockTile<8, kSmallBlock>::kH;
             le = launch_kernel(k, dim3((cam->width + BlockTile<8>::kW - 1) / BlockTile<8>::kW, (rows + th - 1) / th),

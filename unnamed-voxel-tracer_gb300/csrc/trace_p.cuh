@@ -961,11 +961,11 @@ __device__ __forceinline__ bool walk_general(const WorldView& w, const unsigned 
 
 // Whether the shadow ray from so is blocked (a sun that passes ordinary_inv):
 // the fields of its walk that depend on the sun alone are given, and an origin
-// at least one cell inside the grid starts in its own cell (pray_start).  so may be
-// anywhere, or not a number, where it comes from a caller's hit records or a
-// camera at 2^40; Walker takes such a ray, as it takes any (the test and its code
-// cost 0.3% of a 4K frame with bounce rays, nothing measurable elsewhere; a call
-// out of line 5%).
+// at least one cell inside the grid starts in its own cell (pray_start).  ANY: so
+// may be anywhere, as where it is made from a caller's hit records; where it is
+// not near, Walker takes the ray, as it takes any (inline: a call out of line
+// costs 2 to 5%).  Otherwise so is near, or not a number (a miss).
+template <bool ANY>
 __device__ __forceinline__ bool trace_sun(const WorldView& w, const SunWalk& sun, const float so[3], int max_steps) {
     PRay r;
     pray_init_dir(r, so, sun.d, sun.inv);
@@ -992,7 +992,7 @@ __device__ __forceinline__ bool trace_sun(const WorldView& w, const SunWalk& sun
         fw.limit = ((fw.nk[0] + fw.nk[1]) + fw.nk[2]) + __int2float_rn(min(max_steps, 1 << 20));
         fw.flip = sun.flip;
         fw.field = sun.field;
-    } else if (near_origin(so)) {
+    } else if (!ANY || near_origin(so)) {
         go = fw.start(w, r, max_steps);
     } else {
         return walk_general<false, true, true, false>(w, w.cdist, r, max_steps, h);
