@@ -102,8 +102,10 @@ __device__ __forceinline__ float warp_sum4(unsigned lane, float a, float b, floa
 // a sum over the warp per value and float atomics for every sum; now 258.
 // Register caps: 6 blocks per SM (40 registers); backward with 5 269 us, with 7
 // 250, but 2% slower on one view of 1920x1080; forward with 5 2% slower.
-// ANY: a sun direction the forward walk does not take (trace_fast).
-template <bool BWD, bool ANY>
+// ANY: a sun direction the forward walk does not take (trace_fast).  VIS: the
+// shadow term is given, no ray is traced: bound by memory, and a kernel without
+// the walk's registers (3840x2160 63.5 us; in the kernel with the walk 88).
+template <bool BWD, bool ANY, bool VIS = false>
 __global__ void __launch_bounds__(kAdjBlock, 6) k_shade_views(const __grid_constant__ ViewsArgs va) {
     const AdjArgs& a = va.a;
     const ViewP& V = va.v[blockIdx.z];
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(kAdjBlock, 6) k_shade_views(const __grid_const
                 so[j] = __fmaf_rn(d, t, V.pos[j]);
                 if (j == axis) so[j] = so[j] + nrm[j] * 0.001f;
             }
-            if (a.vis_in) {
+            if (VIS) {
                 lit = a.vis_in[p] != 0;
             } else {
                 bool blocked;
@@ -327,7 +329,8 @@ vt_status launch_shade_views(vt_ctx* ctx, const vt_world* world, int32_t n, cons
     }
     const bool any = !ordinary_inv(a.sun.inv);
     auto k = bwd ? (any ? k_shade_views<true, true> : k_shade_views<true, false>)
-                 : (any ? k_shade_views<false, true> : k_shade_views<false, false>);
+                 : (a.vis_in ? k_shade_views<false, false, true>
+                             : (any ? k_shade_views<false, true> : k_shade_views<false, false>));
     ViewsArgs va;
     std::memset(&va, 0, sizeof(va));
     cudaError_t e = cudaSuccess;
