@@ -420,9 +420,12 @@ vt_status vt_shade_forward(vt_ctx* ctx, const vt_world* world, const vt_camera* 
 /* Fused forward + backward of the loss: recomputes the shading (shadow rays
  * traced again, not stored), adds the loss to *d_loss and the gradients to
  * d_grad_palette (256 x 3), d_grad_albedo (X*Y*Z, may be NULL) and
- * d_grad_sun (3).  The caller owns and zeroes these accumulators.  Gradients
- * are accumulated with float atomics, so their last bits depend on the order
- * in which blocks finish. */
+ * d_grad_sun (3).  The caller owns and zeroes these accumulators.  The albedo
+ * gradient is accumulated with float atomics, so its last bits depend on the
+ * order in which blocks finish; the others are summed in 64 bits before they
+ * are added, except while `stream` is being captured, where they too are float
+ * atomics.  At most eight uncaptured backward calls of a context run at once: a
+ * ninth waits, on its stream, for the first. */
 vt_status vt_shade_backward(vt_ctx* ctx, const vt_world* world, const vt_camera* cam, const vt_hit* d_hits,
                             const vt_shade_inputs* in, const float* d_target, float* d_loss, float* d_grad_palette,
                             float* d_grad_albedo, float* d_grad_sun, vt_stream stream);

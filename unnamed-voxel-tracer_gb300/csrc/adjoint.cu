@@ -297,16 +297,23 @@ bool camera_size_ok(const vt_camera* cam) {
 }
 
 // One of the context's accumulator regions for a call on st, which first waits
-// for the call that used the region last (on any stream); the caller records
-// *used after its launches.  None while st is being captured: the
-// graph's replays could overlap other launches.
+// for the call that used the region last (on any stream), or clears it if it is
+// the first; the caller records *used after its launches.  None while st is
+// being captured: the graph's replays could overlap other launches.
 vt_status shade_sums(vt_ctx* ctx, cudaStream_t st, double** sums, cudaEvent_t* used) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     VT_CUDA(ctx, cudaStreamIsCapturing(st, &cs));
     if (cs != cudaStreamCaptureStatusNone) return VT_OK;
-    const unsigned r = ctx->shade_region++ % kShadeRegions;
-    VT_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_shade[r], 0));
-    *sums = reinterpret_cast<double*>(static_cast<char*>(ctx->d_shade_sums) + (size_t)r * kShadeSumBytes);
+    const unsigned r = ctx->shade_region % kShadeRegions;
+    void* region = static_cast<char*>(ctx->d_shade_sums) + (size_t)r * kShadeSumBytes;
+    if (ctx->ev_shade[r]) {
+        VT_CUDA(ctx, cudaStreamWaitEvent(st, ctx->ev_shade[r], 0));
+    } else {
+        VT_CUDA(ctx, cudaMemsetAsync(region, 0, kShadeSumBytes, st));
+        VT_CUDA(ctx, cudaEventCreateWithFlags(&ctx->ev_shade[r], cudaEventDisableTiming));
+    }
+    ++ctx->shade_region;
+    *sums = static_cast<double*>(region);
     *used = ctx->ev_shade[r];
     return VT_OK;
 }

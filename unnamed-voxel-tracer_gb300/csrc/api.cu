@@ -187,12 +187,10 @@ vt_status vt_ctx_create(int32_t device, vt_ctx** out) {
         ctx->sm_count = prop.multiProcessorCount;
         if ((e = dev_alloc(&ctx->d_status, sizeof(unsigned))) != cudaSuccess) { s = check_cuda(ctx, e, "cudaMalloc"); break; }
         if ((e = cudaMemset(ctx->d_status, 0, sizeof(unsigned))) != cudaSuccess) { s = check_cuda(ctx, e, "cudaMemset"); break; }
-        if ((e = dev_alloc(&ctx->d_counters, kNumCounters * sizeof(unsigned long long))) != cudaSuccess) { s = check_cuda(ctx, e, "cudaMalloc"); break; }
+        // (the shading's accumulator regions behind the counters: one allocation)
+        if ((e = dev_alloc(&ctx->d_counters, kNumCounters * sizeof(unsigned long long) + kShadeRegions * kShadeSumBytes)) != cudaSuccess) { s = check_cuda(ctx, e, "cudaMalloc"); break; }
+        ctx->d_shade_sums = ctx->d_counters + kNumCounters;
         if ((e = dev_alloc(&ctx->d_work, kWorkSlots * sizeof(unsigned))) != cudaSuccess) { s = check_cuda(ctx, e, "cudaMalloc"); break; }
-        if ((e = dev_alloc(&ctx->d_shade_sums, kShadeRegions * kShadeSumBytes)) != cudaSuccess) { s = check_cuda(ctx, e, "cudaMalloc"); break; }
-        if ((e = cudaMemset(ctx->d_shade_sums, 0, kShadeRegions * kShadeSumBytes)) != cudaSuccess) { s = check_cuda(ctx, e, "cudaMemset"); break; }
-        for (unsigned i = 0; i < kShadeRegions && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&ctx->ev_shade[i], cudaEventDisableTiming);
-        if (e != cudaSuccess) { s = check_cuda(ctx, e, "cudaEventCreate"); break; }
         if ((e = host_alloc(&ctx->h_status, sizeof(unsigned))) != cudaSuccess) { s = check_cuda(ctx, e, "cudaHostAlloc"); break; }
         *ctx->h_status = 0;
         if ((e = cudaEventCreateWithFlags(&ctx->ev_status, cudaEventDisableTiming)) != cudaSuccess) { s = check_cuda(ctx, e, "cudaEventCreate"); break; }
@@ -233,7 +231,6 @@ vt_status vt_ctx_destroy(vt_ctx* ctx) {
     dev_free(ctx->d_bounce_tail);
     dev_free(ctx->d_bounce_ctr);
     if (ctx->ev_bounce) cudaEventDestroy(ctx->ev_bounce);
-    dev_free(ctx->d_shade_sums);
     for (unsigned i = 0; i < kShadeRegions; ++i)
         if (ctx->ev_shade[i]) cudaEventDestroy(ctx->ev_shade[i]);
     for (int i = 0; i < ctx->n_screen; ++i) dev_free(ctx->screen[i].d);

@@ -168,7 +168,7 @@ struct vt_ctx {
     unsigned* d_bounce_ctr = nullptr;  // {queued, taken}
     size_t bounce_capacity = 0;
     cudaEvent_t ev_bounce = nullptr;   // the last deferred frame is done with the queue
-    void* d_shade_sums = nullptr;      // kShadeRegions accumulator regions, zero between calls
+    void* d_shade_sums = nullptr;      // kShadeRegions accumulator regions (in d_counters), zero between calls from the first on
     unsigned shade_region = 0;
     cudaEvent_t ev_shade[vt::kShadeRegions] = {};
     // screen tables of the frame sizes rendered so far (see screen_table)
