@@ -97,8 +97,8 @@ __device__ __forceinline__ float warp_sum4(unsigned lane, float a, float b, floa
 // way within a binade, and the gradients of such scenes came out up to 4.6e-4
 // from one call per view, where two runs of either differ by up to 9e-5.
 //
-// Bound: issue slots (forward 81%, backward with its albedo atomics waiting for
-// L2).  An iteration on 16 views of 512x512 took 339 us with the general walk,
+// Bound: issue slots (forward 79%, 84 us; backward 63%, 147 us, its palette's
+// clearing and flushing and its albedo atomics waiting for L2).  An iteration on 16 views of 512x512 took 339 us with the general walk,
 // a sum over the warp per value and float atomics for every sum; now 258.
 // Register caps: 6 blocks per SM (40 registers); backward with 5 269 us, with 7
 // 250, but 2% slower on one view of 1920x1080; forward with 5 2% slower.

@@ -14,7 +14,7 @@ constexpr int kBounceBlock = 256;
 // (tuning bounce_refill), and a busy lane makes kActions iterations of the walk
 // between two refill checks: 12 and 3 are fastest of 4-16 and 1-4 with the
 // forward walk (4K cave frame as first measured 1145 us; 8 and 2: 1182, 16 and
-// 4: 1146; refill alone, now: 12 1120 us, 4 1141, 8 1138, 16 1118)
+// 4: 1146; refill alone, now: 12 1135 us, 4 1145, 8 1142, 16 1132)
 constexpr int kRefill = 12;
 constexpr int kActions = 3;
 
@@ -65,10 +65,11 @@ __device__ __forceinline__ void open_pixel(uint4* out, unsigned pixel, unsigned 
 
 // Persistent: every warp loops until the queue is drained.  A lane walks one
 // ray at a time, kActions iterations of the walk per loop turn.
-// Bound: issue slots (76%) at 12 lanes an instruction, the lanes of a warp
+// Bound: issue slots (78%) at 11.7 lanes an instruction, the lanes of a warp
 // being in different phases of unrelated walks; the register cap (4 blocks of
 // 64 registers; uncapped 96) hides the lookups' latency.  7 M rays of a 4K
-// cave frame: 601 us.  Measured against 614 then, slower: setting 32 rays up at a time in shared
+// cave frame: 622 us (601 without chunk jumps and the far test).  Measured
+// against 614 then, slower: setting 32 rays up at a time in shared
 // memory for idle lanes to take (727 us: the copies cost more instructions
 // than the set-ups at few lanes), one code path for jumps and unit steps (568 us
 // here, but 11% slower on a 1021x577 frame whose queue is short).

@@ -37,8 +37,8 @@ vt_status parse_vox(const uint8_t* bytes, size_t n, std::vector<std::vector<uint
 namespace {
 
 constexpr int kModels = 32768;
-// 16 x 8 pixels; 8 blocks per SM (1080p frame 620 us; uncapped 643, 16 x 16
-// pixels 651)
+// 16 x 8 pixels; 8 blocks per SM (1080p frame 620 us; uncapped 643; 16 x 16
+// pixels with as many warps per SM 621, uncapped 651)
 constexpr int kRefBlock = 128;
 
 struct RefView {
@@ -77,9 +77,9 @@ __device__ __forceinline__ unsigned ref_get_subvoxel(const RefView& w, unsigned 
 //   - one branch leaves the path of most steps (an empty chunk, crossed voxel
 //     by voxel); chunk, voxel and sub-voxel bits are masked in place.
 // With the light's sky per block and the entity boxes' slab test before their
-// divisions, a 1080p frame went from 752 M to 475 M warp instructions and from
-// 846 to 531 us (ncu, 16 x 16 blocks, another scene than kRefBlock's figures).  Selects instead of the three-way branch at the end of
-// a step: 515 M, 593 us.
+// divisions, a 1080p frame went from 960 to 651 us (kRefBlock's frame, 620 with
+// its blocks; 478 M warp instructions).  Selects instead of the three-way branch
+// at the end of a step: 8% more instructions, 12% more time.
 __device__ void trace_map(const RefView& w, const float o[3], const float din[3], int max_steps, RefHit& out) {
     float d[3] = {din[0], din[1], din[2]};
 #pragma unroll

@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(NB, OCC ? (NB == kSmallBlock ? kSmallBlocks : 
 }
 
 // Explicit ray list (production traversal); record.rgba is 0.
-// Bound: latency and issue (70%) at 9.5 lanes, the rays being unrelated; a
+// Bound: latency and issue (73%) at 8.5 lanes, the rays being unrelated; a
 // block waits for its longest ray, so blocks are two warps (a million rays:
 // 74.5 us in blocks of 256, 72.3 of 128, 71.6 of 64, 75.1 of 32; 64 with 16 to
 // 24 blocks per SM 70.7-72.7).  Lanes that take the next ray as theirs ends: 88 us.

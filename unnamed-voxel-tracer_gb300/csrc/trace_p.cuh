@@ -673,8 +673,8 @@ struct Walker {
 // do not use it, hence the arithmetic on magic floats.  1080p terrain frame,
 // primary + shadow: 168 us (Walker) -> 109, with the steps since (walk
 // constants per frame, converged warps, plane times in occupied bricks only,
-// blocks of 128) 99; 2.96 G thread instructions at 30.4 lanes (Walker: 27.4),
-// 35 M of 97 M warp instructions on that pipe.
+// blocks of 128) 99; 2.99 G thread instructions at 30.3 lanes (Walker: 27.4),
+// 35 M of 99 M warp instructions on that pipe.
 constexpr float kMagic = 12582912.0f;    // 1.5 * 2^23: float spacing 1, and integers of either sign around it
 constexpr float kMagic4 = 50331648.0f;   // 1.5 * 2^25: the same with spacing 4
 
